@@ -7,7 +7,10 @@
 //           warp takes (query row, head of the GQA group) pairs: lanes own keys for Q.K (fp32, the query in shared
 //           memory), the warp reduces max / sum, lanes own head-dim slices for P.V.  Writes the partial output and
 //           its (max, sum) per split.
-//   pass 2 (attn_small_q_merge): one warp per (batch, head, row) folds the splits with the log-sum-exp identity.
+//   pass 2 (attn_small_q_merge): one CTA per (batch, head, row) folds the splits with the log-sum-exp identity.
+//
+// Up to 8 (row, head) pairs per key/value head (a decode step of grouped-query attention) take attn_decode_partial
+// instead of pass 1: bound by reading the cache once, so keys and values go from global memory straight to registers.
 //
 // Causal mask with bottom-right alignment (query row r sits at key position Tk - Tq + r) and an optional sliding
 // window, as flash_attn_func(causal=True, window_size=(W-1, 0)) applies them on the cached decode path of the
@@ -137,37 +140,274 @@ __global__ void __launch_bounds__(SQ_WARPS * 32) attn_small_q_partial_kernel(con
   }
 }
 
-// out[b, row, h, :] = sum_s o_s 2^(m_s - M) / sum_s l_s 2^(m_s - M)
+// ---------------------------------------------------------------------------------------------------------------
+// At most R (query row, head of the group) pairs per key/value head.  D / 8 lanes hold a cached row (16 bytes each),
+// so a warp-wide load brings KPW = 32 / (D / 8) keys; a warp takes U such loads of K and of V at a time, all issued
+// before the first use.  A lane forms the products of its 8 dims for U keys x R pairs, a transposing reduction over
+// the lanes of a key leaves every lane with NV = U R / (D / 8) whole scores (so that each exponential is computed
+// once), and the probabilities travel back by shuffles for the fp32 P V.  Running max per pair, moved only when it
+// grows by 2^8.  No shared memory until the warps of a CTA are merged.
+// The fill count decides the split borders, so that every CTA of a captured launch has work however full the cache is.
+// Bound by the cache's bytes.  One launch for 1 x 8192 keys, 16/8 heads, D 128 (33.6 MB): the staging kernel above
+// took 40.8 us (135 KB of shared memory, so one CTA per SM that first loads and then computes, 1.7 waves).
+constexpr int DEC_WARPS = 8;
+
+template <int D, int R>
+struct DecodeCfg {
+  static constexpr int LPR = D / 8;                 // lanes per cached row
+  static constexpr int KPW = 32 / LPR;              // keys per warp-wide load
+  static constexpr int U = R <= 4 ? 8 : 4;          // loads in flight (of K and of V each)
+  static constexpr int KEYS = KPW * U;              // keys per warp and turn
+  static constexpr int N = U * R;                   // scores per lane group and turn
+  static constexpr int NV = N >= LPR ? N / LPR : 1; // ... of which a lane ends up with
+  static constexpr int DUP = N >= LPR ? 1 : LPR / N;// lanes that hold the same score
+};
+
+template <int D, int R>
+__global__ void __launch_bounds__(DEC_WARPS * 32, R <= 2 ? 2 : 1) attn_decode_partial_kernel(const SmallQParams p) {
+  using C = DecodeCfg<D, R>;
+  constexpr int LPR = C::LPR, KPW = C::KPW, U = C::U, NV = C::NV, DUP = C::DUP;
+  static_assert(NV <= R && (R & (R - 1)) == 0, "a lane's scores belong to different pairs");
+  __shared__ float s_m[DEC_WARPS * KPW][R], s_l[DEC_WARPS * KPW][R];
+  __shared__ __align__(16) float s_o[DEC_WARPS][R][D];
+  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / LPR, l = lane % LPR;       // key of a load, lane of the key
+  const int G = p.H / p.HK, pairs = p.Tq * G;
+  const int Tk = p.kv_len != nullptr ? min(max(*p.kv_len, p.Tq), p.Tk) : p.Tk;
+  // keys [first, Tk) are seen by some row; a split takes a multiple of the CTA's keys per turn
+  const int first = p.window > 0 ? max(0, Tk - p.Tq - p.window + 1) : 0;
+  constexpr int TURN = DEC_WARPS * C::KEYS;
+  const int per = ((Tk - first + p.splits - 1) / p.splits + TURN - 1) / TURN * TURN;
+  const int lo = first + split * per, hi = min(Tk, lo + per);
+
+  // this lane's 8 dims of every query pair (pairs beyond the real ones: zero)
+  float2 q[R][4];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+    if (r < pairs)
+      raw = *reinterpret_cast<const uint4*>(p.q + static_cast<int64_t>(b) * p.sq + static_cast<int64_t>(r / G) * p.ldq +
+                                            (kvh * G + r % G) * D + l * 8);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[r][i] = unpack_bf16(w[i]);
+    }
+  }
+  const bf16* kbase = p.k + static_cast<int64_t>(b) * p.sk + kvh * D + l * 8;
+  const bf16* vbase = p.v + static_cast<int64_t>(b) * p.sv + kvh * D + l * 8;
+
+  float2 o[R][4];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[r][i] = make_float2(0.f, 0.f);
+  // the scores this lane ends up with: n = own0 + j, pair n % R, key n / R
+  const int own0 = (l / DUP) * NV;
+  float m_ref[NV], l_sum[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) { m_ref[j] = -INFINITY; l_sum[j] = 0.f; }
+
+  for (int t0 = lo + warp * C::KEYS; t0 < hi; t0 += TURN) {
+    uint4 kr[U], vr[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {                   // rows past the end re-read the last one (masked below)
+      const int64_t key = min(t0 + u * KPW + grp, Tk - 1);
+      kr[u] = *reinterpret_cast<const uint4*>(kbase + key * p.ldk);
+      vr[u] = *reinterpret_cast<const uint4*>(vbase + key * p.ldv);
+    }
+    float sc[C::N];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float2 k0 = unpack_bf16(kr[u].x), k1 = unpack_bf16(kr[u].y), k2 = unpack_bf16(kr[u].z), k3 = unpack_bf16(kr[u].w);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float2 a = __fmul2_rn(q[r][0], k0);
+        a = __ffma2_rn(q[r][1], k1, a);
+        a = __ffma2_rn(q[r][2], k2, a);
+        a = __ffma2_rn(q[r][3], k3, a);
+        sc[u * R + r] = a.x + a.y;
+      }
+    }
+    // transposing reduction over the lanes of a key: halve the scores while there are several, then plain sums
+#pragma unroll
+    for (int d = LPR / 2, n = C::N; d > 0; d >>= 1) {
+      const bool up = (l & d) != 0;
+      if (n > 1) {
+        n >>= 1;
+#pragma unroll
+        for (int i = 0; i < C::N / 2; ++i)
+          if (i < n) {
+            const float send = up ? sc[i] : sc[n + i], keep = up ? sc[n + i] : sc[i];
+            sc[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+          }
+      } else {
+        sc[0] += __shfl_xor_sync(0xffffffffu, sc[0], d);
+      }
+    }
+    float pr[NV];
+    bool need = false;
+    float m_new[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const int n = own0 + j, r = n % R, key = t0 + (n / R) * KPW + grp;
+      const int qpos = Tk - p.Tq + r / G;
+      const bool vis = key < hi && key <= qpos && (p.window <= 0 || key > qpos - p.window);
+      pr[j] = vis ? sc[j] * p.scale_log2 : -INFINITY;
+      float m = pr[j];
+#pragma unroll
+      for (int d = R / NV * DUP; d < LPR; d <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));   // over the keys
+      m_new[j] = fmaxf(m, m_ref[j]);
+      need = need || m_new[j] > m_ref[j] + 8.f || (m_ref[j] == -INFINITY && m_new[j] > -INFINITY);
+    }
+    if (__any_sync(0xffffffffu, need)) {
+      float f[NV];
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        f[j] = m_ref[j] == -INFINITY ? 0.f : exp2f(m_ref[j] - m_new[j]);
+        l_sum[j] *= f[j];
+        m_ref[j] = m_new[j];
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float fr = __shfl_sync(0xffffffffu, f[r % NV], r / NV * DUP, LPR);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[r][i] = make_float2(o[r][i].x * fr, o[r][i].y * fr);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      pr[j] = pr[j] == -INFINITY ? 0.f : exp2f(pr[j] - m_ref[j]);
+      l_sum[j] += pr[j];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float2 v0 = unpack_bf16(vr[u].x), v1 = unpack_bf16(vr[u].y), v2 = unpack_bf16(vr[u].z), v3 = unpack_bf16(vr[u].w);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int n = u * R + r;
+        const float e = __shfl_sync(0xffffffffu, pr[n % NV], n / NV * DUP, LPR);
+        const float2 e2 = make_float2(e, e);
+        o[r][0] = __ffma2_rn(e2, v0, o[r][0]);
+        o[r][1] = __ffma2_rn(e2, v1, o[r][1]);
+        o[r][2] = __ffma2_rn(e2, v2, o[r][2]);
+        o[r][3] = __ffma2_rn(e2, v3, o[r][3]);
+      }
+    }
+  }
+  // ---- merge the lane groups of all warps: row (warp, group) of s_m / s_l, then one common max per pair
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    float s = l_sum[j];
+#pragma unroll
+    for (int d = R / NV * DUP; d < LPR; d <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (l < R / NV * DUP && l % DUP == 0) {         // the lanes of the first key hold every pair once
+      s_m[warp * KPW + grp][(own0 + j) % R] = m_ref[j];
+      s_l[warp * KPW + grp][(own0 + j) % R] = s;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    float M = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < DEC_WARPS * KPW; ++i) M = fmaxf(M, s_m[i][r]);
+    const float mine = s_m[warp * KPW + grp][r];
+    const float f = mine == -INFINITY ? 0.f : exp2f(mine - M);
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { x[2 * i] = o[r][i].x * f; x[2 * i + 1] = o[r][i].y * f; }
+#pragma unroll
+    for (int d = LPR; d < 32; d <<= 1)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] += __shfl_xor_sync(0xffffffffu, x[i], d);
+    if (grp == 0) {
+      *reinterpret_cast<float4*>(&s_o[warp][r][l * 8]) = make_float4(x[0], x[1], x[2], x[3]);
+      *reinterpret_cast<float4*>(&s_o[warp][r][l * 8 + 4]) = make_float4(x[4], x[5], x[6], x[7]);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < pairs * D; i += DEC_WARPS * 32) {
+    const int r = i / D, d = i % D;
+    float acc = 0.f;
+#pragma unroll
+    for (int w = 0; w < DEC_WARPS; ++w) acc += s_o[w][r][d];
+    const int64_t pidx = ((static_cast<int64_t>(b) * p.H + kvh * G + r % G) * p.Tq + r / G) * p.splits + split;
+    p.part_o[pidx * D + d] = acc;
+    if (d == 0) {
+      float M = -INFINITY, s = 0.f;
+      for (int w = 0; w < DEC_WARPS * KPW; ++w) M = fmaxf(M, s_m[w][r]);
+      for (int w = 0; w < DEC_WARPS * KPW; ++w) s += s_m[w][r] == -INFINITY ? 0.f : s_l[w][r] * exp2f(s_m[w][r] - M);
+      p.part_ml[pidx * 2] = M;
+      p.part_ml[pidx * 2 + 1] = s;
+    }
+  }
+}
+
+// out[b, row, h, :] = sum_s o_s 2^(m_s - M) / sum_s l_s 2^(m_s - M): one CTA per item, warps over the splits, a lane
+// owns D / 32 consecutive dims.  (One warp walking all splits in order took 8.7 us for 16 items of 32 splits.)
+constexpr int MERGE_WARPS = 4;
 template <int D>
-__global__ void __launch_bounds__(256) attn_small_q_merge_kernel(const float* __restrict__ part_o,
-                                                                 const float* __restrict__ part_ml, bf16* __restrict__ out,
-                                                                 int64_t items, int Tq, int H, int splits) {
-  const int lane = threadIdx.x & 31;
-  const int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);   // (b, h, row)
-  if (item >= items) return;
+__global__ void __launch_bounds__(MERGE_WARPS * 32) attn_small_q_merge_kernel(const float* __restrict__ part_o,
+                                                                              const float* __restrict__ part_ml,
+                                                                              bf16* __restrict__ out, int Tq, int H, int splits) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t item = blockIdx.x;                  // (b, h, row)
   constexpr int DPL = D / 32;
+  __shared__ float s_o[MERGE_WARPS][D], s_l[MERGE_WARPS];
+  const float2* ml = reinterpret_cast<const float2*>(part_ml) + item * splits;
   float M = -INFINITY;
-  for (int s = lane; s < splits; s += 32) M = fmaxf(M, part_ml[(item * splits + s) * 2]);
+  for (int s = lane; s < splits; s += 32) M = fmaxf(M, ml[s].x);
   M = warp_max(M);
   float o[DPL], l = 0.f;
 #pragma unroll
   for (int e = 0; e < DPL; ++e) o[e] = 0.f;
-  for (int s = 0; s < splits; ++s) {
-    const float m = part_ml[(item * splits + s) * 2];
-    if (m == -INFINITY) continue;
-    const float w = exp2f(m - M);
-    l = fmaf(part_ml[(item * splits + s) * 2 + 1], w, l);
+#pragma unroll 4
+  for (int s = warp; s < splits; s += MERGE_WARPS) {
+    const float2 t = ml[s];
+    const float* src = part_o + (item * splits + s) * D + lane * DPL;
+    float x[DPL];
 #pragma unroll
-    for (int e = 0; e < DPL; ++e) o[e] = fmaf(part_o[(item * splits + s) * D + lane * DPL + e], w, o[e]);
+    for (int e = 0; e < DPL; ++e) x[e] = src[e];
+    const bool some = t.x != -INFINITY;             // an empty split: its partial output counts for nothing
+    const float w = some ? exp2f(t.x - M) : 0.f;
+    l = fmaf(some ? t.y : 0.f, w, l);
+#pragma unroll
+    for (int e = 0; e < DPL; ++e) o[e] = fmaf(some ? x[e] : 0.f, w, o[e]);
   }
-  const float inv = l > 0.f ? 1.f / l : 0.f;
-  const int row = static_cast<int>(item % Tq);
-  const int64_t bh = item / Tq;
-  const int h = static_cast<int>(bh % H);
-  const int64_t b = bh / H;
-  bf16* dst = out + ((b * Tq + row) * H + h) * D + lane * DPL;
 #pragma unroll
-  for (int e = 0; e < DPL; ++e) dst[e] = __float2bfloat16(o[e] * inv);
+  for (int e = 0; e < DPL; ++e) s_o[warp][lane * DPL + e] = o[e];
+  if (lane == 0) s_l[warp] = l;
+  __syncthreads();
+  if (threadIdx.x < D) {
+    float acc = 0.f, tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < MERGE_WARPS; ++w) { acc += s_o[w][threadIdx.x]; tot += s_l[w]; }
+    const int row = static_cast<int>(item % Tq);
+    const int64_t bh = item / Tq, b = bh / H, h = bh % H;
+    out[((b * Tq + row) * H + h) * D + threadIdx.x] = __float2bfloat16(acc * (tot > 0.f ? 1.f / tot : 0.f));
+  }
+}
+
+template <int D>
+static int launch_merge(const SmallQParams& p, bf16* out, cudaStream_t stream) {
+  const int64_t items = static_cast<int64_t>(p.B) * p.H * p.Tq;
+  attn_small_q_merge_kernel<D><<<static_cast<unsigned>(items), MERGE_WARPS * 32, 0, stream>>>(p.part_o, p.part_ml, out, p.Tq,
+                                                                                            p.H, p.splits);
+  return static_cast<int>(cudaGetLastError());
+}
+
+template <int D>
+static int launch_decode(const SmallQParams& p, bf16* out, cudaStream_t stream) {
+  const int pairs = p.Tq * (p.H / p.HK);
+  const dim3 grid(p.splits, p.HK, p.B);
+  if (pairs <= 1) attn_decode_partial_kernel<D, 1><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
+  else if (pairs <= 2) attn_decode_partial_kernel<D, 2><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
+  else if (pairs <= 4) attn_decode_partial_kernel<D, 4><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
+  else attn_decode_partial_kernel<D, 8><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
+  TTCD_CUDA_CHECK(cudaGetLastError());
+  return launch_merge<D>(p, out, stream);
 }
 
 template <int D>
@@ -181,10 +421,7 @@ static int launch_small_q(const SmallQParams& p, bf16* out, cudaStream_t stream)
   }
   k1<<<dim3(p.splits, p.HK, p.B), SQ_WARPS * 32, S::TOTAL, stream>>>(p);
   TTCD_CUDA_CHECK(cudaGetLastError());
-  const int64_t items = static_cast<int64_t>(p.B) * p.H * p.Tq;
-  attn_small_q_merge_kernel<D><<<static_cast<unsigned>((items + 7) / 8), 256, 0, stream>>>(p.part_o, p.part_ml, out, items,
-                                                                                        p.Tq, p.H, p.splits);
-  return static_cast<int>(cudaGetLastError());
+  return launch_merge<D>(p, out, stream);
 }
 
 }  // namespace ttcd
@@ -194,22 +431,51 @@ static int launch_small_q(const SmallQParams& p, bf16* out, cudaStream_t stream)
 // [B, H, Tq, splits, 2] are caller-provided scratch; splits must equal ceil(Tk / 256).  window <= 0: unlimited.
 // kv_len (may be null): a device int holding how many of the Tk key rows are filled, read when the kernel runs, so
 // that a captured launch follows a cache that grows between replays; the causal alignment then counts from it.
-TTCD_EXPORT int ttcd_attn_small_q(const void* q, const void* k, const void* v, void* out, float* part_o, float* part_ml,
-                                  int B, int Tq, int Tk, int H, int HK, int D, long long ldq, long long ldk, long long ldv,
-                                  long long sq, long long sk, long long sv, int window, float scale, int splits,
-                                  const int* kv_len, void* stream_ptr) {
+static int small_q_params(ttcd::SmallQParams& p, const void* q, const void* k, const void* v, float* part_o, float* part_ml,
+                          int B, int Tq, int Tk, int H, int HK, int D, long long ldq, long long ldk, long long ldv,
+                          long long sq, long long sk, long long sv, int window, float scale, int splits, const int* kv_len) {
   using namespace ttcd;
   if (B <= 0 || Tq <= 0 || Tq >= 128 || Tk < Tq || H <= 0 || HK <= 0 || H % HK != 0 || (D != 64 && D != 128))
     return TTCD_ERR_ARG;
-  if (splits != (Tk + SQ_KEYS - 1) / SQ_KEYS || ldk % 8 != 0 || ldv % 8 != 0 || sk % 8 != 0 || sv % 8 != 0) return TTCD_ERR_ARG;
+  if (ldk % 8 != 0 || ldv % 8 != 0 || sk % 8 != 0 || sv % 8 != 0) return TTCD_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(k) & 15u) || (reinterpret_cast<uintptr_t>(v) & 15u)) return TTCD_ERR_ARG;
-  SmallQParams p;
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
   p.part_o = part_o; p.part_ml = part_ml; p.kv_len = kv_len;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.HK = HK; p.splits = splits; p.window = window;
   p.ldq = ldq; p.ldk = ldk; p.ldv = ldv; p.sq = sq; p.sk = sk; p.sv = sv;
   p.scale_log2 = scale * 1.4426950408889634f;
+  return TTCD_OK;
+}
+
+TTCD_EXPORT int ttcd_attn_small_q(const void* q, const void* k, const void* v, void* out, float* part_o, float* part_ml,
+                                  int B, int Tq, int Tk, int H, int HK, int D, long long ldq, long long ldk, long long ldv,
+                                  long long sq, long long sk, long long sv, int window, float scale, int splits,
+                                  const int* kv_len, void* stream_ptr) {
+  using namespace ttcd;
+  if (splits != (Tk + SQ_KEYS - 1) / SQ_KEYS) return TTCD_ERR_ARG;
+  SmallQParams p;
+  const int rc = small_q_params(p, q, k, v, part_o, part_ml, B, Tq, Tk, H, HK, D, ldq, ldk, ldv, sq, sk, sv, window, scale,
+                                splits, kv_len);
+  if (rc != TTCD_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return D == 128 ? launch_small_q<128>(p, static_cast<bf16*>(out), stream)
                   : launch_small_q<64>(p, static_cast<bf16*>(out), stream);
+}
+
+// The same call for at most 8 (query row, head of the group) pairs per key/value head: Tq * (H / HK) <= 8.  q rows are
+// 16-byte aligned too; splits is any number from 1 to 65535 (the kernel cuts the filled keys into that many ranges).
+TTCD_EXPORT int ttcd_attn_decode(const void* q, const void* k, const void* v, void* out, float* part_o, float* part_ml,
+                                 int B, int Tq, int Tk, int H, int HK, int D, long long ldq, long long ldk, long long ldv,
+                                 long long sq, long long sk, long long sv, int window, float scale, int splits,
+                                 const int* kv_len, void* stream_ptr) {
+  using namespace ttcd;
+  if (splits < 1 || splits > 65535 || B > 65535 || HK > 65535) return TTCD_ERR_ARG;
+  SmallQParams p;
+  const int rc = small_q_params(p, q, k, v, part_o, part_ml, B, Tq, Tk, H, HK, D, ldq, ldk, ldv, sq, sk, sv, window, scale,
+                                splits, kv_len);
+  if (rc != TTCD_OK) return rc;
+  if (Tq * (H / HK) > 8 || ldq % 8 != 0 || sq % 8 != 0 || (reinterpret_cast<uintptr_t>(q) & 15u)) return TTCD_ERR_ARG;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  return D == 128 ? launch_decode<128>(p, static_cast<bf16*>(out), stream)
+                  : launch_decode<64>(p, static_cast<bf16*>(out), stream);
 }

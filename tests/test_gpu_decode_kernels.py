@@ -1,0 +1,56 @@
+"""The decode step's kernels against float64: attention of a few (query row, head) pairs over a key/value cache (its pair
+counts, partly filled rings, windows, key counts around the sizes of a turn and of a split) and the products of up to 16 rows
+with a weight (row, column and K remainders)."""
+import pytest
+import torch
+
+from ttcd_b200.ops import cuda
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _attention64(q, k, v, window, n):
+    """q [B,Tq,H,D] at the end of the first n keys, bottom-right causal."""
+    B, Tq, H, D = q.shape
+    G = H // k.shape[2]
+    kf, vf = (t[:, :n].double().repeat_interleave(G, dim=2) for t in (k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), kf) * D ** -0.5
+    qpos = torch.arange(n - Tq, n, device=q.device)[:, None]
+    key = torch.arange(n, device=q.device)[None, :]
+    vis = (key <= qpos) if window is None else (key <= qpos) & (key > qpos - window)
+    return torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s.masked_fill(~vis, float("-inf")), -1), vf)
+
+
+@pytest.mark.parametrize("B,Tq,Tk,H,HK,D,W,filled", [
+    (1, 1, 1, 1, 1, 128, None, None), (2, 1, 127, 4, 4, 64, None, None), (1, 1, 128, 4, 2, 128, None, None),
+    (3, 1, 129, 6, 2, 64, 100, None), (1, 2, 2049, 8, 2, 128, 500, None), (1, 1, 8192, 16, 8, 128, None, 1501),
+    (5, 1, 640, 15, 5, 64, None, 1), (2, 8, 999, 2, 2, 128, 64, None), (1, 1, 70001, 2, 1, 64, None, None),
+    (2, 1, 300, 14, 2, 128, None, 299), (1, 2, 1000, 4, 1, 64, None, 257)])
+def test_decode_attention_against_float64(B, Tq, Tk, H, HK, D, W, filled):
+    assert Tq * (H // HK) <= 8
+    torch.manual_seed(Tk)
+    q, k, v = (torch.randn(B, t, h, D, device=DEV).bfloat16() for t, h in ((Tq, H), (Tk, HK), (Tk, HK)))
+    q = q * 2                                                # a sharper softmax: the running max moves
+    n = Tk if filled is None else filled
+    if filled is not None:                                   # rows past the fill count must not be read
+        k[:, n:], v[:, n:] = float("nan"), float("nan")
+    kv_len = None if filled is None else torch.tensor([n], dtype=torch.int32, device=DEV)
+    got = cuda.attn_small_q(q, k, v, W, None, kv_len).double()
+    want = _attention64(q, k, v, W, n)
+    # fp32 sums (scores up to ~40: absolute error below 1e-5, so is the probabilities' relative one) and one rounding to bf16
+    bound = want.abs() * 2.0 ** -8 + 1e-4
+    assert ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (1, 1024, 2048), (3, 129, 72), (8, 6144, 1024), (8, 1001, 3072), (9, 130, 264),
+                                   (16, 4096, 1024), (16, 20000, 520), (5, 151936, 1024)])
+def test_few_rows_times_weight_against_float64(M, N, K):
+    torch.manual_seed(N + K)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    w = (torch.randn(N, K, device=DEV) * K ** -0.5).bfloat16()
+    got = cuda.gemm(x, w.transpose(0, 1), alpha=0.5).double()
+    want = 0.5 * x.double() @ w.double().t()
+    # fp32 accumulation (K terms of size ~K^-1/2) and one rounding to bf16
+    bound = want.abs() * 2.0 ** -8 + 2.0 ** -22 * K ** 0.5
+    assert got.shape == (M, N) and ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())

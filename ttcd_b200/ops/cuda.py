@@ -811,14 +811,22 @@ def attn_small_q(q, k, v, window=None, scale=None, kv_len=None):
     q, ldq, sq = _attn_layout(q)
     k, ldk, sk = _attn_layout(k)
     v, ldv, sv = _attn_layout(v)
-    splits = -(-Tk // 256)                  # 256 keys per CTA; the partial results are merged by a second pass
+    few = Tq * (H // HK) <= 8               # a decode step: the register kernel, else 256 keys per CTA through shared memory
+    splits = _decode_splits(B * HK, Tk) if few else -(-Tk // 256)     # the partial results are merged by a second pass
     out = torch.empty(B, Tq, H, D, dtype=_BF16, device=q.device)
     part_o = torch.empty(B, H, Tq, splits, D, dtype=torch.float32, device=q.device)
     part_ml = torch.empty(B, H, Tq, splits, 2, dtype=torch.float32, device=q.device)
-    nv.call("ttcd_attn_small_q", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(out), nv.ptr(part_o), nv.ptr(part_ml), nv.i32(B),
-            nv.i32(Tq), nv.i32(Tk), nv.i32(H), nv.i32(HK), nv.i32(D), nv.i64(ldq), nv.i64(ldk), nv.i64(ldv), nv.i64(sq),
-            nv.i64(sk), nv.i64(sv), nv.i32(window or 0), nv.f32(scale), nv.i32(splits), nv.ptr(kv_len), nv.stream_ptr())
+    nv.call("ttcd_attn_decode" if few else "ttcd_attn_small_q", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(out), nv.ptr(part_o),
+            nv.ptr(part_ml), nv.i32(B), nv.i32(Tq), nv.i32(Tk), nv.i32(H), nv.i32(HK), nv.i32(D), nv.i64(ldq), nv.i64(ldk),
+            nv.i64(ldv), nv.i64(sq), nv.i64(sk), nv.i64(sv), nv.i32(window or 0), nv.f32(scale), nv.i32(splits),
+            nv.ptr(kv_len), nv.stream_ptr())
     return out
+
+
+def _decode_splits(heads: int, Tk: int, sms: int = 148) -> int:
+    """Key ranges per (sample, key/value head) of a decode step: two CTAs per SM in one wave, but no range shorter than
+    the 128 keys that a CTA takes per turn."""
+    return max(1, min(-(-Tk // 128), 2 * sms // heads))
 
 
 def lse_merge(o_a, lse_a, o_b, lse_b):
