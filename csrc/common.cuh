@@ -45,6 +45,9 @@ static __device__ unsigned long long g_wait_ns = TTCD_WAIT_NS;
 int make_tmap_bf16_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t batch,
                       uint64_t row_stride_elems, uint64_t batch_stride_elems, uint32_t box_inner,
                       uint32_t box_rows);
+// The same for fp32: inner box 32 elements (128 bytes), strides multiples of 4 elements.
+int make_tmap_f32_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t batch,
+                     uint64_t row_stride_elems, uint64_t batch_stride_elems, uint32_t box_inner, uint32_t box_rows);
 int sm_count();
 
 #ifdef __CUDACC__
@@ -183,6 +186,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const CUtensorMap
 }
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src_smem, int x, int y, int z) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(src_smem), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
+// The tile is added to the tensor in memory (fp32: one round-to-nearest add per element, done by the L2).
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32_t src_smem, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(map)),
                "r"(src_smem), "r"(x), "r"(y), "r"(z)
                : "memory");

@@ -893,23 +893,26 @@ def cross_entropy(logits, labels, ignore_index=-100, label_smoothing=0.0, z_loss
 
 
 def _lce_chunk_rows(n_rows: int, hidden: int, num_chunks: int, sms: int = 148) -> int:
-    """Rows per chunk of the chunked lm_head pass: about ``n_rows / num_chunks``, moved (by up to a quarter either way)
-    to the multiple of 128 whose dx GEMM ([rows, vocab] x [vocab, hidden]: rows/128 x hidden/256 output tiles, the only
-    one of the three GEMMs with few tiles) fills whole waves of the persistent kernel's CTAs; 8192 rows x 1024 would be
-    256 tiles = 1.73 waves, 9472 rows are 296 tiles = 2 waves."""
-    target = max(1, -(-n_rows // max(1, num_chunks)) // 128)
+    """Rows per chunk of the chunked lm_head pass: about ``n_rows / num_chunks`` (a quarter either way), but up to 2560
+    where that is less, whichever the two gradient GEMMs finish soonest with.  Their cost per vocabulary entry, at the
+    measured GEMM and copy rates: dx ([rows, vocab] x [vocab, hidden]) has only rows/128 x hidden/256 output tiles, so it
+    costs whole waves of the persistent kernel's CTAs; dW runs rows x hidden products but at least the time in which its
+    fp32 accumulator is read and written once.  (5003 rows, hidden 2048, vocabulary 128256: eight chunks of 640 rows leave
+    108 of 148 SMs idle in every dx and pass over the 1 GB accumulator eight times; three chunks of at most 2304 do not.)"""
     total = -(-n_rows // 128)
-    if target >= total:
+    target = max(1, -(-n_rows // max(1, num_chunks)) // 128)
+    hi = max(target + target // 4, 20)
+    if hi >= total and target >= total:
         return total * 128
     n_tiles = max(1, -(-hidden // 256))
-    best, best_key = target, None
-    for m in range(max(1, target - target // 4), min(total, target + target // 4) + 1):
-        tiles = m * n_tiles
-        eff = tiles / (-(-tiles // sms) * sms)
-        key = (round(eff, 2), -abs(m - target))
-        if best_key is None or key > best_key:
-            best, best_key = m, key
-    return best * 128
+
+    def cost(m: int) -> float:
+        sizes = [m] * (total // m) + ([total % m] if total % m else [])
+        waves = sum(-(-s * n_tiles // sms) for s in sizes)
+        return waves * 5.8e-9 + sum(max(s * 128 * hidden * 1.2e-15, hidden * 1.25e-12) for s in sizes)
+
+    candidates = range(max(1, target - target // 4), min(total, hi) + 1)
+    return 128 * min(candidates, key=lambda m: (round(cost(m), 10), abs(m - target)))
 
 
 class _LinearCrossEntropy(torch.autograd.Function):
@@ -928,7 +931,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         need_grad = hidden.requires_grad or weight.requires_grad
         chunk = _lce_chunk_rows(N, Hd, num_chunks)
         dx = torch.empty_like(hidden) if need_grad else None
-        dw = torch.zeros(V, Hd, dtype=torch.float32, device=hidden.device) if need_grad else None
+        dw = torch.empty(V, Hd, dtype=torch.float32, device=hidden.device) if need_grad else None
         loss = torch.zeros((), dtype=torch.float32, device=hidden.device)
         logits = torch.empty(min(chunk + 127, N), V, dtype=_BF16, device=hidden.device)
         # the row statistics come out of the logits GEMM's epilogue (the l2-warp term needs the arg-max: row pass)
@@ -950,8 +953,9 @@ class _LinearCrossEntropy(torch.autograd.Function):
             loss = loss + loss_rows.sum()
             if need_grad:
                 gemm(lg, w, out=dx[s:e].view(1, e - s, Hd))
-                gemm(lg.transpose(0, 1), hidden[s:e], out=dw.view(1, V, Hd), out_dtype=torch.float32, beta=1.0,
-                     c_in=dw.view(1, V, Hd))
+                first = s == 0                 # writes the accumulator, the others add to it
+                gemm(lg.transpose(0, 1), hidden[s:e], out=dw.view(1, V, Hd), out_dtype=torch.float32,
+                     beta=0.0 if first else 1.0, c_in=None if first else dw.view(1, V, Hd))
         if need_grad:
             ctx.save_for_backward(dx, dw.to(weight.dtype))
         return (loss * inv_total).reshape(())
