@@ -32,14 +32,16 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
 // l2_factor > 0 adds the l2-warp term on EVERY row (ignored ones too, as the reference's fused linear-CE does,
 // fla/modules/fused_linear_cross_entropy.py:250-283): max logit * l2_factor * (*grad_scale) at the arg-max column
 // (the lowest column on ties); the loss value is unchanged by it.
-__global__ void __launch_bounds__(1024) ce_rows_kernel(bf16* __restrict__ logits, const int64_t* __restrict__ labels,
+// The gradient goes to `grad` (rows ld apart like the logits; it may be `logits` itself).
+__global__ void __launch_bounds__(1024) ce_rows_kernel(const bf16* logits, bf16* grad, const int64_t* __restrict__ labels,
                                                        float* __restrict__ loss_row, float* __restrict__ lse_row,
                                                        const float* __restrict__ grad_scale, int V, int64_t ld,
                                                        int ignore_index, int write_grad, float eps, float zeta,
                                                        float l2_factor, const float2* __restrict__ lse_part, int n_parts) {
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
-  bf16* lr = logits + row * ld;
+  const bf16* lr = logits + row * ld;
+  bf16* gr = grad + row * ld;
   const int64_t label = labels[row];
   const int nvec = V / 8;
   float m = -INFINITY, s = 0.f, sumx = 0.f;
@@ -124,11 +126,11 @@ __global__ void __launch_bounds__(1024) ce_rows_kernel(bf16* __restrict__ logits
       w[k] = pack_bf16(t.x, t.y);
     }
     raw.x = w[0]; raw.y = w[1]; raw.z = w[2]; raw.w = w[3];
-    *reinterpret_cast<uint4*>(lr + i * 8) = raw;
+    *reinterpret_cast<uint4*>(gr + i * 8) = raw;
   }
   for (int i = nvec * 8 + threadIdx.x; i < V; i += blockDim.x) {
     const float f = __bfloat162float(lr[i]);
-    lr[i] = __float2bfloat16((__expf(f - lse) * pw - (i == label ? hot : 0.f) - flat) * scale + (i == arg_col ? warp_term : 0.f));
+    gr[i] = __float2bfloat16((__expf(f - lse) * pw - (i == label ? hot : 0.f) - flat) * scale + (i == arg_col ? warp_term : 0.f));
   }
 }
 
@@ -223,6 +225,20 @@ __global__ void __launch_bounds__(256) cast_scale_kernel(const TI* __restrict__ 
   }
 }
 
+// y = x * (*factor): a gradient times the scalar that arrives from downstream, 16 bytes per access (the broadcast
+// multiplication of the library ran at 1.9 TB/s on the 2.1 GB of a 32768 x 32000 logits gradient).
+__global__ void __launch_bounds__(256) scale_by_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
+                                                       const float* __restrict__ factor, int64_t nvec) {
+  const float f = *factor;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < nvec;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const uint4 raw = reinterpret_cast<const uint4*>(x)[i];
+    const float2 a = unpack_bf16(raw.x), b = unpack_bf16(raw.y), c = unpack_bf16(raw.z), d = unpack_bf16(raw.w);
+    reinterpret_cast<uint4*>(y)[i] = make_uint4(pack_bf16(a.x * f, a.y * f), pack_bf16(b.x * f, b.y * f),
+                                                pack_bf16(c.x * f, c.y * f), pack_bf16(d.x * f, d.y * f));
+  }
+}
+
 }  // namespace ttcd
 
 using namespace ttcd;
@@ -231,18 +247,18 @@ static unsigned flat_grid(long long n) {
   return static_cast<unsigned>(std::max<long long>(1, std::min<long long>((n + 255) / 256, 148LL * 16)));
 }
 
-// logits: [rows][ld] bf16 (modified in place when write_grad); labels: int64 [rows].
+// logits: [rows][ld] bf16; labels: int64 [rows]; grad (used when write_grad): [rows][ld] bf16, may be logits.
 // lse_part (may be null): fp32 [rows][n_parts][2] left by ttcd_gemm_bf16_lse for these logits; the first pass over the
 // row is then skipped (not with label smoothing or the l2-warp term, which need the row's mean / arg-max).
-TTCD_EXPORT int ttcd_ce_rows(void* logits, const long long* labels, float* loss_row, float* lse_row,
+TTCD_EXPORT int ttcd_ce_rows(const void* logits, void* grad, const long long* labels, float* loss_row, float* lse_row,
                              const float* grad_scale, long long rows, int V, long long ld, int ignore_index,
                              int write_grad, float label_smoothing, float lse_square_scale, float l2_factor,
                              const float* lse_part, int n_parts, void* stream_ptr) {
-  if (rows <= 0 || V <= 0 || ld % 8 != 0 || (write_grad && grad_scale == nullptr)) return TTCD_ERR_ARG;
+  if (rows <= 0 || V <= 0 || ld % 8 != 0 || (write_grad && (grad_scale == nullptr || grad == nullptr))) return TTCD_ERR_ARG;
   if (label_smoothing < 0.f || label_smoothing >= 1.f || V >= (1 << 24)) return TTCD_ERR_ARG;
   if (lse_part != nullptr && (n_parts <= 0 || label_smoothing != 0.f || l2_factor != 0.f)) return TTCD_ERR_ARG;
   ce_rows_kernel<<<static_cast<unsigned>(rows), 1024, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
-      static_cast<bf16*>(logits), reinterpret_cast<const int64_t*>(labels), loss_row, lse_row, grad_scale, V, ld,
+      static_cast<const bf16*>(logits), static_cast<bf16*>(grad), reinterpret_cast<const int64_t*>(labels), loss_row, lse_row, grad_scale, V, ld,
       ignore_index, write_grad, label_smoothing, lse_square_scale, l2_factor, reinterpret_cast<const float2*>(lse_part),
       n_parts);
   return static_cast<int>(cudaGetLastError());
@@ -292,5 +308,15 @@ TTCD_EXPORT int ttcd_cast_scale(const void* x, void* y, long long n, float scale
     case 3: cast_scale_kernel<bf16, bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(x), static_cast<bf16*>(y), n, scale, accumulate); break;
     default: return TTCD_ERR_ARG;
   }
+  return static_cast<int>(cudaGetLastError());
+}
+
+// y[i] = x[i] * (*factor), bf16, n a multiple of 8, x and y 16-byte aligned; factor: one fp32 on the device.
+TTCD_EXPORT int ttcd_scale_by(const void* x, void* y, const float* factor, long long n, void* stream_ptr) {
+  if (n <= 0) return TTCD_OK;
+  if (n % 8 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u)) return TTCD_ERR_ARG;
+  const long long blocks = std::min<long long>((n / 8 + 255) / 256, 148LL * 32);
+  scale_by_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
+      static_cast<const bf16*>(x), static_cast<bf16*>(y), factor, n / 8);
   return static_cast<int>(cudaGetLastError());
 }

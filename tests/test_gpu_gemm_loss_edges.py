@@ -1,0 +1,65 @@
+"""fp32 outputs of the GEMM (stored and added in place) at tile edges, the chunking of the linear cross-entropy, and the
+cross-entropy's gradient next to untouched logits."""
+import pytest
+import torch
+
+from ttcd_b200.ops import cuda
+
+DEV = "cuda:0"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,batch", [(128, 128, 64, 1), (129, 132, 72, 1), (300, 260, 136, 3), (1000, 516, 640, 1), (128, 1028, 64, 2)])
+@pytest.mark.parametrize("a_t,b_t", [(False, True), (True, False)])
+def test_fp32_output_and_accumulation(M, N, K, batch, a_t, b_t):
+    torch.manual_seed(M + N)
+    pad = lambda n: -(-n // 8) * 8                                                     # noqa: E731  (operand rows: 16 bytes)
+    a = torch.randn(batch, K, pad(M), device=DEV).bfloat16()[..., :M].transpose(-1, -2) if a_t else torch.randn(batch, M, pad(K), device=DEV).bfloat16()[..., :K]
+    b = torch.randn(batch, N, pad(K), device=DEV).bfloat16()[..., :K].transpose(-1, -2) if b_t else torch.randn(batch, K, pad(N), device=DEV).bfloat16()[..., :N]
+    want = a.double() @ b.double()
+    guard = torch.full((batch + 1, M, N), 7.0, device=DEV)                             # what lies behind the output stays
+    out = guard[:batch]
+    cuda.gemm(a, b, out_dtype=torch.float32, out=out)
+    bound = 2.0 ** -20 * K                                                             # K products of size ~1 summed in fp32
+    assert (out.double() - want).abs().max() <= bound
+    cuda.gemm(a, b, out_dtype=torch.float32, out=out, beta=1.0, c_in=out, alpha=0.5)
+    assert (out.double() - 1.5 * want).abs().max() <= 2 * bound
+    other = torch.randn_like(out)
+    sep = torch.empty_like(out)
+    cuda.gemm(a, b, out_dtype=torch.float32, out=sep, beta=2.0, c_in=other)            # another addend: the reading epilogue
+    assert (sep.double() - (want + 2 * other.double())).abs().max() <= 2 * bound
+    assert (guard[batch] == 7.0).all()
+
+
+@pytest.mark.parametrize("n,hidden,chunks", [(128, 64, 8), (600, 1024, 8), (5003, 2048, 8), (65536, 1024, 8), (65536, 960, 32), (2560, 2048, 1),
+                                             (24000, 4096, 8), (1, 1024, 8)])
+def test_lm_head_chunks_cover_the_rows_and_stay_bounded(n, hidden, chunks):
+    rows = cuda._lce_chunk_rows(n, hidden, chunks)
+    assert rows % 128 == 0 and rows > 0
+    assert rows <= max(-(-n // 128) * 128 if chunks == 1 or n <= 2560 else 0, 2560, int(1.25 * n / chunks) + 128)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,vocab,offset", [(3, 1000, 0), (130, 128, 0), (7, 4096, 8), (5, 1000, 4)])
+@pytest.mark.parametrize("smoothing,z", [(0.0, 0.0), (0.1, 1e-3)])
+def test_cross_entropy_gradient_beside_the_logits(rows, vocab, offset, smoothing, z):
+    torch.manual_seed(rows)
+    store = (3 * torch.randn(rows * vocab + offset, device=DEV)).bfloat16()
+    leaf = store.requires_grad_()
+    logits = leaf[offset:].view(rows, vocab)                # offset 4: 8-byte aligned only
+    labels = torch.randint(0, vocab, (rows,), device=DEV)
+    labels[0] = -100
+    kept = logits.detach().clone()
+    loss = cuda.cross_entropy(logits, labels, label_smoothing=smoothing, z_loss=z)
+    grads = [torch.autograd.grad(loss * s, leaf, retain_graph=True)[0][offset:].view(rows, vocab).double() for s in (1.0, 3.0, 1.0)]
+    assert torch.equal(logits, kept) and torch.equal(grads[0], grads[2])
+    x = kept.double().requires_grad_()
+    lse = torch.logsumexp(x, -1)
+    valid = labels != -100
+    per = lse - (1 - smoothing) * x.gather(1, labels.clamp_min(0)[:, None])[:, 0] - smoothing * x.mean(-1) + z * lse ** 2
+    want_loss = (per * valid).sum() / valid.sum()
+    (want,) = torch.autograd.grad(want_loss, x)
+    assert abs(float(loss) - float(want_loss)) < 1e-4 * abs(float(want_loss))
+    # one rounding to bf16 of values whose exponentials carry a few fp32 roundings; scaled by 3: one more
+    assert ((grads[0] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
+    assert ((grads[1] - 3 * want).abs() <= 2.0 ** -7 * 3 * want.abs() + 1e-6).all()

@@ -842,11 +842,13 @@ def lse_merge(o_a, lse_a, o_b, lse_b):
 # losses
 # =============================================================================================
 
-def _ce_rows(logits2, labels, inv_total, ignore_index, write_grad, smoothing=0.0, z_scale=0.0, l2_factor=0.0, lse_part=None):
-    """``lse_part`` [rows, tiles, 2] (from ``_logits_with_lse``): the kernel merges it instead of a first pass over the row."""
+def _ce_rows(logits2, labels, inv_total, ignore_index, write_grad, smoothing=0.0, z_scale=0.0, l2_factor=0.0, lse_part=None,
+             grad=None):
+    """``lse_part`` [rows, tiles, 2] (from ``_logits_with_lse``): the kernel merges it instead of a first pass over the row.
+    The gradient goes to ``grad`` (strides of the logits), without one into the logits themselves."""
     rows, V = logits2.shape
     loss_rows = torch.empty(rows, dtype=torch.float32, device=logits2.device)
-    nv.call("ttcd_ce_rows", nv.ptr(logits2), nv.ptr(labels), nv.ptr(loss_rows), nv.ptr(None), nv.ptr(inv_total),
+    nv.call("ttcd_ce_rows", nv.ptr(logits2), nv.ptr(logits2 if grad is None else grad), nv.ptr(labels), nv.ptr(loss_rows), nv.ptr(None), nv.ptr(inv_total),
             nv.i64(rows), nv.i32(V), nv.i64(logits2.stride(0)), nv.i32(ignore_index), nv.i32(1 if write_grad else 0),
             nv.f32(smoothing), nv.f32(z_scale), nv.f32(l2_factor), nv.ptr(lse_part),
             nv.i32(0 if lse_part is None else lse_part.shape[1]), nv.stream_ptr())
@@ -867,25 +869,28 @@ def _logits_with_lse(hidden2, w, out):
 
 
 class _CrossEntropy(torch.autograd.Function):
-    """Mean CE over valid rows; the gradient is computed in the forward, in place on a copy."""
+    """Mean CE over valid rows; the gradient (for a loss gradient of one) is computed in the forward."""
 
     @staticmethod
     def forward(ctx, logits, labels, ignore_index, smoothing=0.0, z_scale=0.0):
-        lg = logits.contiguous().clone() if logits.requires_grad else logits.contiguous()
+        lg = logits.contiguous()
+        if lg.data_ptr() % 16:                               # 16-byte accesses
+            lg = lg.clone()
         if lg.stride(0) % 8:
             raise ValueError("vocab size must be a multiple of 8 for the CE kernel")
         labels = labels.contiguous().to(torch.int64)
         total = labels.ne(ignore_index).sum().clamp_min(1).to(torch.float32)
         inv_total = (1.0 / total).reshape(1)
-        loss_rows = _ce_rows(lg, labels, inv_total, ignore_index, logits.requires_grad, smoothing, z_scale)
-        if logits.requires_grad:
-            ctx.save_for_backward(lg)
+        grad = torch.empty_like(lg) if logits.requires_grad else None
+        loss_rows = _ce_rows(lg, labels, inv_total, ignore_index, grad is not None, smoothing, z_scale, grad=grad)
+        if grad is not None:
+            ctx.save_for_backward(grad)
         return (loss_rows.sum() * inv_total).reshape(())
 
     @staticmethod
     def backward(ctx, g):
         (dlogits,) = ctx.saved_tensors
-        return dlogits * g.to(dlogits.dtype), None, None, None, None
+        return _scale_by(dlogits, g), None, None, None, None
 
 
 def cross_entropy(logits, labels, ignore_index=-100, label_smoothing=0.0, z_loss=0.0):
@@ -900,6 +905,15 @@ def _lce_chunk_rows(n_rows: int, hidden: int, num_chunks: int, sms: int = 148) -
     fp32 accumulator is read and written once.  (5003 rows, hidden 2048, vocabulary 128256: eight chunks of 640 rows leave
     108 of 148 SMs idle in every dx and pass over the 1 GB accumulator eight times; three chunks of at most 2304 do not.)"""
     total = -(-n_rows // 128)
+def _scale_by(t: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    """t * g for a gradient held since the forward and the scalar that arrives from downstream (on the device)."""
+    if t.dtype != _BF16 or not t.is_contiguous() or t.numel() % 8 or t.data_ptr() % 16:
+        return t * g.to(t.dtype)
+    out = torch.empty_like(t)
+    nv.call("ttcd_scale_by", nv.ptr(t), nv.ptr(out), nv.ptr(g.float().contiguous()), nv.i64(t.numel()), nv.stream_ptr())
+    return out
+
+
     target = max(1, -(-n_rows // max(1, num_chunks)) // 128)
     hi = max(target + target // 4, 20)
     if hi >= total and target >= total:
@@ -963,7 +977,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         dx, dw = ctx.saved_tensors
-        return dx * g.to(dx.dtype), None, dw * g.to(dw.dtype), None, None, None
+        return _scale_by(dx, g), None, _scale_by(dw, g), None, None, None
 
 
 def linear_cross_entropy(hidden, labels, weight, ignore_index=-100, num_chunks=8, l2_penalty=0.0):
