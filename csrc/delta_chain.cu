@@ -1,5 +1,5 @@
 // The chunk-to-chunk chain of the (gated) delta rule (sm_100a; the two products of a step, 64 x D x 32 each, run on the
-// tensor cores as TF32 mma.sync tiles with fp32 accumulation: they are far too small for a tcgen05 pipeline; the point
+// tensor cores as bf16 mma.sync tiles with fp32 accumulation: they are far too small for a tcgen05 pipeline; the point
 // of the kernel is to run the n dependent steps in ONE launch with the state resident in registers).
 //
 // For one (batch, head) pair, S [D, Dv] the running state and i the chunk index:
@@ -15,8 +15,8 @@
 // b_i [64, D] (bf16) in shared memory with asynchronous 16-byte copies that overlap the publication of S.  S [D, columns]
 // lives in the accumulator registers of the second product (D / 32 m16n8 tiles per warp) across chunks, in fp32, and is
 // mirrored in shared memory, rounded to bf16, as the B operand of the first; y is rounded the same way for the second.
-// Every operand of a product is thus a bf16 value (an exact TF32 operand after a 16-bit shift; the precision the
-// reference's Triton kernels multiply at), the sums and the state stay fp32, and two CTAs fit an SM at every D.
+// Every operand of a product is thus a bf16 value (the precision the reference's Triton kernels multiply at) and comes to
+// the products by ldmatrix, the sums and the state stay fp32.
 // The only asynchronous copies are the CTA's own cp.async groups (waited for with wait_group); nothing here waits on
 // another CTA, so nothing can spin.
 #include "common.cuh"
@@ -27,7 +27,7 @@ constexpr int DC_C = 64;         // rows of a chunk
 constexpr int DC_THREADS = 256;  // 8 warps
 
 struct DeltaChainParams {
-  const bf16* a; const bf16* b;   // bf16: exact TF32 operands after a 16-bit shift, half the staging traffic
+  const bf16* a; const bf16* b;
   const float* gamma; const float* x; const float* add; const float* s_init;
   float* y; float* states; float* s_last;
   int n, D, Dv;
@@ -38,34 +38,54 @@ struct DeltaChainParams {
   const float* dot_with; float* dot_out;
 };
 
-__device__ __forceinline__ uint32_t dc_bf16_bits(const bf16* p) {   // a bf16 value as a TF32 operand
-  return static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(p)) << 16;
+__device__ __forceinline__ void dc_cp_async16(uint32_t dst_smem, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
 }
-__device__ __forceinline__ void dc_cp_async16(void* dst_smem, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void dc_cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
+__device__ __forceinline__ void dc_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void dc_cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void dc_ldm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void dc_ldm4t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void dc_ldm2t(uint32_t& r0, uint32_t& r1, uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr) : "memory");
+}
+// B fragments of N8 n-tiles (k x n stored row-wise, `addr` = the lane's address of the first pair) against one A fragment
+template <int N8>
+__device__ __forceinline__ void dc_load_b(uint32_t (&b)[N8][2], uint32_t addr) {
+#pragma unroll
+  for (int t = 0; t + 1 < N8; t += 2) {
+    uint32_t r[4];
+    dc_ldm4t(r, addr + 16 * t);
+    b[t][0] = r[0]; b[t][1] = r[1]; b[t + 1][0] = r[2]; b[t + 1][1] = r[3];
+  }
+  if constexpr (N8 % 2 != 0) dc_ldm2t(b[N8 - 1][0], b[N8 - 1][1], addr + 16 * (N8 - 1));
+}
 
-template <int D, int DC_COLS>
-__global__ void __launch_bounds__(DC_THREADS, (D <= 128 ? 4 : 2)) delta_chain_kernel(const DeltaChainParams p) {
-  constexpr int LDT = D + 8;                 // bf16 row stride of the a_i / b_i tiles: rows 4 banks apart, 16-byte rows
-  constexpr int DC_LDS = DC_COLS + 8;        // bf16 row stride of the [*, columns] tiles read column-wise as B operands
+// PIPE: the a / b tiles of the next step travel while this one is computed (two stages of shared memory, fewer CTAs per SM)
+template <int D, int DC_COLS, bool PIPE>
+__global__ void __launch_bounds__(DC_THREADS, (PIPE ? (D <= 128 ? 2 : 1) : (D <= 128 ? 4 : 2)))
+delta_chain_kernel(const DeltaChainParams p) {
+  constexpr int LDT = D + 8;                 // bf16 row stride of the a_i / b_i tiles: 16-byte rows, 4 banks apart (ldmatrix)
+  constexpr int DC_LDS = DC_COLS + 8;        // bf16 row stride of the [*, columns] tiles read as B operands
   constexpr int NTM = DC_COLS / 8;           // n-tiles per m-tile of S
   constexpr int TPW = (D / 16) * NTM / 8;    // m16n8 tiles of S per warp: tile id = warp * TPW + x -> (id / NTM, id % NTM)
   constexpr int NT = TPW >= NTM ? NTM : TPW; // ... of which NT share an m-tile
   constexpr int MT = TPW / NT;
   constexpr int YT = DC_COLS / 16;           // n-tiles of y per warp
+  constexpr int STAGE = 2 * DC_C * LDT;      // bf16 of one (a, b) stage
   extern __shared__ __align__(16) float dc_smem[];
-  bf16* As = reinterpret_cast<bf16*>(dc_smem);              // [64][LDT]
-  bf16* Bs = As + DC_C * LDT;                               // [64][LDT]
-  bf16* Ss = Bs + DC_C * LDT;                               // [D][columns + 8]   S as the B operand of a S
+  bf16* stages = reinterpret_cast<bf16*>(dc_smem);          // [1 or 2][a | b][64][LDT]
+  bf16* Ss = stages + (PIPE ? 2 : 1) * STAGE;               // [D][columns + 8]   S as the B operand of a S
   bf16* Ys = Ss + D * DC_LDS;                               // [64][columns + 8]  sign_b * y as the B operand of b^T y
   float* red = reinterpret_cast<float*>(Ys + DC_C * DC_LDS);    // [8] per-warp partial sums of the optional dot product
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
@@ -83,6 +103,38 @@ __global__ void __launch_bounds__(DC_THREADS, (D <= 128 ? 4 : 2)) delta_chain_ke
   const int mt0 = (warp * TPW) / NTM, nt0 = (warp * TPW) % NTM;
   // the warp's YT tiles of y: m-tile warp / 2, n-tiles YT (warp % 2) ..
   const int ymt = warp >> 1, ynt0 = YT * (warp & 1);
+  // ldmatrix: which 8 x 8 matrix a lane addresses
+  const int l8 = lane & 7, hi8 = 8 * ((lane >> 3) & 1), hi16 = 8 * (lane >> 4);
+  const uint32_t st_addr = smem_u32(stages), ss_addr = smem_u32(Ss), ys_addr = smem_u32(Ys);
+  const uint32_t a_off = 2u * ((16 * ymt + l8 + hi8) * LDT + hi16);                      // a as A (row-wise)
+  const uint32_t sb_addr = ss_addr + 2u * ((l8 + hi8) * DC_LDS + 8 * ynt0 + hi16);       // S as B
+  const uint32_t b_off = 2u * (DC_C * LDT + (l8 + hi16) * LDT + 16 * mt0 + hi8);         // b^T as A (transposed on load)
+  const uint32_t yb_addr = ys_addr + 2u * ((l8 + hi8) * DC_LDS + 8 * nt0 + hi16);        // y as B
+
+  auto load_stage = [&](int step) {
+    const int i = p.reverse ? p.n - 1 - step : step;
+    const uint4* ga = reinterpret_cast<const uint4*>(a_base + static_cast<int64_t>(i) * DC_C * D);
+    const uint4* gb = reinterpret_cast<const uint4*>(b_base + static_cast<int64_t>(i) * DC_C * D);
+    const uint32_t dst = st_addr + (PIPE ? (step & 1) * 2u * STAGE : 0u);
+#pragma unroll 4
+    for (int v = threadIdx.x; v < DC_C * D / 8; v += DC_THREADS) {
+      const uint32_t at = dst + 2u * ((v / (D / 8)) * LDT + (v % (D / 8)) * 8);
+      dc_cp_async16(at, ga + v);
+      dc_cp_async16(at + 2u * DC_C * LDT, gb + v);
+    }
+    dc_cp_async_commit();
+  };
+  float2 xv[YT][2];                          // x of the next step's y tiles, in flight
+  auto load_x = [&](int step) {
+    const int i = p.reverse ? p.n - 1 - step : step;
+#pragma unroll
+    for (int t = 0; t < YT; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        xv[t][h] = *reinterpret_cast<const float2*>(
+            x_base + (static_cast<int64_t>(i) * DC_C + 16 * ymt + g + 8 * h) * Dv + 8 * (ynt0 + t) + 2 * c);
+  };
+  if (PIPE) load_stage(0);
 
   float s[MT][NT][4];
 #pragma unroll
@@ -94,17 +146,12 @@ __global__ void __launch_bounds__(DC_THREADS, (D <= 128 ? 4 : 2)) delta_chain_ke
       const float2 hi = *reinterpret_cast<const float2*>(p.s_init + (bh * D + row + 8) * Dv + col0 + col);
       s[m][t][0] = lo.x; s[m][t][1] = lo.y; s[m][t][2] = hi.x; s[m][t][3] = hi.y;
     }
+  load_x(0);
 
   for (int step = 0; step < p.n; ++step) {
     const int i = p.reverse ? p.n - 1 - step : step;
-    // ---- stage a_i, b_i; publish S (to shared memory for the y products, to global memory as states[i])
-    const uint4* ga = reinterpret_cast<const uint4*>(a_base + static_cast<int64_t>(i) * DC_C * D);
-    const uint4* gb = reinterpret_cast<const uint4*>(b_base + static_cast<int64_t>(i) * DC_C * D);
-    for (int v = threadIdx.x; v < DC_C * D / 8; v += DC_THREADS) {
-      const int row = v / (D / 8), c8 = (v % (D / 8)) * 8;
-      dc_cp_async16(As + row * LDT + c8, ga + v);
-      dc_cp_async16(Bs + row * LDT + c8, gb + v);
-    }
+    if (!PIPE) load_stage(step);
+    // ---- publish S (to shared memory for the y products, to global memory as states[i])
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -116,46 +163,37 @@ __global__ void __launch_bounds__(DC_THREADS, (D <= 128 ? 4 : 2)) delta_chain_ke
         *reinterpret_cast<float2*>(st_base + (static_cast<int64_t>(i) * D + row) * Dv + col) = lo;
         *reinterpret_cast<float2*>(st_base + (static_cast<int64_t>(i) * D + row + 8) * Dv + col) = hi;
       }
-    if (dot_base != nullptr) {
-      float part = 0.f;
+    dc_cp_async_wait_all();
+    __syncthreads();
+    if (PIPE && step + 1 < p.n) load_stage(step + 1);        // the other stage was last read before this barrier
+    const float gm = p.gamma[bh * p.n + i];
+    // a tile of the warp's elements of a [D, Dv] tensor of step i: with PIPE issued a product before its use
+    float ld[MT][NT][4];
+    auto load_tile = [&](const float* base) {
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
           const int row = 16 * (mt0 + m) + g, col = 8 * (nt0 + t) + 2 * c;
-          const float2 lo = *reinterpret_cast<const float2*>(dot_base + (static_cast<int64_t>(i) * D + row) * Dv + col);
-          const float2 hi = *reinterpret_cast<const float2*>(dot_base + (static_cast<int64_t>(i) * D + row + 8) * Dv + col);
-          part += s[m][t][0] * lo.x + s[m][t][1] * lo.y + s[m][t][2] * hi.x + s[m][t][3] * hi.y;
+          const float2 lo = *reinterpret_cast<const float2*>(base + (static_cast<int64_t>(i) * D + row) * Dv + col);
+          const float2 hi = *reinterpret_cast<const float2*>(base + (static_cast<int64_t>(i) * D + row + 8) * Dv + col);
+          ld[m][t][0] = lo.x; ld[m][t][1] = lo.y; ld[m][t][2] = hi.x; ld[m][t][3] = hi.y;
         }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      if (lane == 0) red[warp] = part;
-    }
-    dc_cp_async_wait_all();
-    __syncthreads();
-    if (dot_base != nullptr && threadIdx.x == 0) {
-      float tot = 0.f;
-#pragma unroll
-      for (int wv = 0; wv < DC_THREADS / 32; ++wv) tot += red[wv];
-      p.dot_out[(bh * p.n + i) * (Dv / 32) + blockIdx.x] = tot;        // rows of Dv / 32 slots (zero-filled by the caller)
-    }
+    };
+    if (PIPE && dot_base != nullptr) load_tile(dot_base);
     // ---- y = x + sign_a * (a S): the warp's YT 16 x 8 tiles
+    const uint32_t stage = st_addr + (PIPE ? (step & 1) * 2u * STAGE : 0u);
     {
       float acc[YT][4];
 #pragma unroll
       for (int t = 0; t < YT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-      const bf16* arow = As + (16 * ymt + g) * LDT + c;
-      const bf16* sb0 = Ss + c * DC_LDS + 8 * ynt0 + g;
 #pragma unroll 4
-      for (int k0 = 0; k0 < D; k0 += 8) {
-        uint32_t a[4];
-        a[0] = dc_bf16_bits(arow + k0); a[1] = dc_bf16_bits(arow + 8 * LDT + k0);
-        a[2] = dc_bf16_bits(arow + k0 + 4); a[3] = dc_bf16_bits(arow + 8 * LDT + k0 + 4);
+      for (int k0 = 0; k0 < D; k0 += 16) {
+        uint32_t a[4], b[YT][2];
+        dc_ldm4(a, stage + a_off + 2 * k0);
+        dc_load_b<YT>(b, sb_addr + 2 * k0 * DC_LDS);
 #pragma unroll
-        for (int t = 0; t < YT; ++t) {
-          const bf16* sb = sb0 + k0 * DC_LDS + 8 * t;
-          dc_mma(acc[t], a, dc_bf16_bits(sb), dc_bf16_bits(sb + 4 * DC_LDS));
-        }
+        for (int t = 0; t < YT; ++t) dc_mma(acc[t], a, b[t][0], b[t][1]);
       }
 #pragma unroll
       for (int t = 0; t < YT; ++t)
@@ -163,42 +201,64 @@ __global__ void __launch_bounds__(DC_THREADS, (D <= 128 ? 4 : 2)) delta_chain_ke
         for (int h = 0; h < 2; ++h) {
           const int row = 16 * ymt + g + 8 * h, col = 8 * (ynt0 + t) + 2 * c;
           const int64_t off = (static_cast<int64_t>(i) * DC_C + row) * Dv + col;
-          const float2 xv = *reinterpret_cast<const float2*>(x_base + off);
-          const float2 yv = make_float2(xv.x + p.sign_a * acc[t][2 * h], xv.y + p.sign_a * acc[t][2 * h + 1]);
+          const float2 yv = make_float2(xv[t][h].x + p.sign_a * acc[t][2 * h], xv[t][h].y + p.sign_a * acc[t][2 * h + 1]);
           *reinterpret_cast<float2*>(y_base + off) = yv;
           *reinterpret_cast<__nv_bfloat162*>(Ys + row * DC_LDS + col) = __floats2bfloat162_rn(p.sign_b * yv.x, p.sign_b * yv.y);
         }
     }
+    if (step + 1 < p.n) load_x(step + 1);
+    if (dot_base != nullptr) {
+      if (!PIPE) load_tile(dot_base);
+      float part = 0.f;
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) part = fmaf(s[m][t][e], ld[m][t][e], part);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      if (lane == 0) red[warp] = part;
+    }
+    // ---- S = gamma S + sign_b * (b^T y) + add, accumulated in place
+    if (PIPE && add_base != nullptr) load_tile(add_base);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[m][t][e] *= gm;
     __syncthreads();
-    // ---- S = gamma S + add + sign_b * (b^T y), accumulated in place
-    const float gm = p.gamma[bh * p.n + i];
+    if (dot_base != nullptr && threadIdx.x == 0) {
+      float tot = 0.f;
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
+      for (int wv = 0; wv < DC_THREADS / 32; ++wv) tot += red[wv];
+      p.dot_out[(bh * p.n + i) * (Dv / 32) + blockIdx.x] = tot;        // rows of Dv / 32 slots (zero-filled by the caller)
+    }
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const int row = 16 * (mt0 + m) + g, col = 8 * (nt0 + t) + 2 * c;
-        float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);
-        if (add_base != nullptr) {
-          lo = *reinterpret_cast<const float2*>(add_base + (static_cast<int64_t>(i) * D + row) * Dv + col);
-          hi = *reinterpret_cast<const float2*>(add_base + (static_cast<int64_t>(i) * D + row + 8) * Dv + col);
-        }
-        s[m][t][0] = fmaf(gm, s[m][t][0], lo.x); s[m][t][1] = fmaf(gm, s[m][t][1], lo.y);
-        s[m][t][2] = fmaf(gm, s[m][t][2], hi.x); s[m][t][3] = fmaf(gm, s[m][t][3], hi.y);
-      }
-      const bf16* bcol = Bs + c * LDT + 16 * (mt0 + m) + g;              // b^T as the A operand: A[d][k] = b[k][d]
-#pragma unroll 4
-      for (int k0 = 0; k0 < DC_C; k0 += 8) {
+    for (int k0 = 0; k0 < DC_C; k0 += 16) {
+      uint32_t b[NT][2];
+      dc_load_b<NT>(b, yb_addr + 2 * k0 * DC_LDS);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
         uint32_t a[4];
-        a[0] = dc_bf16_bits(bcol + k0 * LDT); a[1] = dc_bf16_bits(bcol + k0 * LDT + 8);
-        a[2] = dc_bf16_bits(bcol + (k0 + 4) * LDT); a[3] = dc_bf16_bits(bcol + (k0 + 4) * LDT + 8);
+        dc_ldm4t(a, stage + b_off + 2 * (k0 * LDT + 16 * m));
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const bf16* yb = Ys + (k0 + c) * DC_LDS + 8 * (nt0 + t) + g;
-          dc_mma(s[m][t], a, dc_bf16_bits(yb), dc_bf16_bits(yb + 4 * DC_LDS));
-        }
+        for (int t = 0; t < NT; ++t) dc_mma(s[m][t], a, b[t][0], b[t][1]);
       }
     }
-    __syncthreads();                           // As / Bs / Ss / Ys are rewritten by the next step
+    if (add_base != nullptr) {
+      if (!PIPE) load_tile(add_base);
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[m][t][e] += ld[m][t][e];
+    }
+    // (what this step still reads, b and y, is rewritten after the next step's first barrier; PIPE's only stage 0 / 1
+    // alternate, a single stage is rewritten at once)
+    if (!PIPE) __syncthreads();
   }
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -210,11 +270,11 @@ __global__ void __launch_bounds__(DC_THREADS, (D <= 128 ? 4 : 2)) delta_chain_ke
     }
 }
 
-template <int D, int COLS>
+template <int D, int COLS, bool PIPE>
 static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t stream) {
-  constexpr int smem = (2 * DC_C * (D + 8) + D * (COLS + 8) + DC_C * (COLS + 8)) * static_cast<int>(sizeof(bf16)) +
+  constexpr int smem = ((PIPE ? 4 : 2) * DC_C * (D + 8) + D * (COLS + 8) + DC_C * (COLS + 8)) * static_cast<int>(sizeof(bf16)) +
                        8 * static_cast<int>(sizeof(float));
-  auto kern = delta_chain_kernel<D, COLS>;
+  auto kern = delta_chain_kernel<D, COLS, PIPE>;
   static bool configured = false;
   if (!configured) {
     TTCD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -222,6 +282,19 @@ static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t st
   }
   kern<<<dim3(p.Dv / COLS, BH), DC_THREADS, smem, stream>>>(p);
   return static_cast<int>(cudaGetLastError());
+}
+
+// The chain is a string of dependent steps, so what a step waits for is what it costs.  Two stages of a / b, with the
+// addend and the states of the dot product in flight over the products, pay where a CTA has its SM to itself (D = 256,
+// at most one CTA per SM) and in the reverse chain, which reads two [D, Dv] tensors more; elsewhere more CTAs per SM hide
+// each other's waits.  us, one stage | two stages (BH x steps, D, Dv):  forward 32 x 64, 128, 128: 160 | 169;
+// 12 x 47, 256, 512: 293 | 246; 96 x 64, 256, 512: 1801 | 1882.  reverse, the same: 299 | 232; 557 | 419; 3749 | 3305.
+// (TF32 products out of scalar 16-bit shared-memory reads, before: forward 291; 455; 2769, reverse 387; 720; 4466.)
+template <int D, int COLS>
+static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t stream) {
+  const bool alone = D == 256 && static_cast<int64_t>(p.Dv / COLS) * BH <= sm_count();
+  if (p.add != nullptr || alone) return launch_delta_chain<D, COLS, true>(p, BH, stream);
+  return launch_delta_chain<D, COLS, false>(p, BH, stream);
 }
 
 static int delta_chain_dispatch(const DeltaChainParams& p, int BH, cudaStream_t stream) {
