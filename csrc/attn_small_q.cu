@@ -36,6 +36,7 @@ struct SmallQParams {
   const bf16* q; const bf16* k; const bf16* v;
   float* part_o;        // [B, H, Tq, splits, D]
   float* part_ml;       // [B, H, Tq, splits, 2]  (max in log2 units, sum)
+  bf16* out;            // [B, Tq, H, D]
   const int* kv_len;    // optional device word: the number of valid keys (<= Tk); read at launch time
   int B, Tq, Tk, H, HK, splits, window;
   int64_t ldq, ldk, ldv, sq, sk, sv;
@@ -170,6 +171,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, R <= 2 ? 2 : 1) attn_decode_pa
   static_assert(NV <= R && (R & (R - 1)) == 0, "a lane's scores belong to different pairs");
   __shared__ float s_m[DEC_WARPS * KPW][R], s_l[DEC_WARPS * KPW][R];
   __shared__ __align__(16) float s_o[DEC_WARPS][R][D];
+  pdl_wait();
+  pdl_launch_dependents();
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane / LPR, l = lane % LPR;       // key of a load, lane of the key
@@ -349,14 +352,15 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, R <= 2 ? 2 : 1) attn_decode_pa
 // owns D / 32 consecutive dims.  (One warp walking all splits in order took 8.7 us for 16 items of 32 splits.)
 constexpr int MERGE_WARPS = 4;
 template <int D>
-__global__ void __launch_bounds__(MERGE_WARPS * 32) attn_small_q_merge_kernel(const float* __restrict__ part_o,
-                                                                              const float* __restrict__ part_ml,
-                                                                              bf16* __restrict__ out, int Tq, int H, int splits) {
+__global__ void __launch_bounds__(MERGE_WARPS * 32) attn_small_q_merge_kernel(const SmallQParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int splits = p.splits, Tq = p.Tq, H = p.H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t item = blockIdx.x;                  // (b, h, row)
   constexpr int DPL = D / 32;
   __shared__ float s_o[MERGE_WARPS][D], s_l[MERGE_WARPS];
-  const float2* ml = reinterpret_cast<const float2*>(part_ml) + item * splits;
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + item * splits;
   float M = -INFINITY;
   for (int s = lane; s < splits; s += 32) M = fmaxf(M, ml[s].x);
   M = warp_max(M);
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) attn_small_q_merge_kernel(co
 #pragma unroll 4
   for (int s = warp; s < splits; s += MERGE_WARPS) {
     const float2 t = ml[s];
-    const float* src = part_o + (item * splits + s) * D + lane * DPL;
+    const float* src = p.part_o + (item * splits + s) * D + lane * DPL;
     float x[DPL];
 #pragma unroll
     for (int e = 0; e < DPL; ++e) x[e] = src[e];
@@ -386,32 +390,27 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32) attn_small_q_merge_kernel(co
     for (int w = 0; w < MERGE_WARPS; ++w) { acc += s_o[w][threadIdx.x]; tot += s_l[w]; }
     const int row = static_cast<int>(item % Tq);
     const int64_t bh = item / Tq, b = bh / H, h = bh % H;
-    out[((b * Tq + row) * H + h) * D + threadIdx.x] = __float2bfloat16(acc * (tot > 0.f ? 1.f / tot : 0.f));
+    p.out[((b * Tq + row) * H + h) * D + threadIdx.x] = __float2bfloat16(acc * (tot > 0.f ? 1.f / tot : 0.f));
   }
 }
 
 template <int D>
-static int launch_merge(const SmallQParams& p, bf16* out, cudaStream_t stream) {
+static int launch_merge(const SmallQParams& p, cudaStream_t stream) {
   const int64_t items = static_cast<int64_t>(p.B) * p.H * p.Tq;
-  attn_small_q_merge_kernel<D><<<static_cast<unsigned>(items), MERGE_WARPS * 32, 0, stream>>>(p.part_o, p.part_ml, out, p.Tq,
-                                                                                            p.H, p.splits);
-  return static_cast<int>(cudaGetLastError());
+  return launch_dependent(attn_small_q_merge_kernel<D>, dim3(static_cast<unsigned>(items)), dim3(MERGE_WARPS * 32), 0, stream, p);
 }
 
 template <int D>
-static int launch_decode(const SmallQParams& p, bf16* out, cudaStream_t stream) {
+static int launch_decode(const SmallQParams& p, cudaStream_t stream) {
   const int pairs = p.Tq * (p.H / p.HK);
-  const dim3 grid(p.splits, p.HK, p.B);
-  if (pairs <= 1) attn_decode_partial_kernel<D, 1><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
-  else if (pairs <= 2) attn_decode_partial_kernel<D, 2><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
-  else if (pairs <= 4) attn_decode_partial_kernel<D, 4><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
-  else attn_decode_partial_kernel<D, 8><<<grid, DEC_WARPS * 32, 0, stream>>>(p);
-  TTCD_CUDA_CHECK(cudaGetLastError());
-  return launch_merge<D>(p, out, stream);
+  auto kern = pairs <= 1 ? attn_decode_partial_kernel<D, 1> : pairs <= 2 ? attn_decode_partial_kernel<D, 2>
+              : pairs <= 4 ? attn_decode_partial_kernel<D, 4> : attn_decode_partial_kernel<D, 8>;
+  const int rc = launch_dependent(kern, dim3(p.splits, p.HK, p.B), dim3(DEC_WARPS * 32), 0, stream, p);
+  return rc != TTCD_OK ? rc : launch_merge<D>(p, stream);
 }
 
 template <int D>
-static int launch_small_q(const SmallQParams& p, bf16* out, cudaStream_t stream) {
+static int launch_small_q(const SmallQParams& p, cudaStream_t stream) {
   using S = SmallQSmem<D>;
   auto k1 = attn_small_q_partial_kernel<D>;
   static bool configured = false;
@@ -421,7 +420,7 @@ static int launch_small_q(const SmallQParams& p, bf16* out, cudaStream_t stream)
   }
   k1<<<dim3(p.splits, p.HK, p.B), SQ_WARPS * 32, S::TOTAL, stream>>>(p);
   TTCD_CUDA_CHECK(cudaGetLastError());
-  return launch_merge<D>(p, out, stream);
+  return launch_merge<D>(p, stream);
 }
 
 }  // namespace ttcd
@@ -431,7 +430,7 @@ static int launch_small_q(const SmallQParams& p, bf16* out, cudaStream_t stream)
 // [B, H, Tq, splits, 2] are caller-provided scratch; splits must equal ceil(Tk / 256).  window <= 0: unlimited.
 // kv_len (may be null): a device int holding how many of the Tk key rows are filled, read when the kernel runs, so
 // that a captured launch follows a cache that grows between replays; the causal alignment then counts from it.
-static int small_q_params(ttcd::SmallQParams& p, const void* q, const void* k, const void* v, float* part_o, float* part_ml,
+static int small_q_params(ttcd::SmallQParams& p, const void* q, const void* k, const void* v, void* out, float* part_o, float* part_ml,
                           int B, int Tq, int Tk, int H, int HK, int D, long long ldq, long long ldk, long long ldv,
                           long long sq, long long sk, long long sv, int window, float scale, int splits, const int* kv_len) {
   using namespace ttcd;
@@ -440,7 +439,7 @@ static int small_q_params(ttcd::SmallQParams& p, const void* q, const void* k, c
   if (ldk % 8 != 0 || ldv % 8 != 0 || sk % 8 != 0 || sv % 8 != 0) return TTCD_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(k) & 15u) || (reinterpret_cast<uintptr_t>(v) & 15u)) return TTCD_ERR_ARG;
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
-  p.part_o = part_o; p.part_ml = part_ml; p.kv_len = kv_len;
+  p.out = static_cast<bf16*>(out); p.part_o = part_o; p.part_ml = part_ml; p.kv_len = kv_len;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.HK = HK; p.splits = splits; p.window = window;
   p.ldq = ldq; p.ldk = ldk; p.ldv = ldv; p.sq = sq; p.sk = sk; p.sv = sv;
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -454,12 +453,12 @@ TTCD_EXPORT int ttcd_attn_small_q(const void* q, const void* k, const void* v, v
   using namespace ttcd;
   if (splits != (Tk + SQ_KEYS - 1) / SQ_KEYS) return TTCD_ERR_ARG;
   SmallQParams p;
-  const int rc = small_q_params(p, q, k, v, part_o, part_ml, B, Tq, Tk, H, HK, D, ldq, ldk, ldv, sq, sk, sv, window, scale,
+  const int rc = small_q_params(p, q, k, v, out, part_o, part_ml, B, Tq, Tk, H, HK, D, ldq, ldk, ldv, sq, sk, sv, window, scale,
                                 splits, kv_len);
   if (rc != TTCD_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  return D == 128 ? launch_small_q<128>(p, static_cast<bf16*>(out), stream)
-                  : launch_small_q<64>(p, static_cast<bf16*>(out), stream);
+  return D == 128 ? launch_small_q<128>(p, stream)
+                  : launch_small_q<64>(p, stream);
 }
 
 // The same call for at most 8 (query row, head of the group) pairs per key/value head: Tq * (H / HK) <= 8.  q rows are
@@ -471,11 +470,11 @@ TTCD_EXPORT int ttcd_attn_decode(const void* q, const void* k, const void* v, vo
   using namespace ttcd;
   if (splits < 1 || splits > 65535 || B > 65535 || HK > 65535) return TTCD_ERR_ARG;
   SmallQParams p;
-  const int rc = small_q_params(p, q, k, v, part_o, part_ml, B, Tq, Tk, H, HK, D, ldq, ldk, ldv, sq, sk, sv, window, scale,
+  const int rc = small_q_params(p, q, k, v, out, part_o, part_ml, B, Tq, Tk, H, HK, D, ldq, ldk, ldv, sq, sk, sv, window, scale,
                                 splits, kv_len);
   if (rc != TTCD_OK) return rc;
   if (Tq * (H / HK) > 8 || ldq % 8 != 0 || sq % 8 != 0 || (reinterpret_cast<uintptr_t>(q) & 15u)) return TTCD_ERR_ARG;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
-  return D == 128 ? launch_decode<128>(p, static_cast<bf16*>(out), stream)
-                  : launch_decode<64>(p, static_cast<bf16*>(out), stream);
+  return D == 128 ? launch_decode<128>(p, stream)
+                  : launch_decode<64>(p, stream);
 }

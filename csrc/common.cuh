@@ -340,6 +340,29 @@ __device__ __forceinline__ void tmem_st_n(uint32_t taddr, const uint32_t (&r)[N]
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// ---- programmatic dependent launch -----------------------------------------------------------------------------
+// A kernel launched by launch_dependent may start while the kernel before it on the stream still runs.  pdl_wait()
+// returns when that kernel has finished and its writes are visible; everything that reads or writes memory comes after
+// it (but for reads of memory that no unfinished kernel can be writing).  pdl_launch_dependents() lets the next kernel
+// start; it comes after pdl_wait(), so that a kernel never runs beside one that is two launches older.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename Param>
+static inline int launch_dependent(void (*kern)(Param), dim3 grid, dim3 block, int smem, cudaStream_t stream,
+                                   const Param& param) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, param));
+}
+
 // ---- misc ----------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

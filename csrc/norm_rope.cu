@@ -747,6 +747,71 @@ __global__ void __launch_bounds__(256) qk_norm_rope_fwd_vec_kernel(const QKRopeP
   }
 }
 
+// One decode step's q | k | v rows (one token per sample, packed side by side): per-head norm and rotary of q and k as
+// above, q to its own tensor, k and v into row *slot of the key/value rings.  One launch instead of the norm / rotary
+// kernel, two indexed copies and a conversion of the positions (2.9 + 2 x 3.1 + 1.4 us per layer and token).
+struct DecodeQKVParams {
+  const bf16* qkv; int64_t ld;
+  bf16* q; bf16* ring_k; bf16* ring_v; int64_t ring_sb;       // ring [B][capacity][HK][D]: batch stride in elements
+  const int64_t* slot; const int64_t* positions;              // [1], [B]; positions null without rotary
+  const bf16* qw; const bf16* kw; const bf16* cos; const bf16* sin;
+  int B, H, HK; float eps;
+};
+
+template <int LPH>
+__global__ void __launch_bounds__(256) decode_qkv_kernel(const DecodeQKVParams p) {
+  constexpr int HALF = LPH * 8, D = 2 * HALF;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int sub = threadIdx.x % LPH;
+  const int heads = p.H + 2 * p.HK;
+  const int b = blockIdx.x;
+  const int64_t slot_row = static_cast<int64_t>(b) * p.ring_sb + *p.slot * p.HK * D;
+  const int64_t pos = p.positions != nullptr ? p.positions[b] : 0;
+  // whole groups of LPH lanes run or skip an iteration together; the sums stay inside a group
+  for (int h = threadIdx.x / LPH; h < heads; h += 256 / LPH) {
+    const bf16* in = p.qkv + b * p.ld + h * D + sub * 8;
+    const bool is_v = h >= p.H + p.HK, is_q = h < p.H;
+    Vec8 lo, hi;
+    lo.load(in);
+    hi.load(in + HALF);
+    bf16* out = is_q ? p.q + (static_cast<int64_t>(b) * p.H + h) * D
+                     : (is_v ? p.ring_v + slot_row + (h - p.H - p.HK) * D : p.ring_k + slot_row + (h - p.H) * D);
+    out += sub * 8;
+    if (!is_v) {
+      float x1[8], x2[8];
+      lo.to_float(x1);
+      hi.to_float(x2);
+      const bf16* w = is_q ? p.qw : p.kw;
+      float w1[8], w2[8], c[8], sn[8], rstd = 1.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { w1[i] = w2[i] = c[i] = 1.f; sn[i] = 0.f; }
+      if (w != nullptr) { ld8(w + sub * 8, w1); ld8(w + HALF + sub * 8, w2); }
+      if (p.cos != nullptr) { ld8(p.cos + pos * HALF + sub * 8, c); ld8(p.sin + pos * HALF + sub * 8, sn); }
+      if (w != nullptr) {
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss += x1[i] * x1[i] + x2[i] * x2[i];
+        const uint32_t mask = LPH == 32 ? 0xffffffffu : ((1u << LPH) - 1u) << (threadIdx.x % 32 / LPH * LPH);
+#pragma unroll
+        for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(mask, ss, o);
+        rstd = rsqrtf(ss / D + p.eps);
+      }
+      float o1[8], o2[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float y1 = x1[i] * rstd * w1[i], y2 = x2[i] * rstd * w2[i];
+        o1[i] = y1 * c[i] - y2 * sn[i];
+        o2[i] = y1 * sn[i] + y2 * c[i];
+      }
+      lo.from_float(o1);
+      hi.from_float(o2);
+    }
+    lo.store(out);
+    hi.store(out + HALF);
+  }
+}
+
 template <int LPH>
 __global__ void __launch_bounds__(256) qk_norm_rope_bwd_vec_kernel(const QKRopeParams p) {
   __shared__ float red[2][256];                           // [q|k][D <= 256], shared atomics at the end
@@ -1041,6 +1106,26 @@ TTCD_EXPORT int ttcd_qk_norm_rope_fwd(const void* q_in, long long ldq, const voi
   else if (half <= 64) qk_norm_rope_fwd_kernel<2><<<grid, 256, 0, st>>>(p);
   else qk_norm_rope_fwd_kernel<4><<<grid, 256, 0, st>>>(p);
   return static_cast<int>(cudaGetLastError());
+}
+
+// qkv [B][ld] bf16: H + 2 HK heads of D (64 or 128) side by side; q out [B][H][D]; rings [B][capacity][HK][D] (batch
+// stride ring_sb elements), written at row *slot; positions int64 [B] and cos / sin [.][D / 2] (all null: no rotary);
+// qw, kw [D] (null: no norm).  Everything 16-byte aligned.
+TTCD_EXPORT int ttcd_decode_qkv(const void* qkv, long long ld, void* q, void* ring_k, void* ring_v, long long ring_sb,
+                                const long long* slot, const long long* positions, const void* qw, const void* kw,
+                                const void* cos, const void* sin, int B, int H, int HK, int D, float eps, void* stream_ptr) {
+  if (B <= 0 || H <= 0 || HK <= 0 || (D != 64 && D != 128) || ld % 8 != 0 || ring_sb % 8 != 0 || slot == nullptr) return TTCD_ERR_ARG;
+  if ((cos != nullptr && (sin == nullptr || positions == nullptr)) || (qw == nullptr) != (kw == nullptr)) return TTCD_ERR_ARG;
+  DecodeQKVParams p;
+  p.qkv = static_cast<const bf16*>(qkv); p.ld = ld;
+  p.q = static_cast<bf16*>(q); p.ring_k = static_cast<bf16*>(ring_k); p.ring_v = static_cast<bf16*>(ring_v); p.ring_sb = ring_sb;
+  p.slot = reinterpret_cast<const int64_t*>(slot); p.positions = reinterpret_cast<const int64_t*>(positions);
+  p.qw = static_cast<const bf16*>(qw); p.kw = static_cast<const bf16*>(kw);
+  p.cos = static_cast<const bf16*>(cos); p.sin = static_cast<const bf16*>(sin);
+  p.B = B; p.H = H; p.HK = HK; p.eps = eps;
+  cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
+  return D == 128 ? launch_dependent(decode_qkv_kernel<8>, dim3(B), dim3(256), 0, st, p)
+                  : launch_dependent(decode_qkv_kernel<4>, dim3(B), dim3(256), 0, st, p);
 }
 
 // Backward: dq_in/dk_in (written to q_out/k_out slots) from gradients w.r.t. the rotated outputs.

@@ -4,6 +4,9 @@ with a weight (row, column and K remainders)."""
 import pytest
 import torch
 
+from ttcd_b200.models import IPTTCDv9Config, IPTTCDv9ForCausalLM
+from ttcd_b200.models.decoding import GraphDecoder
+from ttcd_b200.models.layers import WindowKVCache
 from ttcd_b200.ops import cuda
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +57,60 @@ def test_few_rows_times_weight_against_float64(M, N, K):
     # fp32 accumulation (K terms of size ~K^-1/2) and one rounding to bf16
     bound = want.abs() * 2.0 ** -8 + 2.0 ** -22 * K ** 0.5
     assert got.shape == (M, N) and ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (3, 130, 264), (8, 1001, 1024), (9, 256, 2048), (16, 3072, 1032)])
+@pytest.mark.parametrize("norm,swiglu,residual", [(True, False, False), (True, True, False), (False, False, True), (False, True, True)])
+def test_few_rows_with_norm_swiglu_residual(M, N, K, norm, swiglu, residual):
+    """What rides along with the product rounds where the separate ops round."""
+    torch.manual_seed(N + K)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    nw = (1 + 0.1 * torch.randn(K, device=DEV)).bfloat16()
+    w = (torch.randn(2 * N if swiglu else N, K, device=DEV) * K ** -0.5).bfloat16()
+    res = torch.randn(M, N, device=DEV).bfloat16() if residual else None
+    got = cuda.gemv(x, w, norm=(nw, 1e-6) if norm else None, swiglu=swiglu, residual=res).double()
+    xd = x.double()
+    if norm:
+        xd = (xd * (xd.square().mean(-1, keepdim=True) + 1e-6).rsqrt() * nw.double()).bfloat16().double()
+    y = (xd @ w.double().t()).bfloat16().double()
+    if swiglu:
+        y = (torch.nn.functional.silu(y[:, :N]) * y[:, N:]).bfloat16().double()
+    want = y if res is None else (y + res.double())
+    # up to four roundings to bf16 (each may fall to the neighbour) on values and summands of size ~1
+    bound = 2.0 ** -7 * (want.abs() + y.abs()) + 2.0 ** -7
+    assert ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())
+    assert (got - want).abs().mean() < 2.0 ** -9
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,dim,prompt,window", [(1, 4, 2, 128, 200, 256), (3, 5, 5, 64, 40, 64), (16, 8, 2, 64, 130, None)])
+def test_fused_decode_step_matches_module_by_module(batch, heads, kv_heads, dim, prompt, window):
+    """The captured step of a model (fused projections, ring writes, wrapped rings) against the same step run through the
+    modules: same roundings, sums in another order."""
+    torch.manual_seed(3)
+    cfg = IPTTCDv9Config(hidden_size=256, num_hidden_layers=2, num_heads=heads, num_kv_heads=kv_heads, head_dim=dim,
+                         intermediate_size=520, vocab_size=1000, window_size=window, max_position_embeddings=512, ttt_mode=False,
+                         ttt_layers=[], qk_norm=True, tie_word_embeddings=False)
+    model = IPTTCDv9ForCausalLM(cfg).to(DEV, torch.bfloat16).eval()
+    ids = torch.randint(0, 1000, (batch, prompt), device=DEV)
+    cache = WindowKVCache()
+    with torch.no_grad():
+        model(input_ids=ids, past_key_values=cache, use_cache=True, logits_to_keep=1)
+    dec = GraphDecoder(model, cache, 40)
+    assert dec.fused is not None
+    first = ids[:, -1:]
+    steps = 40                                               # past the ring's end for the windowed cases
+    tokens = dec.run(first, steps, set())
+    got, rings = dec.last_logits.clone(), [(k.clone(), v.clone()) for k, v in dec.cache.layers.values()]
+    dec.fused = None                                         # module by module, fed the same tokens
+    dec.load(cache)
+    feed = torch.cat([first, tokens], dim=1)
+    with torch.no_grad():
+        for i in range(steps):
+            dec.token.copy_(feed[:, i:i + 1])
+            want = dec._logits().clone()
+            dec.cache.advance()
+    err = (got.float() - want.float()).norm() / want.float().norm()
+    assert err < 0.02, float(err)
+    for (k, v), (rk, rv) in zip(rings, dec.cache.layers.values()):
+        for a, b in ((k, rk), (v, rv)):
+            assert (a.float() - b.float()).norm() / b.float().norm() < 0.02

@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import torch
 
-from .layers import Attention, GatedMLP, StaticWindowCache, WindowKVCache
+from .layers import Attention, GatedMLP, StaticWindowCache, WindowKVCache, _slab_view
 
 
 def pack_projection_weights(model) -> int:
@@ -33,7 +33,7 @@ def pack_projection_weights(model) -> int:
         ws = [lin.weight for lin in group]
         if any(lin.bias is not None for lin in group) or any(w.data._base is not None or not w.is_contiguous() for w in ws):
             continue
-        if all(ws[i].data_ptr() + ws[i].numel() * ws[i].element_size() == ws[i + 1].data_ptr() for i in range(len(ws) - 1)):
+        if _slab_view(ws) is not None:      # (neighbours by chance, each in its own storage, are no slab)
             continue
         if len({(w.dtype, w.device, w.shape[1]) for w in ws}) != 1:
             continue
@@ -57,6 +57,60 @@ def graph_decoding_supported(model, input_ids, attention_mask, do_sample: bool) 
     return _native.available() and next(model.parameters()).dtype == torch.bfloat16
 
 
+def _fused_block_weights(block, batch: int):
+    """The weights of a block whose decode step runs as seven launches (``_fused_block_step``), or None where the step has
+    to go through the modules: another kind of block, an option the step has no kernel for, a hook on a module."""
+    from .layers import RMSNorm
+    from .modeling_ipttcdv9 import IPTTCDBlock
+    from .modeling_transformer import TransformerBlock
+    if type(block) not in (IPTTCDBlock, TransformerBlock) or block.training or batch > 16:
+        return None
+    if type(block) is IPTTCDBlock and block.is_ttt_layer and block.ttt_chunk <= 1:       # one token would be a whole chunk
+        return None
+    if any(m._forward_hooks or m._forward_pre_hooks for m in block.modules()):
+        return None
+    attn, mlp = block.attn, block.mlp
+    if type(attn) is not Attention or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128):
+        return None
+    if any(type(n) is not RMSNorm or n.weight is None for n in (block.attn_norm, block.mlp_norm)):
+        return None
+    if any(m.bias is not None for m in (attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.gate_proj, mlp.up_proj, mlp.down_proj)):
+        return None
+    qkv = _slab_view([attn.q_proj.weight, attn.k_proj.weight, attn.v_proj.weight])
+    gate_up = _slab_view([mlp.gate_proj.weight, mlp.up_proj.weight])
+    ws = [qkv, gate_up, attn.o_proj.weight, mlp.down_proj.weight, block.attn_norm.weight, block.mlp_norm.weight]
+    if attn.qk_norm:
+        ws += [attn.q_norm.weight, attn.k_norm.weight]
+    hidden = attn.hidden_size
+    if hidden % 8 or hidden > 2048 or mlp.intermediate_size % 8:
+        return None
+    if any(w is None or w.dtype != torch.bfloat16 or not w.is_contiguous() or w.data_ptr() % 16 for w in ws):
+        return None
+    return qkv, gate_up
+
+
+def _fused_block_step(block, weights, x: torch.Tensor, cache: StaticWindowCache) -> torch.Tensor:
+    """One token per sample through a decoder block: x [B, hidden] -> x.  The norms ride in front of the projections that
+    read them, SwiGLU and the residual sums behind the ones that produce them, k and v go straight into the rings; the
+    roundings are those of the module by module step."""
+    from .. import ops
+    from ..ops import cuda
+    attn, mlp, (qkv_w, gate_up_w) = block.attn, block.mlp, weights
+    i = attn.layer_idx
+    c = cache.capacity[i]
+    rk, rv = cache.layers[i]
+    cos = sin = None
+    if not attn.use_nope:
+        cos, sin = attn.rotary.tables(max(cache.max_position, attn.max_position_embeddings or 0), x.device, x.dtype)
+    qw, kw, eps = (attn.q_norm.weight, attn.k_norm.weight, attn.q_norm.eps) if attn.qk_norm else (None, None, 0.0)
+    qkv = cuda.gemv(x, qkv_w, norm=(block.attn_norm.weight, block.attn_norm.eps), early_w=True)
+    q = cuda.decode_qkv(qkv, rk, rv, cache.slot[c], cache.positions, qw, kw, eps, cos, sin, attn.num_heads)
+    o = ops.decode_attention(q, rk, rv, cache.kv_len[c])
+    x = cuda.gemv(o.view(x.shape[0], -1), attn.o_proj.weight, residual=x, early_w=True)
+    z = cuda.gemv(x, gate_up_w, norm=(block.mlp_norm.weight, block.mlp_norm.eps), swiglu=True, early_w=True)
+    return cuda.gemv(z, mlp.down_proj.weight, residual=x, early_w=True)
+
+
 def _windows(model) -> dict[int, int | None]:
     return {m.layer_idx: m.window_size for m in model.modules() if isinstance(m, Attention)}
 
@@ -75,6 +129,7 @@ class GraphDecoder:
         self.out = torch.zeros(batch, max_new_tokens, dtype=torch.long, device=dev)
         self.cursor = torch.zeros(1, dtype=torch.int64, device=dev)
         self.weights_at = self._weights_at()
+        self.fused = self._fused_weights(batch)
         start = self.cache.start
         # warm-up on a side stream (allocator pools, rotary tables, lazily configured kernels), then rewind and capture
         side = torch.cuda.Stream(device=dev)
@@ -92,10 +147,29 @@ class GraphDecoder:
     def _weights_at(self):
         return (self.model.lm_head.weight.data_ptr(), next(self.model.model.layers[0].parameters()).data_ptr())
 
+    def _fused_weights(self, batch: int):
+        """Per block the weights of its fused step; None if any part of the model has to run module by module."""
+        model, head = self.model, self.model.lm_head
+        if any(m._forward_hooks or m._forward_pre_hooks for m in (model, model.model, model.model.norm, model.model.embeddings, head)):
+            return None
+        if head.bias is not None or head.weight.dtype != torch.bfloat16 or not head.weight.is_contiguous() or head.weight.data_ptr() % 16:
+            return None
+        got = [_fused_block_weights(layer, batch) for layer in model.model.layers]
+        return None if any(w is None for w in got) else got
+
+    def _logits(self) -> torch.Tensor:
+        if self.fused is None:
+            return self.model(input_ids=self.token, past_key_values=self.cache, use_cache=True, logits_to_keep=1).logits[:, -1]
+        from ..ops import cuda
+        core = self.model.model
+        x = core.embeddings(self.token.view(-1))
+        for layer, weights in zip(core.layers, self.fused):
+            x = _fused_block_step(layer, weights, x, self.cache)
+        return cuda.gemv(core.norm(x), self.model.lm_head.weight, early_w=True)
+
     @torch.no_grad()
     def _step(self) -> None:
-        logits = self.model(input_ids=self.token, past_key_values=self.cache, use_cache=True, logits_to_keep=1).logits
-        self.last_logits = logits[:, -1]                 # (kept for inspection; lives in the graph's pool)
+        self.last_logits = self._logits()                # (kept for inspection; lives in the graph's pool)
         nxt = self.last_logits.float().argmax(-1, keepdim=True)
         self.token.copy_(nxt)
         self.out.index_copy_(1, self.cursor, nxt)

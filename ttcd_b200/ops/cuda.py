@@ -70,13 +70,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out_dtype=_BF16, alpha: float = 1.
     M0, K0, N0 = a.shape[-2], a.shape[-1], b.shape[-1]
     if (M0 <= 16 and a.dim() == 2 and b.dim() == 2 and out_dtype == _BF16 and beta == 0.0 and c_in is None
             and row_scale is None and out is None and K0 % 8 == 0 and b.stride(0) == 1 and b.stride(1) % 8 == 0
-            and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0
-            and nv.has("ttcd_gemv_small")):
+            and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
         # a few rows times a [N, K] weight (b is its transposed view): the decode step; one pass over the weight
-        y = torch.empty(M0, N0, dtype=_BF16, device=a.device)
-        nv.call("ttcd_gemv_small", nv.ptr(a), nv.ptr(b), nv.ptr(y), nv.i32(M0), nv.i32(N0), nv.i32(K0), nv.i64(a.stride(0)),
-                nv.i64(b.stride(1)), nv.i64(N0), nv.f32(alpha), nv.stream_ptr())
-        return y
+        return gemv(a, b.transpose(0, 1), alpha=alpha)
     if M0 < 128 or N0 < 128 or K0 < 64:
         # tiny problem: zero-pad up to one tile (TMA boxes must fit inside their tensors)
         if out is not None or c_in is not None or row_scale is not None:
@@ -130,6 +126,33 @@ class GradSlab:
         self.buf = None
 
     def get(self, rows: int, device) -> torch.Tensor:
+def gemv(x: torch.Tensor, w: torch.Tensor, *, alpha: float = 1.0, residual=None, norm=None,
+         swiglu: bool = False, early_w: bool = False) -> torch.Tensor:
+    """alpha * x[M, K] @ w[N, K]^T for M <= 16, in one pass over the weight.  ``norm`` = (weight, eps): x is RMS-normalised
+    first (K <= 2048); ``swiglu``: w holds gate rows then up rows; ``residual`` [M, N] is added.  ``early_w``: nothing that
+    may still be running on the stream writes w (weights at rest), so that reading it may start before the previous
+    kernel has finished."""
+    M, K = x.shape
+    N = w.shape[0] // 2 if swiglu else w.shape[0]
+    y = torch.empty(M, N, dtype=_BF16, device=x.device)
+    nw, eps = (None, 0.0) if norm is None else norm
+    nv.call("ttcd_gemv_small", nv.ptr(x), nv.ptr(w), nv.ptr(y), nv.ptr(residual), nv.ptr(nw), nv.i32(M), nv.i32(N), nv.i32(K),
+            nv.i64(x.stride(0)), nv.i64(w.stride(0)), nv.i64(N), nv.i64(0 if residual is None else residual.stride(0)),
+            nv.f32(alpha), nv.f32(eps), nv.i32(int(swiglu)), nv.i32(int(early_w)), nv.stream_ptr())
+    return y
+
+
+def decode_qkv(qkv, ring_k, ring_v, slot, positions, qw, kw, eps, cos, sin, heads: int):
+    """One token per sample: ``qkv`` [B, (H + 2 HK) D] -> per-head norm and rotary; q is returned as [B, 1, H, D], k and v
+    are written to row ``slot`` (int64, on the device) of the rings [B, capacity, HK, D]."""
+    B, HK, D = qkv.shape[0], ring_k.shape[2], ring_k.shape[3]
+    q = torch.empty(B, 1, heads, D, dtype=_BF16, device=qkv.device)
+    nv.call("ttcd_decode_qkv", nv.ptr(qkv), nv.i64(qkv.stride(0)), nv.ptr(q), nv.ptr(ring_k), nv.ptr(ring_v),
+            nv.i64(ring_k.stride(0)), nv.ptr(slot), nv.ptr(None if cos is None else positions), nv.ptr(qw), nv.ptr(kw),
+            nv.ptr(cos), nv.ptr(sin), nv.i32(B), nv.i32(heads), nv.i32(HK), nv.i32(D), nv.f32(eps), nv.stream_ptr())
+    return q
+
+
         if self.buf is None or self.buf.shape[0] != rows:
             self.buf = torch.empty(rows, self.n_total, dtype=_BF16, device=device)
         return self.buf
