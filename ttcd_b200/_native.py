@@ -78,7 +78,8 @@ def has(symbol: str) -> bool:
 
 
 def stream_ptr() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream of the current device (its raw handle: a Stream object per launch costs ten times as much)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
@@ -100,24 +101,33 @@ _MULTI_KERNEL = {"ttcd_attn_bwd": 2, "ttcd_attn_bwd_cp": 2, "ttcd_rmsnorm_bwd_no
                  "ttcd_ipc_close": 0}
 
 
-def call(symbol: str, *args) -> None:
-    """Invoke ``int symbol(args...)`` and raise on a non-zero status."""
-    global launch_count
-    launch_count += _MULTI_KERNEL.get(symbol, 1)
-    lib = load(required=True)
-    fn = getattr(lib, symbol, None)
+_entries: dict[str, tuple] = {}    # symbol -> (entry point, kernels it launches)
+
+
+def _entry(symbol: str) -> tuple:
+    fn = getattr(load(required=True), symbol, None)
     if fn is None:
         raise NativeError(f"native symbol {symbol} missing from {_LIB_PATH}")
     fn.restype = ctypes.c_int
+    _entries[symbol] = got = (fn, _MULTI_KERNEL.get(symbol, 1))
+    return got
+
+
+def call(symbol: str, *args) -> None:
+    """Invoke ``int symbol(args...)`` and raise on a non-zero status."""
+    global launch_count
+    fn, kernels = _entries.get(symbol) or _entry(symbol)
+    launch_count += kernels
     rc = fn(*args)
     if rc != 0:
+        lib = load(required=True)
         detail = _ERRORS.get(rc, f"cudaError {rc}")
         if rc == -4 and hasattr(lib, "ttcd_last_tmap_error"):
             buf = ctypes.create_string_buffer(320)
             lib.ttcd_last_tmap_error(buf, ctypes.c_int(320))
             detail += f" ({buf.value.decode(errors='replace')})"
         raise NativeError(f"{symbol} failed: {detail}")
-    if _CHECK_EVERY_CALL and _MULTI_KERNEL.get(symbol, 1) > 0:
+    if _CHECK_EVERY_CALL and kernels > 0:
         _check_after(symbol)
 
 

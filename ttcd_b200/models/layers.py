@@ -399,6 +399,8 @@ def _slab_view(params: list[torch.Tensor]) -> torch.Tensor | None:
             return None
         expect += p.numel() * p.element_size()
     rows = sum(p.shape[0] for p in params)
+    if (expect - first.data_ptr()) + first.storage_offset() * first.element_size() > first.untyped_storage().nbytes():
+        return None                         # neighbours in memory, but not in one storage
     try:
         return torch.as_strided(first.detach(), (rows, first.shape[1]), (first.shape[1], 1))
     except RuntimeError:

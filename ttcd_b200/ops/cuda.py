@@ -9,6 +9,7 @@ from __future__ import annotations
 import math
 
 import torch
+from torch.autograd import forward_ad as _forward_ad
 
 from .. import _native as nv
 from . import reference
@@ -16,6 +17,25 @@ from .selective import keep
 
 _BF16 = torch.bfloat16
 _SM_BLOCKS = 148 * 2
+
+
+class _Forward:
+    """Stands in for an autograd context where nothing is recorded."""
+    needs_input_grad = ()
+
+    def save_for_backward(self, *_):
+        pass
+
+    def mark_non_differentiable(self, *_):
+        pass
+
+
+def _apply(fn, *args):
+    """``fn.apply(*args)``; with gradients off and no function transform (vmap, forward-mode derivatives, torch.func) at
+    work just its forward: the autograd machinery around a call costs the host more than the launch inside it."""
+    if torch.is_grad_enabled() or torch._C._functorch.peek_interpreter_stack() is not None or _forward_ad._current_level >= 0:
+        return fn.apply(*args)
+    return fn.forward(_Forward(), *args)
 
 
 def _check(t: torch.Tensor, name: str):
@@ -40,21 +60,18 @@ def _dense_rows(x: torch.Tensor) -> torch.Tensor:
 # =============================================================================================
 
 def _operand(t: torch.Tensor):
-    """Describe a [.., R, C] matrix for the kernel: (tensor, is_row_major, ld, batch_stride)."""
-    if t.dim() == 2:
-        t = t.unsqueeze(0)
+    """Describe a [.., R, C] matrix for the kernel: (tensor, is_row_major, ld, batch, batch_stride, R, C)."""
     if t.dim() > 3:
         t = t.reshape(-1, t.shape[-2], t.shape[-1]) if t.is_contiguous() else t.contiguous().view(-1, *t.shape[-2:])
-    ok_row = t.stride(-1) == 1 and t.stride(-2) % 8 == 0 and t.stride(-2) >= t.shape[-1]
-    ok_col = t.stride(-2) == 1 and t.stride(-1) % 8 == 0 and t.stride(-1) >= t.shape[-2]
-    if t.shape[-1] == 1 and t.shape[-2] == 1:
-        ok_row, ok_col = False, False
-    if not (ok_row or ok_col) or t.data_ptr() % 16 or (t.shape[0] > 1 and t.stride(0) % 8):
+    shape, stride = t.shape, t.stride()
+    R, C, sr, sc = shape[-2], shape[-1], stride[-2], stride[-1]
+    batch = shape[0] if len(shape) == 3 else 1
+    ok_row = sc == 1 and sr % 8 == 0 and sr >= C
+    ok_col = sr == 1 and sc % 8 == 0 and sc >= R
+    if not (ok_row or ok_col) or (R == 1 and C == 1) or t.data_ptr() % 16 or (batch > 1 and stride[0] % 8):
         t = t.contiguous()
-        ok_row, ok_col = True, False
-    row_major = ok_row
-    ld = t.stride(-2) if row_major else t.stride(-1)
-    return t, row_major, ld, (t.stride(0) if t.shape[0] > 1 else 0)
+        ok_row, stride = True, t.stride()
+    return t, ok_row, (stride[-2] if ok_row else stride[-1]), batch, (stride[0] if batch > 1 else 0), R, C
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, out_dtype=_BF16, alpha: float = 1.0, beta: float = 0.0,
@@ -82,19 +99,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out_dtype=_BF16, alpha: float = 1.
         bp = torch.nn.functional.pad(b, (0, Np - N0, 0, Kp - K0))
         full = gemm(ap, bp, out_dtype=out_dtype, alpha=alpha)
         return full[..., :M0, :N0].contiguous()
-    a3, a_row, lda, sa = _operand(a)
-    b3, b_row, ldb, sb = _operand(b)
-    batch = max(a3.shape[0], b3.shape[0])
-    M, K = a3.shape[-2], a3.shape[-1]
-    K2, N = b3.shape[-2], b3.shape[-1]
+    a3, a_row, lda, batch_a, sa, M, K = _operand(a)
+    b3, b_row, ldb, batch_b, sb, K2, N = _operand(b)
+    batch = max(batch_a, batch_b)
     if K != K2:
         raise ValueError(f"gemm shape mismatch: {tuple(a.shape)} @ {tuple(b.shape)}")
-    if a3.shape[0] not in (1, batch) or b3.shape[0] not in (1, batch):
+    if batch_a not in (1, batch) or batch_b not in (1, batch):
         raise ValueError("gemm batch mismatch")
-    if a3.shape[0] == 1:
-        sa = 0
-    if b3.shape[0] == 1:
-        sb = 0
     if out is None:
         out = torch.empty((batch, M, N), dtype=out_dtype, device=a.device)
     c3 = out.view(batch, M, N) if out.dim() != 3 else out
@@ -115,17 +126,6 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, out_dtype=_BF16, alpha: float = 1.
     return out
 
 
-class GradSlab:
-    """Meeting point for the gradients of the column slices of one fused projection (q|k|v): the backward
-    kernels of the consumers write straight into one [rows, n_total] buffer, so the projection's backward
-    finds its packed gradient in place instead of assembling it with copies.  The forward tags the slices
-    (``tag``); whichever backward runs first allocates the buffer."""
-
-    def __init__(self, n_total: int):
-        self.n_total = n_total
-        self.buf = None
-
-    def get(self, rows: int, device) -> torch.Tensor:
 def gemv(x: torch.Tensor, w: torch.Tensor, *, alpha: float = 1.0, residual=None, norm=None,
          swiglu: bool = False, early_w: bool = False) -> torch.Tensor:
     """alpha * x[M, K] @ w[N, K]^T for M <= 16, in one pass over the weight.  ``norm`` = (weight, eps): x is RMS-normalised
@@ -153,6 +153,17 @@ def decode_qkv(qkv, ring_k, ring_v, slot, positions, qw, kw, eps, cos, sin, head
     return q
 
 
+class GradSlab:
+    """Meeting point for the gradients of the column slices of one fused projection (q|k|v): the backward
+    kernels of the consumers write straight into one [rows, n_total] buffer, so the projection's backward
+    finds its packed gradient in place instead of assembling it with copies.  The forward tags the slices
+    (``tag``); whichever backward runs first allocates the buffer."""
+
+    def __init__(self, n_total: int):
+        self.n_total = n_total
+        self.buf = None
+
+    def get(self, rows: int, device) -> torch.Tensor:
         if self.buf is None or self.buf.shape[0] != rows:
             self.buf = torch.empty(rows, self.n_total, dtype=_BF16, device=device)
         return self.buf
@@ -210,7 +221,7 @@ def matmul(a, b):
         a = a.to(_BF16)
     if b.dtype != _BF16:
         b = b.to(_BF16)
-    return _MatMul.apply(a, b)
+    return _apply(_MatMul, a, b)
 
 
 def _split_k_factor(M: int, N: int, K: int, sms: int = 148) -> int:
@@ -330,7 +341,7 @@ def _adjacent_columns(grads, splits, n_total):
 def linear(x, weight, bias=None):
     _check(x, "x")
     w = weight if weight.dtype == _BF16 else weight.to(_BF16)
-    y = _Linear.apply(x, None, w)
+    y = _apply(_Linear, x, None, w)
     return y if bias is None else y + bias.to(y.dtype)
 
 
@@ -344,7 +355,7 @@ def fused_linear(x, weights, slab):
     if handle is not None:
         weights[0]._ttcd_gather = None
         _gather_handle = handle if handle.pending else None
-    return _Linear.apply(x, slab, *ws)
+    return _apply(_Linear, x, slab, *ws)
 
 
 # =============================================================================================
@@ -404,7 +415,7 @@ class _RMSNorm(torch.autograd.Function):
 
 def rmsnorm(x, weight, eps, residual=None, prenorm=False):
     _check(x, "x")
-    return _RMSNorm.apply(x, residual, weight, float(eps), bool(prenorm))
+    return _apply(_RMSNorm, x, residual, weight, float(eps), bool(prenorm))
 
 
 class _RMSNormDual(torch.autograd.Function):
@@ -454,7 +465,7 @@ class _RMSNormDual(torch.autograd.Function):
 
 def rmsnorm_dual(a_t, a_s, residual, weight, eps):
     _check(a_t, "a_t")
-    return _RMSNormDual.apply(a_t, a_s, residual, weight, float(eps))
+    return _apply(_RMSNormDual, a_t, a_s, residual, weight, float(eps))
 
 
 # =============================================================================================
@@ -541,13 +552,13 @@ class _QKNormRope(torch.autograd.Function):
 
 def qk_norm_rope(q, k, q_weight, k_weight, eps, cos, sin, offset=0, positions=None):
     _check(q, "q"), _check(k, "k")
-    return _QKNormRope.apply(q, k, q_weight, k_weight, float(eps), cos, sin, offset, positions)
+    return _apply(_QKNormRope, q, k, q_weight, k_weight, float(eps), cos, sin, offset, positions)
 
 
 def rope(x, cos, sin, offset=0, positions=None):
     """Rotary on one tensor (runs the fused kernel with a zero-head partner)."""
     k_dummy = x[:, :, :0]
-    out, _ = _QKNormRope.apply(x, k_dummy.reshape(x.shape[0], x.shape[1], 0, x.shape[3]), None, None, 0.0, cos, sin,
+    out, _ = _apply(_QKNormRope, x, k_dummy.reshape(x.shape[0], x.shape[1], 0, x.shape[3]), None, None, 0.0, cos, sin,
                                offset, positions)
     return out
 
@@ -588,12 +599,12 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(gate, up):
     _check(gate, "gate")
-    return _SwiGLU.apply(gate, up)
+    return _apply(_SwiGLU, gate, up)
 
 
 def swiglu_packed(gate_up):
     d = gate_up.shape[-1] // 2
-    return _SwiGLU.apply(gate_up[..., :d], gate_up[..., d:])
+    return _apply(_SwiGLU, gate_up[..., :d], gate_up[..., d:])
 
 
 # =============================================================================================
@@ -636,7 +647,7 @@ def dwconv_chunked(x, w2, causal=True):
     K = w2.shape[-1]
     if K < 2 or K > 8 or x.shape[-1] % 8:
         return reference.dwconv_chunked(x, w2, causal)
-    return _DWConv.apply(x, w2, bool(causal))
+    return _apply(_DWConv, x, w2, bool(causal))
 
 
 # =============================================================================================
@@ -804,7 +815,7 @@ def attention(q, k, v, window=None, scale=None, cu_seqlens=None, return_lse=Fals
         return reference.attention(q, k, v, window, scale, cu_seqlens, return_lse)
     scale = q.shape[-1] ** -0.5 if scale is None else scale
     seg_start, seg_end = _packed_args(q, k, cu_seqlens)
-    o, lse = _Attention.apply(q, k, v, window, window, scale, False, seg_start, seg_end)
+    o, lse = _apply(_Attention, q, k, v, window, window, scale, False, seg_start, seg_end)
     return (o, lse) if return_lse else o
 
 
@@ -814,7 +825,7 @@ def dual_window_attention(q, k, v, window_teacher, window_student, scale=None, c
         return reference.dual_window_attention(q, k, v, window_teacher, window_student, scale, cu_seqlens)
     scale = q.shape[-1] ** -0.5 if scale is None else scale
     seg_start, seg_end = _packed_args(q, k, cu_seqlens)
-    o_t, o_s, _, _ = _Attention.apply(q, k, v, window_teacher, window_student, scale, True, seg_start, seg_end)
+    o_t, o_s, _, _ = _apply(_Attention, q, k, v, window_teacher, window_student, scale, True, seg_start, seg_end)
     return o_t, o_s
 
 
@@ -891,6 +902,15 @@ def _logits_with_lse(hidden2, w, out):
     return parts
 
 
+def _scale_by(t: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    """t * g for a gradient held since the forward and the scalar that arrives from downstream (on the device)."""
+    if t.dtype != _BF16 or not t.is_contiguous() or t.numel() % 8 or t.data_ptr() % 16:
+        return t * g.to(t.dtype)
+    out = torch.empty_like(t)
+    nv.call("ttcd_scale_by", nv.ptr(t), nv.ptr(out), nv.ptr(g.float().contiguous()), nv.i64(t.numel()), nv.stream_ptr())
+    return out
+
+
 class _CrossEntropy(torch.autograd.Function):
     """Mean CE over valid rows; the gradient (for a loss gradient of one) is computed in the forward."""
 
@@ -917,7 +937,7 @@ class _CrossEntropy(torch.autograd.Function):
 
 
 def cross_entropy(logits, labels, ignore_index=-100, label_smoothing=0.0, z_loss=0.0):
-    return _CrossEntropy.apply(logits, labels, int(ignore_index), float(label_smoothing), float(z_loss))
+    return _apply(_CrossEntropy, logits, labels, int(ignore_index), float(label_smoothing), float(z_loss))
 
 
 def _lce_chunk_rows(n_rows: int, hidden: int, num_chunks: int, sms: int = 148) -> int:
@@ -928,15 +948,6 @@ def _lce_chunk_rows(n_rows: int, hidden: int, num_chunks: int, sms: int = 148) -
     fp32 accumulator is read and written once.  (5003 rows, hidden 2048, vocabulary 128256: eight chunks of 640 rows leave
     108 of 148 SMs idle in every dx and pass over the 1 GB accumulator eight times; three chunks of at most 2304 do not.)"""
     total = -(-n_rows // 128)
-def _scale_by(t: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
-    """t * g for a gradient held since the forward and the scalar that arrives from downstream (on the device)."""
-    if t.dtype != _BF16 or not t.is_contiguous() or t.numel() % 8 or t.data_ptr() % 16:
-        return t * g.to(t.dtype)
-    out = torch.empty_like(t)
-    nv.call("ttcd_scale_by", nv.ptr(t), nv.ptr(out), nv.ptr(g.float().contiguous()), nv.i64(t.numel()), nv.stream_ptr())
-    return out
-
-
     target = max(1, -(-n_rows // max(1, num_chunks)) // 128)
     hi = max(target + target // 4, 20)
     if hi >= total and target >= total:
@@ -1007,7 +1018,7 @@ def linear_cross_entropy(hidden, labels, weight, ignore_index=-100, num_chunks=8
     _check(hidden, "hidden")
     if hidden.shape[0] < 128 or hidden.shape[1] < 64 or weight.shape[0] < 128:       # below one GEMM tile
         return reference.linear_cross_entropy(hidden, labels, weight, None, ignore_index, l2_penalty)
-    return _LinearCrossEntropy.apply(hidden, labels, weight, int(ignore_index), int(num_chunks), float(l2_penalty))
+    return _apply(_LinearCrossEntropy, hidden, labels, weight, int(ignore_index), int(num_chunks), float(l2_penalty))
 
 
 # =============================================================================================
@@ -1174,4 +1185,4 @@ def ttt_scan(z_out, z_tgt, z_hat, beta, w_down, w_update_t, lr: float, cp=None, 
     """Returns ``(y [b,T,C,d_h], norm of the last chunk update)``; see ``_TTTScan``."""
     for name, t in (("z_out", z_out), ("z_tgt", z_tgt), ("z_hat", z_hat)):
         _check(t, name)
-    return _TTTScan.apply(z_out, z_tgt, z_hat, beta, w_down, w_update_t, float(lr), cp, key)
+    return _apply(_TTTScan, z_out, z_tgt, z_hat, beta, w_down, w_update_t, float(lr), cp, key)
