@@ -21,6 +21,11 @@
 // multicast) with per-slot "free" barriers.  One swizzled tile serves as a K-major operand of one MMA and an
 // MN-major operand of another (Q and dO in dkdv, K in dq), so nothing is transposed in memory.
 //
+// What bounds them: the chain S / dP -> element-wise -> accumulate of a step against the other steps in flight (ncu at
+// D = 128: tensor pipe 68 % and 62 % busy, issue 43 % and 33 %).  At D = 64 the 512 TMEM columns hold three S / dP sets
+// instead of two, and the MMAs run two steps ahead.  us at 2 x 10007 tokens, 15/5 heads, D 64, dual window, two sets | three:
+// dkdv 1237 | 1048, dq 832 | 692 (with the second pass's loads in flight over the first).
+//
 // Packed batches (several sequences in one row): per-token `seg_start` / `seg_end` arrays bound the visible keys of
 // a query to its own sequence inside the kernels (the role of flash_attn_varlen_func in fla/layers/attn.py:229-270),
 // and the block ranges are clipped to the sequences that a tile touches.
@@ -51,6 +56,20 @@ __device__ __forceinline__ float ex2(float x) {
 }
 __device__ __forceinline__ void named_barrier_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
+// waits for the tensor-memory loads in flight; the registers pass through, so that nothing that uses them moves ahead of it
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&a)[16], uint32_t (&b)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]), "+r"(a[8]),
+                 "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15])
+               :
+               : "memory");
+  asm volatile(""
+               : "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]), "+r"(b[8]),
+                 "+r"(b[9]), "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15])
+               :
+               : "memory");
 }
 
 // TMEM column offset (inside an S / dP column group of 64) of the 8 packed bf16 columns that hold k-step `k` (16
@@ -174,8 +193,8 @@ __device__ __forceinline__ void dq_elementwise(const uint32_t (&sv)[NC], const u
 template <int D>
 struct DkdvCfg {
   static constexpr int DB = D / 64;
-  static constexpr int NSETS = 2;               // S/dP accumulator sets in TMEM
-  static constexpr int NSLOTS = 4;              // Q/dO tile ring: a tile load has two steps to arrive
+  static constexpr int NSETS = D == 64 ? 3 : 2; // S/dP accumulator sets in TMEM: as many as the 512 columns hold
+  static constexpr int NSLOTS = D == 64 ? 8 : 4;// Q/dO tile ring: a tile load has NSLOTS - NSETS steps to arrive
   static constexpr int SET_COLS = 128;
   static constexpr int KEY_REGION = 128 * 128;  // [128 keys x 64 d] swizzled
   static constexpr int ROW_REGION = 64 * 128;   // [64 rows x 64 d] swizzled
@@ -186,8 +205,9 @@ struct DkdvCfg {
   static constexpr int RING_OFF = V_OFF + DB * KEY_REGION;            // NSLOTS x NTILES x TILE_BYTES
   static constexpr int VEC_OFF = RING_OFF + NSLOTS * NTILES * TILE_BYTES;   // 4 slots x 4 vectors x 64 words
   static constexpr int BAR_OFF = VEC_OFF + 4 * 4 * 64 * 4;
-  // kv_full, tiles_full[NSLOTS], sdp_full[NSETS], ew_done[2], all_done, slot_free[NSLOTS]
-  static constexpr int NBARS = 1 + NSLOTS + NSETS + 2 + 1 + NSLOTS;
+  // kv_full, tiles_full[NSLOTS], sdp_full[NSETS], ew_done[NSETS], all_done, slot_free[NSLOTS]
+  static constexpr int NBARS = 1 + NSLOTS + NSETS + NSETS + 1 + NSLOTS;
+  static_assert(2 * D + NSETS * SET_COLS <= 512, "tensor memory");
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16;
 };
 
@@ -205,8 +225,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   const uint32_t kv_full = bars;
   auto tiles_full = [&](int s) { return bars + 8u * (1 + s); };
   auto sdp_full = [&](int s) { return bars + 8u * (1 + C::NSLOTS + s); };
-  auto ew_done = [&](int g) { return bars + 8u * (1 + C::NSLOTS + C::NSETS + g); };
-  const uint32_t all_done = ew_done(2);
+  auto ew_done = [&](int s) { return bars + 8u * (1 + C::NSLOTS + C::NSETS + s); };
+  const uint32_t all_done = ew_done(C::NSETS);
   auto slot_free = [&](int s) { return all_done + 8u * (1 + s); };   // the MMAs that read ring slot s have completed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::BAR_OFF + C::NBARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -247,9 +267,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
     if (*abort_flag) atomicCAS(&g_status, 0, 399);
     mbar_init(kv_full, 1);
     for (int s = 0; s < C::NSLOTS; ++s) mbar_init(tiles_full(s), 1);
-    for (int s = 0; s < C::NSETS; ++s) mbar_init(sdp_full(s), 1);
-    mbar_init(ew_done(0), 8);
-    mbar_init(ew_done(1), 8);
+    for (int s = 0; s < C::NSETS; ++s) { mbar_init(sdp_full(s), 1); mbar_init(ew_done(s), 8); }
     mbar_init(all_done, 1);
     for (int s = 0; s < C::NSLOTS; ++s) mbar_init(slot_free(s), 1);
     mbar_fence_init();
@@ -262,8 +280,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t t_dk = tmem_base, t_dv = tmem_base + 128;
-  auto t_set = [&](int it) { return tmem_base + 256 + (it & 1) * C::SET_COLS; };  // S^T | dP^T
+  const uint32_t t_dk = tmem_base, t_dv = tmem_base + D;
+  // step `it` works on set it % NSETS for the it / NSETS-th time
+  auto set_of = [&](int it) { return it % C::NSETS; };
+  auto phase_of = [&](int it) { return (it / C::NSETS) & 1; };
+  auto t_set = [&](int it) { return tmem_base + 2 * D + set_of(it) * C::SET_COLS; };  // S^T | dP^T
   const bool healthy = (*abort_flag == 0);
 
   const FastDiv by_steps(steps);
@@ -349,7 +370,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
           const uint32_t ro = ((k / 4) * C::ROW_REGION + (k % 4) * 32) >> 4;
           umma_ss(ts + 64, umma_desc_join(v_lo + ko, HI), umma_desc_join(do_lo + ro, HI), idesc_s, k != 0);
         }
-        umma_commit(sdp_full(it & 1));
+        umma_commit(sdp_full(set_of(it)));
       };
       auto issue_acc = [&](int it) {
         const uint32_t sq = slot_base(it);
@@ -365,19 +386,19 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
           umma_ts(t_dk, ts + 64 + ts_packed_off(k), umma_desc_join(qm_lo + k * (2048 >> 4), HI), idesc_acc, acc | (k != 0));
       };
 
+      // S/dP run NSETS - 1 steps ahead of the accumulate MMAs, so that the element-wise work of a step has as long
       bool ok = mbar_wait(kv_full, 0, abort_flag, 301);
-      if (ok) ok = mbar_wait(tiles_full(0), 0, abort_flag, 302);
-      if (ok) { tc_fence_after_sync(); issue_sdp(0); }
+      auto start = [&](int it) {
+        ok = mbar_wait(tiles_full(it & (C::NSLOTS - 1)), (it / C::NSLOTS) & 1, abort_flag, 303);
+        if (!ok) return;
+        tc_fence_after_sync();
+        issue_sdp(it);  // its TMEM set was last read by the accumulate MMAs of step it - NSETS, issued before
+      };
+      for (int it = 0; it < C::NSETS - 1 && it < n_iters && ok; ++it) start(it);
       for (int it = 0; it < n_iters && ok; ++it) {
-        // S/dP for the step the element-wise warps will need next
-        const int nxt = it + 1;
-        if (nxt < n_iters) {
-          ok = mbar_wait(tiles_full(nxt & (C::NSLOTS - 1)), (nxt / C::NSLOTS) & 1, abort_flag, 303);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_sdp(nxt);  // its TMEM set was last read by the accumulate MMAs of step nxt - 2, issued before
-        }
-        ok = mbar_wait(ew_done(it & 1), (it >> 1) & 1, abort_flag, 305);
+        if (it + C::NSETS - 1 < n_iters) start(it + C::NSETS - 1);
+        if (!ok) break;
+        ok = mbar_wait(ew_done(set_of(it)), phase_of(it), abort_flag, 305);
         if (!ok) break;
         tc_fence_after_sync();
         issue_acc(it);
@@ -420,10 +441,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       const float* vslot = vslot_of(it);
       const float next_stat = (it + 2 < n_iters) ? fetch_stat(it + 2) : 0.f;  // in flight during this step
       named_barrier_sync(1 + grp, 256);
-      ok = wait_all(sdp_full(it & 1), (it >> 1) & 1, 311);
+      ok = wait_all(sdp_full(set_of(it)), phase_of(it), 311);
       if (!ok) break;
       tc_fence_after_sync();
-      const uint32_t ts = t_set(it) + lane_addr + part * 32;      // set == grp
+      const uint32_t ts = t_set(it) + lane_addr + part * 32;
       const int qlo_b = r0 + off, qhi_b = r0 + 63 + off;
       const bool key_ok = key < p.Tk;
       // visible pairs of this step:  qpos - hi < key <= qpos - lo  (dual: student part, then teacher-only part)
@@ -455,7 +476,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
       if (it + 2 < n_iters) vslot_of(it + 2)[ctid] = finish_stat(next_stat);
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ew_done(it & 1));
+      if (lane == 0) mbar_arrive(ew_done(set_of(it)));
     }
     // epilogue: dK, dV -> global (this thread: key row `krow`, one half of the D columns; group 0 writes dK and
     // group 1 dV)
@@ -501,7 +522,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
 template <int D, bool DUAL>
 struct DqCfg {
   static constexpr int DB = D / 64;
-  static constexpr int NSLOTS = DUAL ? 4 : 5;      // K/V ring: a tile load has NSLOTS - 2 steps to arrive
+  static constexpr int NSETS = D == 64 ? 3 : 2;    // S/dP accumulator sets in TMEM: as many as the 512 columns hold
+  static constexpr int NSLOTS = D == 64 ? 8 : DUAL ? 4 : 5;      // K/V ring: a tile load has NSLOTS - NSETS steps to arrive
   static constexpr int SET_COLS = 128;
   static constexpr int Q_REGION = 128 * 128;
   static constexpr int KV_REGION = 64 * 128;
@@ -511,12 +533,13 @@ struct DqCfg {
   static constexpr int DOC_OFF = DOT_OFF + DB * Q_REGION;                 // dO': only used when DUAL
   static constexpr int RING_OFF = DOC_OFF + (DUAL ? DB * Q_REGION : 0);   // NSLOTS x (K, V)
   static constexpr int BAR_OFF = RING_OFF + NSLOTS * 2 * KV_BYTES;
-  // q_full, kv_full[NSLOTS], sdp_full[2], ew_done[2], a_ready, all_done, slot_free[NSLOTS]
-  static constexpr int NBARS = 1 + NSLOTS + 2 + 2 + 2 + NSLOTS;
-  // 128 (dQ) + 2 x 128 (S | dP sets) leaves 128 columns: Q and one dO as bf16 A operands in tensor memory (single
+  // q_full, kv_full[NSLOTS], sdp_full[NSETS], ew_done[NSETS], a_ready, all_done, slot_free[NSLOTS]
+  static constexpr int NBARS = 1 + NSLOTS + NSETS + NSETS + 2 + NSLOTS;
+  // D (dQ) + NSETS x 128 (S | dP sets) leaves D columns: Q and one dO as bf16 A operands in tensor memory (single
   // window: dO; dual window: dO', used by the steps inside the student window; the teacher-only steps read dO_T from
   // shared memory)
   static constexpr int A_COLS = D / 2;
+  static_assert(D + NSETS * SET_COLS + 2 * A_COLS <= 512, "tensor memory");
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16;
 };
 
@@ -534,8 +557,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
   const uint32_t q_full = bars;
   auto kv_full = [&](int s) { return bars + 8u * (1 + s); };
   auto sdp_full = [&](int s) { return bars + 8u * (1 + C::NSLOTS + s); };
-  auto ew_done = [&](int g) { return bars + 8u * (3 + C::NSLOTS + g); };
-  const uint32_t a_ready = ew_done(2);
+  auto ew_done = [&](int s) { return bars + 8u * (1 + C::NSLOTS + C::NSETS + s); };
+  const uint32_t a_ready = ew_done(C::NSETS);
   const uint32_t all_done = a_ready + 8u;
   auto slot_free = [&](int s) { return all_done + 8u * (1 + s); };   // the MMAs that read ring slot s have completed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + C::BAR_OFF + C::NBARS * 8);
@@ -588,10 +611,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
     if (*abort_flag) atomicCAS(&g_status, 0, 398);
     mbar_init(q_full, 1);
     for (int s = 0; s < C::NSLOTS; ++s) mbar_init(kv_full(s), 1);
-    mbar_init(sdp_full(0), 1);
-    mbar_init(sdp_full(1), 1);
-    mbar_init(ew_done(0), 8);
-    mbar_init(ew_done(1), 8);
+    for (int s = 0; s < C::NSETS; ++s) { mbar_init(sdp_full(s), 1); mbar_init(ew_done(s), 8); }
     mbar_init(a_ready, NEW);
     mbar_init(all_done, 1);
     for (int s = 0; s < C::NSLOTS; ++s) mbar_init(slot_free(s), 1);
@@ -608,9 +628,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
   const uint32_t t_dq = tmem_base;
   // every mode: dS goes back into tensor memory over the S columns it was computed from (bf16 pairs) and feeds the
   // dQ MMA as its TMEM A operand; the S MMA that next writes those columns is issued after that dQ MMA
-  const uint32_t t_qa = tmem_base + 128 + 2 * C::SET_COLS;      // [384, 384 + D/2): Q, then dO (dual: dO')
+  const uint32_t t_qa = tmem_base + D + C::NSETS * C::SET_COLS; // Q, then dO (dual: dO'), D / 2 columns each
   const uint32_t t_doa = t_qa + C::A_COLS;
-  auto t_set = [&](int it) { return tmem_base + 128 + (it & 1) * C::SET_COLS; };  // S | dP
+  // step `it` works on set it % NSETS for the it / NSETS-th time
+  auto set_of = [&](int it) { return it % C::NSETS; };
+  auto phase_of = [&](int it) { return (it / C::NSETS) & 1; };
+  auto t_set = [&](int it) { return tmem_base + D + set_of(it) * C::SET_COLS; };  // S | dP
   const bool healthy = (*abort_flag == 0);
 
   if (warp == NEW + 1 && healthy) {
@@ -681,20 +704,22 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
             umma_ss(ts + 64, umma_desc_join(dot_lo + qo, HI), umma_desc_join(v_lo + ko, HI), idesc_s, k != 0);
           }
         }
-        umma_commit(sdp_full(it & 1));
+        umma_commit(sdp_full(set_of(it)));
       };
-      bool ok = true;
-      ok = mbar_wait(q_full, 0, abort_flag, 321) && mbar_wait(kv_full(0), 0, abort_flag, 322);
+      bool ok = mbar_wait(q_full, 0, abort_flag, 321);
       if (ok) ok = mbar_wait(a_ready, 0, abort_flag, 326);      // Q and dO copied into tensor memory
-      if (ok) { tc_fence_after_sync(); issue_sdp(0); }
+      // S/dP run NSETS - 1 steps ahead of the dQ MMAs, so that the element-wise work of a step has as long
+      auto start = [&](int it) {
+        ok = mbar_wait(kv_full(by_slots.mod(it)), by_slots.div(it) & 1, abort_flag, 323);
+        if (!ok) return;
+        tc_fence_after_sync();
+        issue_sdp(it);  // its TMEM set was last read by the dQ MMA of step it - NSETS, issued before
+      };
+      for (int it = 0; it < C::NSETS - 1 && it < n_iters && ok; ++it) start(it);
       for (int it = 0; it < n_iters && ok; ++it) {
-        if (it + 1 < n_iters) {
-          ok = mbar_wait(kv_full(by_slots.mod(it + 1)), by_slots.div(it + 1) & 1, abort_flag, 323);
-          if (!ok) break;
-          tc_fence_after_sync();
-          issue_sdp(it + 1);  // its TMEM set was last read by the dQ MMA of step it - 1, issued before
-        }
-        ok = mbar_wait(ew_done(it & 1), (it >> 1) & 1, abort_flag, 325);
+        if (it + C::NSETS - 1 < n_iters) start(it + C::NSETS - 1);
+        if (!ok) break;
+        ok = mbar_wait(ew_done(set_of(it)), phase_of(it), abort_flag, 325);
         if (!ok) break;
         tc_fence_after_sync();
         // the K tile as the MN-major B operand: 64 keys of the contraction, the next 64 columns KV_REGION bytes on
@@ -752,7 +777,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
     }
     for (int it = grp; it < n_iters && ok; it += 2) {
       const int key0 = iter_key0(it) + part * 32;
-      ok = wait_all(sdp_full(it & 1), (it >> 1) & 1, 331);
+      ok = wait_all(sdp_full(set_of(it)), phase_of(it), 331);
       if (!ok) break;
       tc_fence_after_sync();
       const uint32_t ts = t_set(it) + lane_addr + part * 32;
@@ -762,24 +787,28 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
       const int lo = combine ? (inner ? 0 : p.w_s) : 0, hi = combine ? (inner ? p.w_s : p.w_t) : p.w_t;
       const float del = (combine && inner) ? del_c : del_t;
       const bool full = (kb0 + 63 <= qlo - lo) && (kb0 > qhi - hi) && (kb0 >= seg_last);
+      // two passes of 16 columns; the second one's loads are in flight over the first
+      uint32_t sv[2][NC], dpt[2][NC];
+      tmem_ld_n<NC>(ts, sv[0]);
+      tmem_ld_n<NC>(ts + 64, dpt[0]);
+      tmem_ld_wait_for(sv[0], dpt[0]);
+      tmem_ld_n<NC>(ts + NC, sv[1]);
+      tmem_ld_n<NC>(ts + 64 + NC, dpt[1]);
 #pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {          // two passes of 16 columns keep the registers low
-        uint32_t sv[NC], dpt[NC];
-        tmem_ld_n<NC>(ts + hh * NC, sv);
-        tmem_ld_n<NC>(ts + 64 + hh * NC, dpt);
-        tmem_ld_wait();
+      for (int hh = 0; hh < 2; ++hh) {
+        if (hh == 1) tmem_ld_wait_for(sv[1], dpt[1]);
         uint32_t dsp[NC / 2];
         const int kpos0 = key0 + hh * NC;
         if (full)
-          dq_elementwise<false, NC>(sv, dpt, p.scale_log2, nlse_t, del, qpos, kpos0, lo, hi, seg_lo, dsp);
+          dq_elementwise<false, NC>(sv[hh], dpt[hh], p.scale_log2, nlse_t, del, qpos, kpos0, lo, hi, seg_lo, dsp);
         else
-          dq_elementwise<true, NC>(sv, dpt, p.scale_log2, nlse_t, del, qpos, kpos0, lo, hi, seg_lo, dsp);
+          dq_elementwise<true, NC>(sv[hh], dpt[hh], p.scale_log2, nlse_t, del, qpos, kpos0, lo, hi, seg_lo, dsp);
         tmem_st_n<NC / 2>(ts + hh * (NC / 2), dsp);    // over this thread's own S columns (already read)
       }
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(ew_done(it & 1));
+      if (lane == 0) mbar_arrive(ew_done(set_of(it)));
     }
     if (ok) {
       ok = wait_all(all_done, 0, 333);
