@@ -1,5 +1,5 @@
 // The chunk-to-chunk chain of the (gated) delta rule (sm_100a; the two products of a step, 64 x D x 32 each, run on the
-// tensor cores as bf16 mma.sync tiles with fp32 accumulation: they are far too small for a tcgen05 pipeline; the point
+// tensor cores as TF32 mma.sync tiles with fp32 accumulation: they are far too small for a tcgen05 pipeline; the point
 // of the kernel is to run the n dependent steps in ONE launch with the state resident in registers).
 //
 // For one (batch, head) pair, S [D, Dv] the running state and i the chunk index:
@@ -15,8 +15,9 @@
 // b_i [64, D] (bf16) in shared memory with asynchronous 16-byte copies that overlap the publication of S.  S [D, columns]
 // lives in the accumulator registers of the second product (D / 32 m16n8 tiles per warp) across chunks, in fp32, and is
 // mirrored in shared memory, rounded to bf16, as the B operand of the first; y is rounded the same way for the second.
-// Every operand of a product is thus a bf16 value (the precision the reference's Triton kernels multiply at) and comes to
-// the products by ldmatrix, the sums and the state stay fp32.
+// Every operand of a product is thus a bf16 value (the precision the reference's Triton kernels multiply at), comes to the
+// products by ldmatrix and is widened to TF32 there (exactly; bf16 products of 16 would save 10 % of the forward, but sum
+// in another order, which a deep model's gradients show), the sums and the state stay fp32.
 // The only asynchronous copies are the CTA's own cp.async groups (waited for with wait_group); nothing here waits on
 // another CTA, so nothing can spin.
 #include "common.cuh"
@@ -43,10 +44,18 @@ __device__ __forceinline__ void dc_cp_async16(uint32_t dst_smem, const void* src
 }
 __device__ __forceinline__ void dc_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void dc_cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+__device__ __forceinline__ void dc_mma8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 16 of the contraction as two TF32 products of 8 (a bf16 value is an exact TF32 operand after a 16-bit shift).  A register
+// of a bf16 fragment holds k = 2 c and 2 c + 1; they take the slots c and c + 4 of both operands.
+__device__ __forceinline__ void dc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  constexpr uint32_t HI = 0xffff0000u;
+  dc_mma8(d, a[0] << 16, a[1] << 16, a[0] & HI, a[1] & HI, b0 << 16, b0 & HI);
+  dc_mma8(d, a[2] << 16, a[3] << 16, a[2] & HI, a[3] & HI, b1 << 16, b1 & HI);
 }
 __device__ __forceinline__ void dc_ldm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -97,8 +106,9 @@ delta_chain_kernel(const DeltaChainParams p) {
   const float* x_base = p.x + bh * p.n * DC_C * Dv + col0;
   float* y_base = p.y + bh * p.n * DC_C * Dv + col0;
   float* st_base = p.states + bh * p.n * D * Dv + col0;
-  const float* add_base = p.add != nullptr ? p.add + bh * p.n * D * Dv + col0 : nullptr;
-  const float* dot_base = p.dot_with != nullptr ? p.dot_with + bh * p.n * D * Dv + col0 : nullptr;
+  // (only the two-stage form serves the reverse chain)
+  const float* add_base = PIPE && p.add != nullptr ? p.add + bh * p.n * D * Dv + col0 : nullptr;
+  const float* dot_base = PIPE && p.dot_with != nullptr ? p.dot_with + bh * p.n * D * Dv + col0 : nullptr;
   // the warp's tiles of S: m-tile mt0 + m (rows 16 (mt0 + m) + g, + 8), n-tiles nt0 .. nt0 + NT - 1 (columns 8 nt + 2 c, + 1)
   const int mt0 = (warp * TPW) / NTM, nt0 = (warp * TPW) % NTM;
   // the warp's YT tiles of y: m-tile warp / 2, n-tiles YT (warp % 2) ..
@@ -167,7 +177,7 @@ delta_chain_kernel(const DeltaChainParams p) {
     __syncthreads();
     if (PIPE && step + 1 < p.n) load_stage(step + 1);        // the other stage was last read before this barrier
     const float gm = p.gamma[bh * p.n + i];
-    // a tile of the warp's elements of a [D, Dv] tensor of step i: with PIPE issued a product before its use
+    // a tile of the warp's elements of a [D, Dv] tensor of step i: issued a product (or a barrier) before its use
     float ld[MT][NT][4];
     auto load_tile = [&](const float* base) {
 #pragma unroll
@@ -180,7 +190,7 @@ delta_chain_kernel(const DeltaChainParams p) {
           ld[m][t][0] = lo.x; ld[m][t][1] = lo.y; ld[m][t][2] = hi.x; ld[m][t][3] = hi.y;
         }
     };
-    if (PIPE && dot_base != nullptr) load_tile(dot_base);
+    if (dot_base != nullptr) load_tile(dot_base);
     // ---- y = x + sign_a * (a S): the warp's YT 16 x 8 tiles
     const uint32_t stage = st_addr + (PIPE ? (step & 1) * 2u * STAGE : 0u);
     {
@@ -208,26 +218,18 @@ delta_chain_kernel(const DeltaChainParams p) {
     }
     if (step + 1 < p.n) load_x(step + 1);
     if (dot_base != nullptr) {
-      if (!PIPE) load_tile(dot_base);
       float part = 0.f;
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
         for (int t = 0; t < NT; ++t)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) part = fmaf(s[m][t][e], ld[m][t][e], part);
+          part += s[m][t][0] * ld[m][t][0] + s[m][t][1] * ld[m][t][1] + s[m][t][2] * ld[m][t][2] + s[m][t][3] * ld[m][t][3];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
       if (lane == 0) red[warp] = part;
     }
-    // ---- S = gamma S + sign_b * (b^T y) + add, accumulated in place
-    if (PIPE && add_base != nullptr) load_tile(add_base);
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-      for (int t = 0; t < NT; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[m][t][e] *= gm;
+    // ---- S = gamma S + add + sign_b * (b^T y), accumulated in place; the addend is on its way over the barrier
+    if (add_base != nullptr) load_tile(add_base);
     __syncthreads();
     if (dot_base != nullptr && threadIdx.x == 0) {
       float tot = 0.f;
@@ -235,6 +237,12 @@ delta_chain_kernel(const DeltaChainParams p) {
       for (int wv = 0; wv < DC_THREADS / 32; ++wv) tot += red[wv];
       p.dot_out[(bh * p.n + i) * (Dv / 32) + blockIdx.x] = tot;        // rows of Dv / 32 slots (zero-filled by the caller)
     }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[m][t][e] = add_base != nullptr ? fmaf(gm, s[m][t][e], ld[m][t][e]) : gm * s[m][t][e];
 #pragma unroll
     for (int k0 = 0; k0 < DC_C; k0 += 16) {
       uint32_t b[NT][2];
@@ -246,15 +254,6 @@ delta_chain_kernel(const DeltaChainParams p) {
 #pragma unroll
         for (int t = 0; t < NT; ++t) dc_mma(s[m][t], a, b[t][0], b[t][1]);
       }
-    }
-    if (add_base != nullptr) {
-      if (!PIPE) load_tile(add_base);
-#pragma unroll
-      for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) s[m][t][e] += ld[m][t][e];
     }
     // (what this step still reads, b and y, is rewritten after the next step's first barrier; PIPE's only stage 0 / 1
     // alternate, a single stage is rewritten at once)
@@ -287,9 +286,9 @@ static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t st
 // The chain is a string of dependent steps, so what a step waits for is what it costs.  Two stages of a / b, with the
 // addend and the states of the dot product in flight over the products, pay where a CTA has its SM to itself (D = 256,
 // at most one CTA per SM) and in the reverse chain, which reads two [D, Dv] tensors more; elsewhere more CTAs per SM hide
-// each other's waits.  us, one stage | two stages (BH x steps, D, Dv):  forward 32 x 64, 128, 128: 160 | 169;
-// 12 x 47, 256, 512: 293 | 246; 96 x 64, 256, 512: 1801 | 1882.  reverse, the same: 299 | 232; 557 | 419; 3749 | 3305.
-// (TF32 products out of scalar 16-bit shared-memory reads, before: forward 291; 455; 2769, reverse 387; 720; 4466.)
+// each other's waits.  us (BH x steps, D, Dv), before (scalar 16-bit shared-memory reads, every tile waited for) | now:
+// forward 32 x 64, 128, 128: 291 | 179; 12 x 47, 256, 512: 455 | 295; 96 x 64, 256, 512: 2769 | 2045 (one stage);
+// reverse, the same: 387 | 240; 720 | 429; 4466 | 3380 (one stage instead of two: 299; 557; 3749).
 template <int D, int COLS>
 static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t stream) {
   const bool alone = D == 256 && static_cast<int64_t>(p.Dv / COLS) * BH <= sm_count();
