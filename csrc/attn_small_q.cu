@@ -37,6 +37,7 @@ struct SmallQParams {
   float* part_o;        // [B, H, Tq, splits, D]
   float* part_ml;       // [B, H, Tq, splits, 2]  (max in log2 units, sum)
   bf16* out;            // [B, Tq, H, D]
+  int* turns;           // optional [B * HK], zero: CTAs that have finished; the last one of a head merges the splits
   const int* kv_len;    // optional device word: the number of valid keys (<= Tk); read at launch time
   int B, Tq, Tk, H, HK, splits, window;
   int64_t ldq, ldk, ldv, sq, sk, sv;
@@ -183,7 +184,6 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, R <= 2 ? 2 : 1) attn_decode_pa
   constexpr int TURN = DEC_WARPS * C::KEYS;
   const int per = ((Tk - first + p.splits - 1) / p.splits + TURN - 1) / TURN * TURN;
   const int lo = first + split * per, hi = min(Tk, lo + per);
-
   // this lane's 8 dims of every query pair (pairs beyond the real ones: zero)
   float2 q[R][4];
 #pragma unroll
@@ -346,6 +346,55 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, R <= 2 ? 2 : 1) attn_decode_pa
       p.part_ml[pidx * 2 + 1] = s;
     }
   }
+  if (p.turns == nullptr) return;
+  // ---- the last CTA of this (sample, head) folds the splits, as the merge kernel below does (a launch less: 3 us)
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int* turn = p.turns + b * p.HK + kvh;
+    s_last = atomicAdd(turn, 1) == p.splits - 1;
+    if (s_last) *turn = 0;                          // as the next call finds it
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  constexpr int DPL = D / 32, WPP = DEC_WARPS / R;  // warps per pair
+  const int r = warp / WPP, sub = warp % WPP;
+  float* l_parts = &s_l[0][0];
+  if (r < pairs) {
+    const int64_t item = (static_cast<int64_t>(b) * p.H + kvh * G + r % G) * p.Tq + r / G;
+    const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + item * p.splits;
+    float M = -INFINITY;
+    for (int s = lane; s < p.splits; s += 32) M = fmaxf(M, __ldcg(&ml[s]).x);
+    M = warp_max(M);
+    float acc[DPL], lsum = 0.f;
+#pragma unroll
+    for (int e = 0; e < DPL; ++e) acc[e] = 0.f;
+#pragma unroll 8
+    for (int s = sub; s < p.splits; s += WPP) {
+      const float2 t = __ldcg(&ml[s]);
+      float x[DPL];
+#pragma unroll
+      for (int e = 0; e < DPL; ++e) x[e] = __ldcg(p.part_o + (item * p.splits + s) * D + lane * DPL + e);
+      const bool some = t.x != -INFINITY;
+      const float w = some ? exp2f(t.x - M) : 0.f;
+      lsum = fmaf(some ? t.y : 0.f, w, lsum);
+#pragma unroll
+      for (int e = 0; e < DPL; ++e) acc[e] = fmaf(some ? x[e] : 0.f, w, acc[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < DPL; ++e) s_o[sub][r][lane * DPL + e] = acc[e];
+    if (lane == 0) l_parts[warp] = lsum;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < pairs * D; i += DEC_WARPS * 32) {
+    const int pr = i / D, d = i % D;
+    float acc = 0.f, tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < WPP; ++w) { acc += s_o[w][pr][d]; tot += l_parts[pr * WPP + w]; }
+    p.out[((static_cast<int64_t>(b) * p.Tq + pr / G) * p.H + kvh * G + pr % G) * D + d] = __float2bfloat16(acc * (tot > 0.f ? 1.f / tot : 0.f));
+  }
 }
 
 // out[b, row, h, :] = sum_s o_s 2^(m_s - M) / sum_s l_s 2^(m_s - M): one CTA per item, warps over the splits, a lane
@@ -406,7 +455,7 @@ static int launch_decode(const SmallQParams& p, cudaStream_t stream) {
   auto kern = pairs <= 1 ? attn_decode_partial_kernel<D, 1> : pairs <= 2 ? attn_decode_partial_kernel<D, 2>
               : pairs <= 4 ? attn_decode_partial_kernel<D, 4> : attn_decode_partial_kernel<D, 8>;
   const int rc = launch_dependent(kern, dim3(p.splits, p.HK, p.B), dim3(DEC_WARPS * 32), 0, stream, p);
-  return rc != TTCD_OK ? rc : launch_merge<D>(p, stream);
+  return rc != TTCD_OK || p.turns != nullptr ? rc : launch_merge<D>(p, stream);
 }
 
 template <int D>
@@ -439,7 +488,7 @@ static int small_q_params(ttcd::SmallQParams& p, const void* q, const void* k, c
   if (ldk % 8 != 0 || ldv % 8 != 0 || sk % 8 != 0 || sv % 8 != 0) return TTCD_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(k) & 15u) || (reinterpret_cast<uintptr_t>(v) & 15u)) return TTCD_ERR_ARG;
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
-  p.out = static_cast<bf16*>(out); p.part_o = part_o; p.part_ml = part_ml; p.kv_len = kv_len;
+  p.out = static_cast<bf16*>(out); p.part_o = part_o; p.part_ml = part_ml; p.kv_len = kv_len; p.turns = nullptr;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.HK = HK; p.splits = splits; p.window = window;
   p.ldq = ldq; p.ldk = ldk; p.ldv = ldv; p.sq = sq; p.sk = sk; p.sv = sv;
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -463,10 +512,12 @@ TTCD_EXPORT int ttcd_attn_small_q(const void* q, const void* k, const void* v, v
 
 // The same call for at most 8 (query row, head of the group) pairs per key/value head: Tq * (H / HK) <= 8.  q rows are
 // 16-byte aligned too; splits is any number from 1 to 65535 (the kernel cuts the filled keys into that many ranges).
+// turns (may be null): int [B * HK], zero before the first call and left so by every call; calls that may overlap need their
+// own.  With it the last CTA of a head merges the splits, without it a second launch does.
 TTCD_EXPORT int ttcd_attn_decode(const void* q, const void* k, const void* v, void* out, float* part_o, float* part_ml,
                                  int B, int Tq, int Tk, int H, int HK, int D, long long ldq, long long ldk, long long ldv,
                                  long long sq, long long sk, long long sv, int window, float scale, int splits,
-                                 const int* kv_len, void* stream_ptr) {
+                                 int* turns, const int* kv_len, void* stream_ptr) {
   using namespace ttcd;
   if (splits < 1 || splits > 65535 || B > 65535 || HK > 65535) return TTCD_ERR_ARG;
   SmallQParams p;
@@ -474,6 +525,7 @@ TTCD_EXPORT int ttcd_attn_decode(const void* q, const void* k, const void* v, vo
                                 splits, kv_len);
   if (rc != TTCD_OK) return rc;
   if (Tq * (H / HK) > 8 || ldq % 8 != 0 || sq % 8 != 0 || (reinterpret_cast<uintptr_t>(q) & 15u)) return TTCD_ERR_ARG;
+  p.turns = turns;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   return D == 128 ? launch_decode<128>(p, stream)
                   : launch_decode<64>(p, stream);

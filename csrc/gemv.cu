@@ -15,7 +15,10 @@
 // issued before it waits for that kernel when the caller says that no kernel still running can be writing w.
 //
 // Measured (us per launch in a graph, weights from HBM; 4096x1024 | 1024x2048 | 6144x1024 | 1024x3072 | 151936x1024):
-//   one warp per column, fp32 FMAs   1 row 3.4 | 4.3 | 4.4 | 5.6 | 49     8 rows 8.1 | 9.9 | 11.6 | 13.8 | 180
+//   this kernel                      1 row 4.1 | 3.0 | 5.5 | 3.6 | 50     8 rows 4.3 | 3.3 | 5.8 | 4.0 | 51     16 rows 5.4 | 3.6 | 5.8 | 5.2 | 74
+//   one warp per column, fp32 FMAs   1 row 3.4 | 4.3 | 4.4 | 5.6 | 49     8 rows 8.1 | 9.9 | 11.6 | 13.8 | 180    16 rows 14 | 17 | 19 | 23 | 342
+// (before; at one row it gained a little where a CTA has more than one group, which the norm, SwiGLU and the early start
+// of the weights pay back in a decode step).
 #include "common.cuh"
 
 #include <algorithm>
@@ -55,44 +58,50 @@ __device__ __forceinline__ uint32_t gv_norm2(uint32_t x, uint32_t w, float r) {
 __host__ __device__ constexpr int gv_pitch(int kc) { return kc * 2 + ((64 - (kc * 2) % 128) + 128) % 128; }      // bytes
 
 __host__ __device__ constexpr int gv_xs(bool hi, bool norm) { return hi || norm ? 8 : 12; }
+__host__ __device__ constexpr int gv_slots(bool hi) { return 148 * (hi ? 1 : 2); }      // CTAs that run at once
 template <int N>
 __device__ __forceinline__ void gv_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// HI: rows 8 .. 15 of x exist.  STAGES: depth of the ring.
-template <bool HI, bool SWIGLU, bool NORM, int STAGES>
+// HI: rows 8 .. 15 of x exist.  WIDE: groups of 16 columns.  STAGES: depth of the ring.
+template <bool HI, bool SWIGLU, bool NORM, bool WIDE, int STAGES>
 __global__ void __launch_bounds__(GV_WARPS * 32, (HI ? 1 : 2)) gemv_small_kernel(const GemvParams p) {
-  constexpr int ROWS = SWIGLU ? 16 : 8;                    // rows of w per group
-  constexpr int T = SWIGLU ? 2 : 1;
+  static_assert(!(SWIGLU && WIDE), "one or the other");
+  constexpr int T = SWIGLU || WIDE ? 2 : 1;                // n-tiles of 8 rows of w per group
+  constexpr int ROWS = 8 * T, COLS = WIDE ? 16 : 8;        // rows of w, columns of y per group
   constexpr int XS = gv_xs(HI, NORM);                         // 32-wide k steps of x a warp holds in registers
   constexpr int KC = XS * 32 * GV_WARPS;                   // columns of w in a stage
   extern __shared__ __align__(16) uint8_t gv_smem[];
   __shared__ float part[GV_WARPS][T][16][8];
   __shared__ float ssum[GV_WARPS][16];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
-  const int groups = (p.N + 7) / 8, chunks = (p.K + KC - 1) / KC;
+  const int groups = (p.N + COLS - 1) / COLS, chunks = (p.K + KC - 1) / KC;
   const int mine = (groups - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
   const int items = mine * chunks;                         // (group, chunk of K) pairs, chunk fastest
   const int pitch = gv_pitch(min(p.K, KC)), stage_bytes = ROWS * pitch;
   const uint32_t sbase = smem_u32(gv_smem);
-  // row r of a group: column 8 group + r of y (SWIGLU: r - 8 for the up half); columns past N re-read the last one
-  auto load_w = [&](int it) {
-    if (it < items) {
-      const int n0 = (static_cast<int>(blockIdx.x) + it / chunks * static_cast<int>(gridDim.x)) * 8, kc0 = it % chunks * KC;
-      const int vecs = min(KC, p.K - kc0) / 8;
-      const uint32_t dst = sbase + (it % STAGES) * stage_bytes;
+  // row r of a group: column COLS group + r of y (SWIGLU: r - 8 for the up half); columns past N re-read the last one.
+  // Called for items 0, 1, 2, ... in turn: the next one's group, chunk and stage are counted, not divided for.
+  int next = 0, next_n0 = static_cast<int>(blockIdx.x) * COLS, next_ch = 0, next_stage = 0;
+  auto load_next = [&]() {
+    if (next < items) {
+      const int kc0 = next_ch * KC, vecs = min(KC, p.K - kc0) / 8;
+      const uint32_t dst = sbase + next_stage * stage_bytes;
 #pragma unroll
       for (int r = warp; r < ROWS; r += GV_WARPS) {
-        const int col = min(n0 + (r & 7), p.N - 1) + (r >= 8 ? p.N : 0);
+        const int col = SWIGLU ? min(next_n0 + (r & 7), p.N - 1) + (r >= 8 ? p.N : 0) : min(next_n0 + r, p.N - 1);
         const bf16* src = p.w + static_cast<int64_t>(col) * p.ldw + kc0;
 #pragma unroll 4
         for (int v = lane; v < vecs; v += 32) gv_cp_async16(dst + r * pitch + v * 16, src + v * 8);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");   // (an empty group keeps the count)
+    ++next;
+    if (++next_stage == STAGES) next_stage = 0;
+    if (++next_ch == chunks) { next_ch = 0; next_n0 += static_cast<int>(gridDim.x) * COLS; }
   };
   auto fill = [&]() {
 #pragma unroll
-    for (int s = 0; s < STAGES; ++s) load_w(s);
+    for (int s = 0; s < STAGES; ++s) load_next();
   };
   if (p.early_w) fill();
   pdl_wait();
@@ -144,8 +153,8 @@ __global__ void __launch_bounds__(GV_WARPS * 32, (HI ? 1 : 2)) gemv_small_kernel
   }
 
   float acc[T][4];
+  int ch = 0, stage = 0, n0 = static_cast<int>(blockIdx.x) * COLS;
   for (int it = 0; it < items; ++it) {
-    const int ch = it % chunks;
     if (ch == 0) {
 #pragma unroll
       for (int t = 0; t < T; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
@@ -153,7 +162,8 @@ __global__ void __launch_bounds__(GV_WARPS * 32, (HI ? 1 : 2)) gemv_small_kernel
     if (!NORM && chunks > 1 && it > 0) load_x(ch);
     gv_cp_async_wait<STAGES - 1>();
     __syncthreads();
-    const uint8_t* ws = gv_smem + (it % STAGES) * stage_bytes;
+    const uint8_t* ws = gv_smem + stage * stage_bytes;
+    if (++stage == STAGES) stage = 0;
 #pragma unroll
     for (int u = 0; u < XS; ++u) {
       if (u < per) {
@@ -175,51 +185,67 @@ __global__ void __launch_bounds__(GV_WARPS * 32, (HI ? 1 : 2)) gemv_small_kernel
       }
     }
     __syncthreads();                                       // the stage is free, the partial sums are there
-    load_w(it + STAGES);
-    if (last && threadIdx.x < p.M * 8) {
-      const int col = threadIdx.x & 7, m = threadIdx.x >> 3;
-      const int n = (static_cast<int>(blockIdx.x) + it / chunks * static_cast<int>(gridDim.x)) * 8 + col;
-      if (n < p.N) {
-        float v = 0.f;
+    load_next();
+    if (last) {
+      if (static_cast<int>(threadIdx.x) < p.M * COLS) {
+        const int col = threadIdx.x % COLS, m = threadIdx.x / COLS, n = n0 + col;
+        if (n < p.N) {
+          float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < GV_WARPS; ++w) v += part[w][0][m][col];
-        bf16 out = __float2bfloat16(v * p.alpha);
-        if constexpr (SWIGLU) {
-          float u = 0.f;
+          for (int w = 0; w < GV_WARPS; ++w) v += part[w][WIDE ? col >> 3 : 0][m][col & 7];
+          bf16 out = __float2bfloat16(v * p.alpha);
+          if constexpr (SWIGLU) {
+            float u = 0.f;
 #pragma unroll
-          for (int w = 0; w < GV_WARPS; ++w) u += part[w][T - 1][m][col];
-          const float gate = __bfloat162float(out), up = __bfloat162float(__float2bfloat16(u * p.alpha));
-          out = __float2bfloat16(gate / (1.f + __expf(-gate)) * up);
+            for (int w = 0; w < GV_WARPS; ++w) u += part[w][T - 1][m][col];
+            const float gate = __bfloat162float(out), up = __bfloat162float(__float2bfloat16(u * p.alpha));
+            out = __float2bfloat16(gate / (1.f + __expf(-gate)) * up);
+          }
+          if (p.res != nullptr) out = __float2bfloat16(__bfloat162float(out) + __bfloat162float(p.res[m * p.ldres + n]));
+          p.y[m * p.ldy + n] = out;
         }
-        if (p.res != nullptr) out = __float2bfloat16(__bfloat162float(out) + __bfloat162float(p.res[m * p.ldres + n]));
-        p.y[m * p.ldy + n] = out;
       }
+      ch = 0;
+      n0 += static_cast<int>(gridDim.x) * COLS;
+    } else {
+      ++ch;
     }
     // (the next item's partial sums are written after its first barrier)
   }
 }
 
-template <bool HI, bool SWIGLU, bool NORM, int STAGES>
+template <bool HI, bool SWIGLU, bool NORM, bool WIDE, int STAGES>
 static int launch_gemv(const GemvParams& p, int smem, cudaStream_t stream) {
-  auto kern = gemv_small_kernel<HI, SWIGLU, NORM, STAGES>;
+  auto kern = gemv_small_kernel<HI, SWIGLU, NORM, WIDE, STAGES>;
   static bool configured = false;
   if (!configured) {
     TTCD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     configured = true;
   }
   // equal turns: as many CTAs as run at once at most, each with the same number of groups (the last ones one less)
-  const int groups = (p.N + 7) / 8, slots = 148 * (HI ? 1 : 2), turns = (groups + slots - 1) / slots;
+  constexpr int cols = WIDE ? 16 : 8;
+  const int groups = (p.N + cols - 1) / cols, slots = gv_slots(HI), turns = (groups + slots - 1) / slots;
   return launch_dependent(kern, dim3((groups + turns - 1) / turns), dim3(GV_WARPS * 32), smem, stream, p);
+}
+
+template <bool HI, bool SWIGLU, bool NORM, bool WIDE>
+static int stages_gemv(const GemvParams& p, cudaStream_t stream) {
+  constexpr int KC = gv_xs(HI, NORM) * 32 * GV_WARPS;
+  const int stage = (SWIGLU || WIDE ? 16 : 8) * gv_pitch(std::min(p.K, KC));
+  // as deep a ring as two CTAs per SM have room for (one stage is at most 99 KB)
+  if (4 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, WIDE, 4>(p, 4 * stage, stream);
+  if (3 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, WIDE, 3>(p, 3 * stage, stream);
+  if (2 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, WIDE, 2>(p, 2 * stage, stream);
+  return launch_gemv<HI, SWIGLU, NORM, WIDE, 1>(p, stage, stream);
 }
 
 template <bool HI, bool SWIGLU, bool NORM>
 static int dispatch_gemv(const GemvParams& p, cudaStream_t stream) {
-  constexpr int KC = gv_xs(HI, NORM) * 32 * GV_WARPS;
-  const int stage = (SWIGLU ? 16 : 8) * gv_pitch(std::min(p.K, KC));
-  // as deep a ring as two CTAs per SM have room for (one stage is at most 99 KB)
-  if (4 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, 4>(p, 4 * stage, stream);
-  if (2 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, 2>(p, 2 * stage, stream);
-  return launch_gemv<HI, SWIGLU, NORM, 1>(p, stage, stream);
+  // many turns per CTA (an output vocabulary): twice the columns per turn halve the barriers (151936 x 1024: 78 -> 50 us, 6.2 TB/s)
+  if constexpr (!SWIGLU) {
+    if (p.N >= 4 * 8 * gv_slots(HI) && p.K <= 2048) return stages_gemv<HI, SWIGLU, NORM, true>(p, stream);
+  }
+  return stages_gemv<HI, SWIGLU, NORM, false>(p, stream);
 }
 
 }  // namespace ttcd

@@ -40,6 +40,10 @@ def test_decode_attention_against_float64(B, Tq, Tk, H, HK, D, W, filled):
         k[:, n:], v[:, n:] = float("nan"), float("nan")
     kv_len = None if filled is None else torch.tensor([n], dtype=torch.int32, device=DEV)
     got = cuda.attn_small_q(q, k, v, W, None, kv_len).double()
+    turns = torch.zeros(B * HK, dtype=torch.int32, device=DEV)          # the splits merged in the same launch, twice
+    for _ in range(2):
+        one = cuda.attn_small_q(q, k, v, W, None, kv_len, turns).double()
+        assert (turns == 0).all() and (one - got).abs().max() <= 2.0 ** -8 * got.abs().max()
     want = _attention64(q, k, v, W, n)
     # fp32 sums (scores up to ~40: absolute error below 1e-5, so is the probabilities' relative one) and one rounding to bf16
     bound = want.abs() * 2.0 ** -8 + 1e-4

@@ -58,7 +58,7 @@ def graph_decoding_supported(model, input_ids, attention_mask, do_sample: bool) 
 
 
 def _fused_block_weights(block, batch: int):
-    """The weights of a block whose decode step runs as seven launches (``_fused_block_step``), or None where the step has
+    """The weights of a block whose decode step runs as six launches (``_fused_block_step``), or None where the step has
     to go through the modules: another kind of block, an option the step has no kernel for, a hook on a module."""
     from .layers import RMSNorm
     from .modeling_ipttcdv9 import IPTTCDBlock
@@ -89,7 +89,7 @@ def _fused_block_weights(block, batch: int):
     return qkv, gate_up
 
 
-def _fused_block_step(block, weights, x: torch.Tensor, cache: StaticWindowCache) -> torch.Tensor:
+def _fused_block_step(block, weights, x: torch.Tensor, cache: StaticWindowCache, turns: torch.Tensor) -> torch.Tensor:
     """One token per sample through a decoder block: x [B, hidden] -> x.  The norms ride in front of the projections that
     read them, SwiGLU and the residual sums behind the ones that produce them, k and v go straight into the rings; the
     roundings are those of the module by module step."""
@@ -105,7 +105,7 @@ def _fused_block_step(block, weights, x: torch.Tensor, cache: StaticWindowCache)
     qw, kw, eps = (attn.q_norm.weight, attn.k_norm.weight, attn.q_norm.eps) if attn.qk_norm else (None, None, 0.0)
     qkv = cuda.gemv(x, qkv_w, norm=(block.attn_norm.weight, block.attn_norm.eps), early_w=True)
     q = cuda.decode_qkv(qkv, rk, rv, cache.slot[c], cache.positions, qw, kw, eps, cos, sin, attn.num_heads)
-    o = ops.decode_attention(q, rk, rv, cache.kv_len[c])
+    o = ops.decode_attention(q, rk, rv, cache.kv_len[c], turns=turns)
     x = cuda.gemv(o.view(x.shape[0], -1), attn.o_proj.weight, residual=x, early_w=True)
     z = cuda.gemv(x, gate_up_w, norm=(block.mlp_norm.weight, block.mlp_norm.eps), swiglu=True, early_w=True)
     return cuda.gemv(z, mlp.down_proj.weight, residual=x, early_w=True)
@@ -130,6 +130,8 @@ class GraphDecoder:
         self.cursor = torch.zeros(1, dtype=torch.int64, device=dev)
         self.weights_at = self._weights_at()
         self.fused = self._fused_weights(batch)
+        heads = max(k.shape[2] for k, _ in self.cache.layers.values())
+        self.turns = torch.zeros(batch * heads, dtype=torch.int32, device=dev)      # this decoder's merge counters
         start = self.cache.start
         # warm-up on a side stream (allocator pools, rotary tables, lazily configured kernels), then rewind and capture
         side = torch.cuda.Stream(device=dev)
@@ -164,7 +166,7 @@ class GraphDecoder:
         core = self.model.model
         x = core.embeddings(self.token.view(-1))
         for layer, weights in zip(core.layers, self.fused):
-            x = _fused_block_step(layer, weights, x, self.cache)
+            x = _fused_block_step(layer, weights, x, self.cache, self.turns)
         return cuda.gemv(core.norm(x), self.model.lm_head.weight, early_w=True)
 
     @torch.no_grad()

@@ -131,12 +131,13 @@ def l2_softmax_attention(q, k, v, scale=None, cu_seqlens=None):
     return reference.l2_softmax_attention(q, k, v, scale, cu_seqlens)
 
 
-def decode_attention(q, k, v, kv_len, scale=None):
+def decode_attention(q, k, v, kv_len, scale=None, turns=None):
     """One decode step over a fixed-capacity cache: q [B,1,H,D] against the first ``kv_len`` rows (a one-element int32
     device tensor, read on the device) of k, v [B,cap,HK,D], in whatever order they sit (a ring buffer): no positional
-    mask, every filled row is visible.  Nothing here reads ``kv_len`` on the host, so the call can be captured."""
+    mask, every filled row is visible.  Nothing here reads ``kv_len`` on the host, so the call can be captured.  ``turns``:
+    see ``cuda.attn_small_q``."""
     if _native.use_native(q) and q.shape[1] == 1 and _cuda().attn_small_q_supported(q, k):
-        return _cuda().attn_small_q(q, k, v, None, scale, kv_len)
+        return _cuda().attn_small_q(q, k, v, None, scale, kv_len, turns)
     B, _, H, D = q.shape
     cap, HK = k.shape[1], k.shape[2]
     scale = D ** -0.5 if scale is None else scale

@@ -834,11 +834,12 @@ def attn_small_q_supported(q, k) -> bool:
             and k.shape[1] >= q.shape[1] and q.shape[2] % k.shape[2] == 0)
 
 
-def attn_small_q(q, k, v, window=None, scale=None, kv_len=None):
+def attn_small_q(q, k, v, window=None, scale=None, kv_len=None, turns=None):
     """Attention of a few query rows (a decode step or a short continuation) over a key/value cache: bottom-right
     aligned causal mask, optional window; forward only (split over the keys, merged by a second pass).  ``kv_len``
     (int32 device tensor of one element) says how many of the key rows are filled and is read by the kernel, so a
-    captured launch follows a cache that fills up between replays."""
+    captured launch follows a cache that fills up between replays.  ``turns`` (int32, zeros, one per sample and key/value
+    head; left zero; not shared by calls that may overlap): a decode step merges its splits in the same launch."""
     B, Tq, H, D = q.shape
     Tk, HK = k.shape[1], k.shape[2]
     scale = D ** -0.5 if scale is None else scale
@@ -853,7 +854,7 @@ def attn_small_q(q, k, v, window=None, scale=None, kv_len=None):
     nv.call("ttcd_attn_decode" if few else "ttcd_attn_small_q", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(out), nv.ptr(part_o),
             nv.ptr(part_ml), nv.i32(B), nv.i32(Tq), nv.i32(Tk), nv.i32(H), nv.i32(HK), nv.i32(D), nv.i64(ldq), nv.i64(ldk),
             nv.i64(ldv), nv.i64(sq), nv.i64(sk), nv.i64(sv), nv.i32(window or 0), nv.f32(scale), nv.i32(splits),
-            nv.ptr(kv_len), nv.stream_ptr())
+            *([nv.ptr(turns)] if few else []), nv.ptr(kv_len), nv.stream_ptr())
     return out
 
 
