@@ -10,8 +10,7 @@
 
 namespace ttcd {
 
-__device__ __forceinline__ void load8(const bf16* p, float (&f)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void unpack8(const uint4& raw, float (&f)[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -20,6 +19,7 @@ __device__ __forceinline__ void load8(const bf16* p, float (&f)[8]) {
     f[2 * i + 1] = t.y;
   }
 }
+__device__ __forceinline__ void load8(const bf16* p, float (&f)[8]) { unpack8(*reinterpret_cast<const uint4*>(p), f); }
 __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
   uint4 raw;
   raw.x = pack_bf16(f[0], f[1]);
@@ -29,23 +29,36 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
+// A thread keeps its 8 columns and takes SW_ROWS rows, whose loads are all in flight before the first is used; nothing is
+// divided.  65536 x 3072: 248 -> 211 us (188 us of bytes at the copy rate).  (The backward, with five streams, gained
+// nothing from it: 320 and 311, but 103 and 105 us at 7035 x 8192.)
+constexpr int SW_THREADS = 128, SW_ROWS = 4;
+
 // z = gate * sigmoid(gate) * up;  gate/up rows may be strided views of one packed buffer.
-__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const bf16* __restrict__ gate, const bf16* __restrict__ up,
-                                                         bf16* __restrict__ z, int64_t rows, int d, int64_t ldg,
-                                                         int64_t ldu, int64_t ldz) {
-  const int vec_per_row = d / 8;
-  const int64_t total = rows * vec_per_row;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / vec_per_row;
-    const int c = static_cast<int>(i % vec_per_row) * 8;
-    float g[8], u[8], o[8];
-    load8(gate + r * ldg + c, g);
-    load8(up + r * ldu + c, u);
+__global__ void __launch_bounds__(SW_THREADS) swiglu_fwd_kernel(const bf16* __restrict__ gate, const bf16* __restrict__ up,
+                                                                bf16* __restrict__ z, int64_t rows, int d, int64_t ldg,
+                                                                int64_t ldu, int64_t ldz) {
+  const int c = (blockIdx.y * SW_THREADS + threadIdx.x) * 8;
+  if (c >= d) return;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * SW_ROWS;
+  const int n = static_cast<int>(min(static_cast<int64_t>(SW_ROWS), rows - row0));
+  uint4 graw[SW_ROWS], uraw[SW_ROWS];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = g[k] / (1.f + __expf(-g[k])) * u[k];
-    store8(z + r * ldz + c, o);
-  }
+  for (int k = 0; k < SW_ROWS; ++k)
+    if (k < n) {
+      graw[k] = *reinterpret_cast<const uint4*>(gate + (row0 + k) * ldg + c);
+      uraw[k] = *reinterpret_cast<const uint4*>(up + (row0 + k) * ldu + c);
+    }
+#pragma unroll
+  for (int k = 0; k < SW_ROWS; ++k)
+    if (k < n) {
+      float g[8], u[8], o[8];
+      unpack8(graw[k], g);
+      unpack8(uraw[k], u);
+#pragma unroll
+      for (int x = 0; x < 8; ++x) o[x] = g[x] / (1.f + __expf(-g[x])) * u[x];
+      store8(z + (row0 + k) * ldz + c, o);
+    }
 }
 
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const bf16* __restrict__ dz, const bf16* __restrict__ gate,
@@ -232,9 +245,10 @@ using namespace ttcd;
 TTCD_EXPORT int ttcd_swiglu_fwd(const void* gate, const void* up, void* z, long long rows, int d, long long ldg,
                                 long long ldu, long long ldz, void* stream_ptr) {
   if (d % 8 != 0 || ldg % 8 != 0 || ldu % 8 != 0 || ldz % 8 != 0 || rows <= 0) return TTCD_ERR_ARG;
-  const long long total = rows * (d / 8);
-  const unsigned grid = static_cast<unsigned>(std::min<long long>((total + 255) / 256, 148LL * 32));
-  swiglu_fwd_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
+  const long long row_blocks = (rows + SW_ROWS - 1) / SW_ROWS;
+  if (row_blocks > 0x7fffffffLL || d > 65535 * SW_THREADS * 8) return TTCD_ERR_SIZE;
+  const dim3 grid(static_cast<unsigned>(row_blocks), (d / 8 + SW_THREADS - 1) / SW_THREADS);
+  swiglu_fwd_kernel<<<grid, SW_THREADS, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
       static_cast<const bf16*>(gate), static_cast<const bf16*>(up), static_cast<bf16*>(z), rows, d, ldg, ldu, ldz);
   return static_cast<int>(cudaGetLastError());
 }
