@@ -278,6 +278,78 @@ __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, const
   }
 }
 
+// Muon around the orthogonalisation, one launch per matrix on each side (a dozen element-wise launches before).
+// Before it: g = grad * coef; m = momentum m + g, kept unless skip; out = bf16(nesterov ? g + momentum m : m).
+// After it: p = p decay - rate u, kept unless skip; p_bf16 (may be null) = the weights after the step.
+// The roundings are those of the separate operations (product and sum on their own, scaled addition fused).
+struct MuonPreParams {
+  const float* grad; float* mom; bf16* out; const float* coef; const int* skip;
+  int64_t n; float momentum; int nesterov;
+};
+struct MuonPostParams {
+  const bf16* u; float* p; bf16* p_bf16; const int* skip;
+  int64_t n; float decay, rate;
+};
+template <int V>
+__global__ void __launch_bounds__(256) muon_pre_kernel(const MuonPreParams a) {
+  const float c = a.coef != nullptr ? *a.coef : 1.f;
+  const bool keep = a.skip == nullptr || *a.skip == 0;
+  for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * V; i < a.n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x * V) {
+    float g[V], m[V];
+    if constexpr (V == 4) {
+      const float4 gv = *reinterpret_cast<const float4*>(a.grad + i), mv = *reinterpret_cast<const float4*>(a.mom + i);
+      g[0] = gv.x; g[1] = gv.y; g[2] = gv.z; g[3] = gv.w;
+      m[0] = mv.x; m[1] = mv.y; m[2] = mv.z; m[3] = mv.w;
+    } else {
+      g[0] = a.grad[i];
+      m[0] = a.mom[i];
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      if (a.coef != nullptr) g[k] = __fmul_rn(g[k], c);
+      m[k] = __fadd_rn(__fmul_rn(m[k], a.momentum), g[k]);
+      g[k] = a.nesterov ? fmaf(a.momentum, m[k], g[k]) : m[k];
+    }
+    if constexpr (V == 4) {
+      if (keep) *reinterpret_cast<float4*>(a.mom + i) = make_float4(m[0], m[1], m[2], m[3]);
+      *reinterpret_cast<uint2*>(a.out + i) = make_uint2(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]));
+    } else {
+      if (keep) a.mom[i] = m[0];
+      a.out[i] = __float2bfloat16(g[0]);
+    }
+  }
+}
+template <int V>
+__global__ void __launch_bounds__(256) muon_post_kernel(const MuonPostParams a) {
+  const bool keep = a.skip == nullptr || *a.skip == 0;
+  for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * V; i < a.n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x * V) {
+    float u[V], p[V];
+    if constexpr (V == 4) {
+      const uint2 uv = *reinterpret_cast<const uint2*>(a.u + i);
+      const float2 lo = unpack_bf16(uv.x), hi = unpack_bf16(uv.y);
+      const float4 pv = *reinterpret_cast<const float4*>(a.p + i);
+      u[0] = lo.x; u[1] = lo.y; u[2] = hi.x; u[3] = hi.y;
+      p[0] = pv.x; p[1] = pv.y; p[2] = pv.z; p[3] = pv.w;
+    } else {
+      u[0] = __bfloat162float(a.u[i]);
+      p[0] = a.p[i];
+    }
+    if (keep) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) p[k] = fmaf(-a.rate, u[k], __fmul_rn(p[k], a.decay));
+    }
+    if constexpr (V == 4) {
+      if (keep) *reinterpret_cast<float4*>(a.p + i) = make_float4(p[0], p[1], p[2], p[3]);
+      if (a.p_bf16 != nullptr) *reinterpret_cast<uint2*>(a.p_bf16 + i) = make_uint2(pack_bf16(p[0], p[1]), pack_bf16(p[2], p[3]));
+    } else {
+      if (keep) a.p[i] = p[0];
+      if (a.p_bf16 != nullptr) a.p_bf16[i] = __float2bfloat16(p[0]);
+    }
+  }
+}
+
 // out[0] += sum(x^2) (atomicAdd of per-block partials; zero `out` beforehand).
 template <typename T>
 __global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, int64_t n, float* __restrict__ out) {
@@ -384,6 +456,32 @@ TTCD_EXPORT int ttcd_adamw(float* p, const void* g, int grad_is_bf16, float* m, 
     if (vec) go(adamw_kernel<float, true>, gf);
     else go(adamw_kernel<float, false>, gf);
   }
+  return static_cast<int>(cudaGetLastError());
+}
+
+// grad, mom fp32 [n], out bf16 [n]; coef, skip: device words or null.
+TTCD_EXPORT int ttcd_muon_pre(const float* grad, float* mom, void* out, const float* coef, const int* skip, long long n,
+                              float momentum, int nesterov, void* stream_ptr) {
+  if (n <= 0) return TTCD_OK;
+  const MuonPreParams a{grad, mom, static_cast<bf16*>(out), coef, skip, n, momentum, nesterov};
+  const bool vec = n % 4 == 0 && ((reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(mom)) & 15u) == 0 &&
+                   (reinterpret_cast<uintptr_t>(out) & 7u) == 0;
+  cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
+  if (vec) muon_pre_kernel<4><<<flat_grid(n / 4), 256, 0, st>>>(a);
+  else muon_pre_kernel<1><<<flat_grid(n), 256, 0, st>>>(a);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// u bf16 [n], p fp32 [n], p_bf16 bf16 [n] or null; skip: a device word or null.
+TTCD_EXPORT int ttcd_muon_post(const void* u, float* p, void* p_bf16, const int* skip, long long n, float decay, float rate,
+                               void* stream_ptr) {
+  if (n <= 0) return TTCD_OK;
+  const MuonPostParams a{static_cast<const bf16*>(u), p, static_cast<bf16*>(p_bf16), skip, n, decay, rate};
+  const bool vec = n % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(p_bf16)) & 7u) == 0;
+  cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
+  if (vec) muon_post_kernel<4><<<flat_grid(n / 4), 256, 0, st>>>(a);
+  else muon_post_kernel<1><<<flat_grid(n), 256, 0, st>>>(a);
   return static_cast<int>(cudaGetLastError());
 }
 

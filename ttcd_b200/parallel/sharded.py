@@ -715,14 +715,21 @@ class ShardedDataParallel:
         for mp in owned:
             saved[id(mp)] = mp.grad32
             mp.grad32 = mp.grad32[:mp.param.numel()]
-        muon_update_many(owned, lr, self.weight_decay, self.muon_momentum, coef,
-                         skip=self._skip if (self.skip_nan_inf or self.peer) else None, tp=self.tensor_parallel)
+        def place(mp):                      # the parameter's place in the flat weights
+            return self.groups[mp.group_index].flat_param[mp.offset:mp.offset + mp.param.numel()]
+
+        here = self.world == 1 and not self.peer and self.param_dtype == torch.bfloat16
+        published = muon_update_many(owned, lr, self.weight_decay, self.muon_momentum, coef,
+                                     skip=self._skip if (self.skip_nan_inf or self.peer) else None, tp=self.tensor_parallel,
+                                     publish=place if here else None)
         for mp in owned:
             mp.grad32 = saved[id(mp)]
         for mp in self.muon_params:
+            if id(mp) in published:
+                continue
             g = self.groups[mp.group_index]
             n = mp.param.numel()
-            dst = g.flat_param[mp.offset:mp.offset + n]
+            dst = place(mp)
             if mp.owner == self.rank:
                 if self.peer:
                     n8 = n // 8 * 8

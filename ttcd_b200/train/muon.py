@@ -77,8 +77,34 @@ def muon_update(mp: MuonParam, lr: float, weight_decay: float, momentum: float, 
     return mp.master
 
 
+def _fused_ok(mp: MuonParam, coef, skip, tp) -> bool:
+    """The element-wise work around the orthogonalisation runs as one kernel on each side of it."""
+    tensors = [t for t in (mp.grad32, mp.momentum, mp.master) if t is not None]
+    return ((tp is None or tp.world == 1) and mp.param.dim() == 2 and min(mp.param.shape) >= 64 and _native.available()
+            and all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == mp.param.numel() for t in tensors)
+            and len(tensors) == 3 and (coef is None or (coef.dtype == torch.float32 and coef.numel() == 1))
+            and (skip is None or (skip.dtype == torch.int32 and skip.numel() == 1)))
+
+
+def _update_fused(params: list[MuonParam], lr: float, weight_decay: float, momentum: float, coef, nesterov: bool, skip,
+                  publish) -> None:
+    """``muon_update_many`` for the parameters of one shape (see ``_fused_ok``)."""
+    from .._native import call, f32, i32, i64, ptr, stream_ptr
+    shape, n = params[0].param.shape, params[0].param.numel()
+    g = torch.empty(len(params), *shape, dtype=torch.bfloat16, device=params[0].master.device)
+    for j, mp in enumerate(params):
+        call("ttcd_muon_pre", ptr(mp.grad32), ptr(mp.momentum), ptr(g[j]), ptr(coef), ptr(skip), i64(n), f32(momentum),
+             i32(int(nesterov)), stream_ptr())
+    u = ops.newton_schulz(g).contiguous()
+    adj_lr = lr * 0.2 * math.sqrt(max(shape))
+    for j, mp in enumerate(params):
+        call("ttcd_muon_post", ptr(u[j]), ptr(mp.master), ptr(None if publish is None else publish(mp)), ptr(skip), i64(n),
+             f32(1.0 - lr * weight_decay), f32(adj_lr), stream_ptr())
+
+
 def muon_update_many(params: list[MuonParam], lr: float, weight_decay: float, momentum: float,
-                     coef: torch.Tensor | None, nesterov: bool = True, skip: torch.Tensor | None = None, tp=None) -> None:
+                     coef: torch.Tensor | None, nesterov: bool = True, skip: torch.Tensor | None = None, tp=None,
+                     publish=None) -> set[int]:
     """Owner-side update of several parameters.  Parameters of one shape are orthogonalised as ONE batched
     Newton-Schulz call (15 GEMM launches for the whole group instead of 15 per matrix: the matrices of a 1024-wide
     model are a handful of tiles each, so per-matrix launches are pure latency); the reference batches the same way
@@ -88,9 +114,23 @@ def muon_update_many(params: list[MuonParam], lr: float, weight_decay: float, mo
     along ``mp.tp_dim``.  Momentum is element-wise and stays on the slice; for the orthogonalisation the slices of
     the group's ranks are gathered into the whole matrix (every rank of the group then runs the same Newton-Schulz
     and keeps its slice of the result), and the update's scale uses the whole matrix's dimensions.  All ranks of a
-    tensor-parallel group hold the same parameters in the same order, so they issue the same gathers."""
+    tensor-parallel group hold the same parameters in the same order, so they issue the same gathers.
+
+    ``publish(mp)`` (optional): where a parameter's new bf16 weights go.  Returns the ids of the parameters whose weights
+    were written there; the caller copies the rest from ``master``."""
+    published: set[int] = set()
+    fused: dict[tuple, list[MuonParam]] = {}
+    for mp in params:
+        if _fused_ok(mp, coef, skip, tp):
+            fused.setdefault(tuple(mp.param.shape), []).append(mp)
+    for group in fused.values():
+        _update_fused(group, lr, weight_decay, momentum, coef, nesterov, skip, publish)
+        if publish is not None:
+            published.update(id(mp) for mp in group)
+    done = {id(mp) for group in fused.values() for mp in group}
+    params = [mp for mp in params if id(mp) not in done]
     if not params:
-        return
+        return published
     pre = []                          # (param, momentum after this step, Nesterov-combined gradient)
     for mp in params:
         g = mp.grad32 if coef is None else mp.grad32 * coef
@@ -144,3 +184,4 @@ def muon_update_many(params: list[MuonParam], lr: float, weight_decay: float, mo
             new_master = torch.where(keep, new_master, mp.master)
         mp.momentum.copy_(new_mom)
         mp.master.copy_(new_master)
+    return published
