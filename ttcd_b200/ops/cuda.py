@@ -30,10 +30,16 @@ class _Forward:
         pass
 
 
+def _watched() -> bool:
+    """Whether a function transform (vmap, forward-mode derivatives, torch.func) or a tracer looks at the calls."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or _forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None)
+
+
 def _apply(fn, *args):
-    """``fn.apply(*args)``; with gradients off and no function transform (vmap, forward-mode derivatives, torch.func) at
-    work just its forward: the autograd machinery around a call costs the host more than the launch inside it."""
-    if torch.is_grad_enabled() or torch._C._functorch.peek_interpreter_stack() is not None or _forward_ad._current_level >= 0:
+    """``fn.apply(*args)``; with gradients off and nobody watching just its forward: the autograd machinery around a call
+    costs the host more than the launch inside it."""
+    if torch.is_grad_enabled() or _watched():
         return fn.apply(*args)
     return fn.forward(_Forward(), *args)
 
