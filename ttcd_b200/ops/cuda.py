@@ -421,7 +421,9 @@ class _RMSNorm(torch.autograd.Function):
 
 def rmsnorm(x, weight, eps, residual=None, prenorm=False):
     _check(x, "x")
-    return _apply(_RMSNorm, x, residual, weight, float(eps), bool(prenorm))
+    out = _apply(_RMSNorm, x, residual, weight, float(eps), bool(prenorm))
+    # without a residual the sum is x itself: handed through as apply does it, a tensor of its own that needs no gradient
+    return (out[0], x.detach()) if prenorm and out[1] is x else out
 
 
 class _RMSNormDual(torch.autograd.Function):
