@@ -63,3 +63,24 @@ def test_cross_entropy_gradient_beside_the_logits(rows, vocab, offset, smoothing
     # one rounding to bf16 of values whose exponentials carry a few fp32 roundings; scaled by 3: one more
     assert ((grads[0] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
     assert ((grads[1] - 3 * want).abs() <= 2.0 ** -7 * 3 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("linear", [False, True])
+def test_loss_gradient_is_linear_in_what_arrives(linear):
+    """A learned weight of the loss (``create_graph``) and several weights at once (``is_grads_batched``)."""
+    torch.manual_seed(1)
+    x = torch.randn(128, 64 if linear else 512, device=DEV).bfloat16().requires_grad_()
+    w = torch.randn(512, 64, device=DEV).bfloat16()
+    labels = torch.randint(0, 512, (128,), device=DEV)
+    loss = lambda: cuda.linear_cross_entropy(x, labels, w) if linear else cuda.cross_entropy(x, labels)     # noqa: E731
+    (one,) = torch.autograd.grad(loss(), x)
+    weight = torch.tensor(2.0, device=DEV, requires_grad=True)
+    (twice,) = torch.autograd.grad(loss() * weight, x, create_graph=True)
+    assert torch.equal(twice, 2 * one)                       # doubling rounds nothing
+    (by_weight,) = torch.autograd.grad(twice.float().sum(), weight)
+    want = one.double().sum()
+    # d(sum of the gradient) / d weight = the sum, of bf16 values that the library adds in fp32 and rounds to bf16
+    assert abs(float(by_weight.double() - want)) <= 2.0 ** -8 * float(want.abs()) + 2.0 ** -20 * float(one.double().abs().sum())
+    (several,) = torch.autograd.grad(loss(), x, torch.tensor([1.0, 4.0], device=DEV), is_grads_batched=True)
+    assert torch.equal(several[0], one) and torch.equal(several[1], 4 * one)

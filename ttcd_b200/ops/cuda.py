@@ -912,8 +912,10 @@ def _logits_with_lse(hidden2, w, out):
 
 
 def _scale_by(t: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
-    """t * g for a gradient held since the forward and the scalar that arrives from downstream (on the device)."""
-    if t.dtype != _BF16 or not t.is_contiguous() or t.numel() % 8 or t.data_ptr() % 16:
+    """t * g for a gradient held since the forward and the scalar that arrives from downstream (on the device).  Where g is
+    differentiated in turn (``create_graph``) or stands for several (``is_grads_batched``), the library multiplies."""
+    if ((torch.is_grad_enabled() and g.requires_grad) or torch._C._functorch.is_legacy_batchedtensor(g) or _watched()
+            or t.dtype != _BF16 or not t.is_contiguous() or t.numel() % 8 or t.data_ptr() % 16):
         return t * g.to(t.dtype)
     out = torch.empty_like(t)
     nv.call("ttcd_scale_by", nv.ptr(t), nv.ptr(out), nv.ptr(g.float().contiguous()), nv.i64(t.numel()), nv.stream_ptr())
