@@ -1,0 +1,111 @@
+"""Which models a decode step may bypass the modules of: the stock ones, and none of whose parts a program has replaced."""
+from types import MethodType, SimpleNamespace
+
+import pytest
+import torch
+import torch.nn as nn
+
+from ttcd_b200 import ops
+from ttcd_b200.models import IPTTCDv9Config, IPTTCDv9ForCausalLM, layers
+from ttcd_b200.models.decoding import GraphDecoder, pack_projection_weights
+from ttcd_b200.models.layers import GatedMLP
+
+
+class _ReluMLP(GatedMLP):
+    def features(self, x):
+        return torch.relu(ops.linear(x, self.gate_proj.weight)) * ops.linear(x, self.up_proj.weight)
+
+
+class _ScaledLogits(IPTTCDv9ForCausalLM):
+    def forward(self, *args, **kwargs):
+        out = super().forward(*args, **kwargs)
+        out.logits = 0.5 * out.logits
+        return out
+
+
+class _HalfEmbedding(nn.Embedding):
+    def forward(self, ids):
+        return 0.5 * super().forward(ids)
+
+
+class _Doubled(nn.Module):
+    def forward(self, w):
+        return 2 * w
+
+
+def _model(cls=IPTTCDv9ForCausalLM):
+    torch.manual_seed(0)
+    model = cls(IPTTCDv9Config(hidden_size=128, num_hidden_layers=2, num_heads=2, num_kv_heads=1, head_dim=64, intermediate_size=256,
+                               vocab_size=64, window_size=32, ttt_mode=True, ttt_chunk=8, ttt_layers=[1], qk_norm=True,
+                               tie_word_embeddings=False)).to(torch.bfloat16).eval()
+    pack_projection_weights(model)
+    return model
+
+
+def _fused(model):
+    return GraphDecoder._fused_weights(SimpleNamespace(model=model), 2)
+
+
+def _replace_mlp(model):
+    old = model.model.layers[1].mlp
+    new = _ReluMLP(128, 256).to(torch.bfloat16).eval()
+    for name in ("gate_proj", "up_proj", "down_proj"):
+        setattr(new, name, getattr(old, name))
+    model.model.layers[1].mlp = new
+
+
+def _replace_embedding(model):
+    model.model.embeddings = _HalfEmbedding.from_pretrained(model.model.embeddings.weight.data)
+
+
+def _replace_method(path, name):
+    def change(model):
+        module = model.get_submodule(path)
+        original = getattr(module, name)
+        setattr(module, name, MethodType(lambda self, *a, **k: original(*a, **k), module))
+    return change
+
+
+CHANGES = {
+    "mlp_of_another_kind": _replace_mlp,
+    "embedding_of_another_kind": _replace_embedding,
+    "mlp_forward_replaced": _replace_method("model.layers.0.mlp", "forward"),
+    "mlp_features_replaced": _replace_method("model.layers.0.mlp", "features"),
+    "attention_finish_replaced": _replace_method("model.layers.1.attn", "finish"),
+    "norm_forward_replaced": _replace_method("model.layers.1.mlp_norm", "forward"),
+    "model_forward_replaced": _replace_method("model", "forward"),
+    "hook_on_a_block": lambda model: model.model.layers[0].register_forward_hook(lambda *a: None),
+    # the weight would be read while the launch that makes it still runs
+    "computed_weight": lambda model: nn.utils.parametrize.register_parametrization(model.model.layers[0].attn.o_proj, "weight", _Doubled()),
+}
+
+
+def test_the_stock_model_is_fused():
+    assert len(_fused(_model())) == 2
+
+
+@pytest.mark.parametrize("change", list(CHANGES))
+def test_a_changed_model_runs_its_modules(change):
+    model = _model()
+    CHANGES[change](model)
+    assert _fused(model) is None
+
+
+def test_a_model_with_its_own_forward_runs_it():
+    assert _fused(_model(_ScaledLogits)) is None
+
+
+def test_hooks_on_all_modules_are_run():
+    model = _model()
+    handle = nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert _fused(model) is None
+    finally:
+        handle.remove()
+    assert _fused(model) is not None
+
+
+def test_a_tensor_parallel_state_runs_the_modules(monkeypatch):
+    model = _model()
+    monkeypatch.setattr(layers, "_tp_state", lambda: SimpleNamespace(world=2))
+    assert _fused(model) is None

@@ -57,30 +57,47 @@ def graph_decoding_supported(model, input_ids, attention_mask, do_sample: bool) 
     return _native.available() and next(model.parameters()).dtype == torch.bfloat16
 
 
+# what the fused step computes on behalf of the modules; a program may replace any of these on an instance
+_STEP_METHODS = ("forward", "project_qkv", "finish", "features", "_block_kwargs")
+
+
+def _as_defined(*modules) -> bool:
+    """No hook and no method replaced on an instance: calling these modules does what their classes say."""
+    from torch.nn.modules import module as hooks
+    if hooks._global_forward_hooks or hooks._global_forward_pre_hooks:
+        return False
+    return not any(m._forward_hooks or m._forward_pre_hooks or any(name in vars(m) for name in _STEP_METHODS) for m in modules)
+
+
+def _at_rest(linear) -> bool:
+    """The weight is the module's own parameter and not made from others in every step (a parametrization)."""
+    return linear._parameters.get("weight") is not None and linear.bias is None
+
+
 def _fused_block_weights(block, batch: int):
     """The weights of a block whose decode step runs as six launches (``_fused_block_step``), or None where the step has
-    to go through the modules: another kind of block, an option the step has no kernel for, a hook on a module."""
-    from .layers import RMSNorm
-    from .modeling_ipttcdv9 import IPTTCDBlock
+    to go through the modules: another kind of block or of a part of it, an option the step has no kernel for, a hook, a
+    replaced method, a weight that is computed."""
+    from .layers import RMSNorm, _tp_state
+    from .modeling_ipttcdv9 import IPTTCDBlock, IPTTCDMLP
     from .modeling_transformer import TransformerBlock
-    if type(block) not in (IPTTCDBlock, TransformerBlock) or block.training or batch > 16:
+    if type(block) not in (IPTTCDBlock, TransformerBlock) or block.training or batch > 16 or _tp_state() is not None:
         return None
     if type(block) is IPTTCDBlock and block.is_ttt_layer and block.ttt_chunk <= 1:       # one token would be a whole chunk
         return None
-    if any(m._forward_hooks or m._forward_pre_hooks for m in block.modules()):
+    if not _as_defined(*block.modules()) or type(block.mlp) not in (GatedMLP, IPTTCDMLP):
         return None
     attn, mlp = block.attn, block.mlp
     if type(attn) is not Attention or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128):
         return None
-    if any(type(n) is not RMSNorm or n.weight is None for n in (block.attn_norm, block.mlp_norm)):
+    norms = [block.attn_norm, block.mlp_norm] + ([attn.q_norm, attn.k_norm] if attn.qk_norm else [])
+    if any(type(n) is not RMSNorm or n.weight is None for n in norms):
         return None
-    if any(m.bias is not None for m in (attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.gate_proj, mlp.up_proj, mlp.down_proj)):
+    if not all(_at_rest(m) for m in (attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.gate_proj, mlp.up_proj, mlp.down_proj)):
         return None
     qkv = _slab_view([attn.q_proj.weight, attn.k_proj.weight, attn.v_proj.weight])
     gate_up = _slab_view([mlp.gate_proj.weight, mlp.up_proj.weight])
-    ws = [qkv, gate_up, attn.o_proj.weight, mlp.down_proj.weight, block.attn_norm.weight, block.mlp_norm.weight]
-    if attn.qk_norm:
-        ws += [attn.q_norm.weight, attn.k_norm.weight]
+    ws = [qkv, gate_up, attn.o_proj.weight, mlp.down_proj.weight, *(n.weight for n in norms)]
     hidden = attn.hidden_size
     if hidden % 8 or hidden > 2048 or mlp.intermediate_size % 8:
         return None
@@ -151,12 +168,17 @@ class GraphDecoder:
 
     def _fused_weights(self, batch: int):
         """Per block the weights of its fused step; None if any part of the model has to run module by module."""
-        model, head = self.model, self.model.lm_head
-        if any(m._forward_hooks or m._forward_pre_hooks for m in (model, model.model, model.model.norm, model.model.embeddings, head)):
+        from .base import DecoderForCausalLM, DecoderModel
+        model, core, head = self.model, self.model.model, self.model.lm_head
+        if type(model).forward is not DecoderForCausalLM.forward or type(core).forward is not DecoderModel.forward:
             return None
-        if head.bias is not None or head.weight.dtype != torch.bfloat16 or not head.weight.is_contiguous() or head.weight.data_ptr() % 16:
+        if type(core)._block_kwargs is not DecoderModel._block_kwargs or type(core.embeddings) is not torch.nn.Embedding:
             return None
-        got = [_fused_block_weights(layer, batch) for layer in model.model.layers]
+        if not _as_defined(model, core, core.norm, core.embeddings, head) or not _at_rest(head):
+            return None
+        if head.weight.dtype != torch.bfloat16 or not head.weight.is_contiguous() or head.weight.data_ptr() % 16:
+            return None
+        got = [_fused_block_weights(layer, batch) for layer in core.layers]
         return None if any(w is None for w in got) else got
 
     def _logits(self) -> torch.Tensor:
