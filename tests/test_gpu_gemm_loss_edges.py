@@ -36,7 +36,14 @@ def test_fp32_output_and_accumulation(M, N, K, batch, a_t, b_t):
 def test_lm_head_chunks_cover_the_rows_and_stay_bounded(n, hidden, chunks):
     rows = cuda._lce_chunk_rows(n, hidden, chunks)
     assert rows % 128 == 0 and rows > 0
-    assert rows <= max(-(-n // 128) * 128 if chunks == 1 or n <= 2560 else 0, 2560, int(1.25 * n / chunks) + 128)
+    assert rows <= max(-(-n // 128) * 128 if chunks == 1 else 0, 2560 if chunks <= 8 else 0, int(1.25 * n / chunks) + 128)
+
+
+@pytest.mark.parametrize("n,hidden", [(5003, 2048), (8192, 2048), (16384, 2048), (40000, 1024), (65536, 960)])
+def test_more_chunks_than_the_default_take_less_memory(n, hidden):
+    rows = [cuda._lce_chunk_rows(n, hidden, chunks) for chunks in (9, 16, 32, 64)]
+    assert all(r <= 1.25 * n / c + 128 for r, c in zip(rows, (9, 16, 32, 64)))
+    assert rows == sorted(rows, reverse=True) and rows[-1] < cuda._lce_chunk_rows(n, hidden, 8)
 
 
 @pytest.mark.gpu

@@ -951,16 +951,20 @@ def cross_entropy(logits, labels, ignore_index=-100, label_smoothing=0.0, z_loss
     return _apply(_CrossEntropy, logits, labels, int(ignore_index), float(label_smoothing), float(z_loss))
 
 
+_LCE_CHUNKS = 8        # the default of ``num_chunks``
+
+
 def _lce_chunk_rows(n_rows: int, hidden: int, num_chunks: int, sms: int = 148) -> int:
-    """Rows per chunk of the chunked lm_head pass: about ``n_rows / num_chunks`` (a quarter either way), but up to 2560
-    where that is less, whichever the two gradient GEMMs finish soonest with.  Their cost per vocabulary entry, at the
-    measured GEMM and copy rates: dx ([rows, vocab] x [vocab, hidden]) has only rows/128 x hidden/256 output tiles, so it
-    costs whole waves of the persistent kernel's CTAs; dW runs rows x hidden products but at least the time in which its
-    fp32 accumulator is read and written once.  (5003 rows, hidden 2048, vocabulary 128256: eight chunks of 640 rows leave
-    108 of 148 SMs idle in every dx and pass over the 1 GB accumulator eight times; three chunks of at most 2304 do not.)"""
+    """Rows per chunk of the chunked lm_head pass: about ``n_rows / num_chunks`` (a quarter either way), whichever the two
+    gradient GEMMs finish soonest with.  Their cost per vocabulary entry, at the measured GEMM and copy rates: dx ([rows,
+    vocab] x [vocab, hidden]) has only rows/128 x hidden/256 output tiles, so it costs whole waves of the persistent
+    kernel's CTAs; dW runs rows x hidden products but at least the time in which its fp32 accumulator is read and written
+    once.  Up to the default number of chunks, up to 2560 rows are taken where that is more: 5003 rows, hidden 2048,
+    vocabulary 128256 in eight chunks of 640 leave 108 of 148 SMs idle in every dx and pass over the 1 GB accumulator eight
+    times; in three of at most 1792 they do not.  Who asks for more chunks than the default wants less memory and gets it."""
     total = -(-n_rows // 128)
     target = max(1, -(-n_rows // max(1, num_chunks)) // 128)
-    hi = max(target + target // 4, 20)
+    hi = max(target + target // 4, 20 if num_chunks <= _LCE_CHUNKS else 0)
     if hi >= total and target >= total:
         return total * 128
     n_tiles = max(1, -(-hidden // 256))
@@ -976,7 +980,7 @@ def _lce_chunk_rows(n_rows: int, hidden: int, num_chunks: int, sms: int = 148) -
 
 class _LinearCrossEntropy(torch.autograd.Function):
     """CE(hidden @ W^T) in token chunks: logits GEMM -> row kernel (LSE + in-place dlogits) ->
-    dx and dW GEMMs, so the [tokens, vocab] logits never exist at once and there is no host sync."""
+    dx and dW GEMMs, so no more than one chunk's logits exist at once and there is no host sync."""
 
     @staticmethod
     def forward(ctx, hidden, labels, weight, ignore_index, num_chunks, l2_factor=0.0):
@@ -1025,7 +1029,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         return _scale_by(dx, g), None, _scale_by(dw, g), None, None, None
 
 
-def linear_cross_entropy(hidden, labels, weight, ignore_index=-100, num_chunks=8, l2_penalty=0.0):
+def linear_cross_entropy(hidden, labels, weight, ignore_index=-100, num_chunks=_LCE_CHUNKS, l2_penalty=0.0):
     _check(hidden, "hidden")
     if hidden.shape[0] < 128 or hidden.shape[1] < 64 or weight.shape[0] < 128:       # below one GEMM tile
         return reference.linear_cross_entropy(hidden, labels, weight, None, ignore_index, l2_penalty)
