@@ -50,6 +50,15 @@ def test_decode_attention_against_float64(B, Tq, Tk, H, HK, D, W, filled):
     assert ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())
 
 
+@pytest.mark.parametrize("Tq,H,HK,D", [(1, 4, 2, 128), (3, 2, 1, 64)])
+def test_decode_attention_takes_a_query_at_any_address(Tq, H, HK, D):
+    torch.manual_seed(Tq)
+    k, v = (torch.randn(1, 300, HK, D, device=DEV).bfloat16() for _ in range(2))
+    q = torch.randn(Tq * H * D + 1, device=DEV).bfloat16()[1:].view(1, Tq, H, D)           # contiguous, 2-byte aligned
+    got, want = cuda.attn_small_q(q, k, v).double(), _attention64(q, k, v, None, 300)
+    assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 128, 64), (1, 1024, 2048), (3, 129, 72), (8, 6144, 1024), (8, 1001, 3072), (9, 130, 264),
                                    (16, 4096, 1024), (16, 20000, 520), (5, 151936, 1024)])
 def test_few_rows_times_weight_against_float64(M, N, K):

@@ -854,7 +854,8 @@ def attn_small_q(q, k, v, window=None, scale=None, kv_len=None, turns=None):
     q, ldq, sq = _attn_layout(q)
     k, ldk, sk = _attn_layout(k)
     v, ldv, sv = _attn_layout(v)
-    few = Tq * (H // HK) <= 8               # a decode step: the register kernel, else 256 keys per CTA through shared memory
+    # a decode step: the register kernel (16-byte reads of q), else 256 keys per CTA through shared memory
+    few = Tq * (H // HK) <= 8 and q.data_ptr() % 16 == 0
     splits = _decode_splits(B * HK, Tk) if few else -(-Tk // 256)     # the partial results are merged by a second pass
     out = torch.empty(B, Tq, H, D, dtype=_BF16, device=q.device)
     part_o = torch.empty(B, H, Tq, splits, D, dtype=torch.float32, device=q.device)
