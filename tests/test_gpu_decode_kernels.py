@@ -4,6 +4,7 @@ with a weight (row, column and K remainders)."""
 import pytest
 import torch
 
+from ttcd_b200 import _native
 from ttcd_b200.models import IPTTCDv9Config, IPTTCDv9ForCausalLM
 from ttcd_b200.models.decoding import GraphDecoder
 from ttcd_b200.models.layers import WindowKVCache
@@ -57,6 +58,15 @@ def test_decode_attention_takes_a_query_at_any_address(Tq, H, HK, D):
     q = torch.randn(Tq * H * D + 1, device=DEV).bfloat16()[1:].view(1, Tq, H, D)           # contiguous, 2-byte aligned
     got, want = cuda.attn_small_q(q, k, v).double(), _attention64(q, k, v, None, 300)
     assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
+
+
+def test_decode_attention_counts_its_launches():
+    q, k = torch.randn(1, 1, 4, 64, device=DEV).bfloat16(), torch.randn(1, 300, 2, 64, device=DEV).bfloat16()
+    before = _native.launch_count
+    cuda.attn_small_q(q, k, k)
+    apart = _native.launch_count
+    cuda.attn_small_q(q, k, k, turns=torch.zeros(2, dtype=torch.int32, device=DEV))
+    assert (apart - before, _native.launch_count - apart) == (2, 1)          # with and without a merge of its own
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 64), (1, 1024, 2048), (3, 129, 72), (8, 6144, 1024), (8, 1001, 3072), (9, 130, 264),

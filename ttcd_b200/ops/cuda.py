@@ -864,6 +864,8 @@ def attn_small_q(q, k, v, window=None, scale=None, kv_len=None, turns=None):
             nv.ptr(part_ml), nv.i32(B), nv.i32(Tq), nv.i32(Tk), nv.i32(H), nv.i32(HK), nv.i32(D), nv.i64(ldq), nv.i64(ldk),
             nv.i64(ldv), nv.i64(sq), nv.i64(sk), nv.i64(sv), nv.i32(window or 0), nv.f32(scale), nv.i32(splits),
             *([nv.ptr(turns)] if few else []), nv.ptr(kv_len), nv.stream_ptr())
+    if few and turns is None:
+        nv.launch_count += 1                # the merge is a launch of its own
     return out
 
 
