@@ -77,8 +77,8 @@ def test_cross_entropy_gradient_beside_the_logits(rows, vocab, offset, smoothing
 def test_loss_gradient_is_linear_in_what_arrives(linear):
     """A learned weight of the loss (``create_graph``) and several weights at once (``is_grads_batched``)."""
     torch.manual_seed(1)
-    x = torch.randn(128, 64 if linear else 512, device=DEV).bfloat16().requires_grad_()
-    w = torch.randn(512, 64, device=DEV).bfloat16()
+    x = torch.randn(128, 128 if linear else 512, device=DEV).bfloat16().requires_grad_()
+    w = torch.randn(512, 128, device=DEV).bfloat16()
     labels = torch.randint(0, 512, (128,), device=DEV)
     loss = lambda: cuda.linear_cross_entropy(x, labels, w) if linear else cuda.cross_entropy(x, labels)     # noqa: E731
     (one,) = torch.autograd.grad(loss(), x)
