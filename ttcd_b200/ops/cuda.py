@@ -681,7 +681,8 @@ def segment_bounds(cu_seqlens: torch.Tensor, total: int):
     return cu[seg].to(torch.int32).contiguous(), cu[seg + 1].clamp(max=total).to(torch.int32).contiguous()
 
 
-def attn_forward(q, k, v, window_t, window_s, scale, dual, seg=None):
+def attn_forward(q, k, v, window_t, window_s, scale, dual, seg=None, form: int = 0):
+    """``form``: 0 lets the kernel's rule choose, 1 and 2 name its long and its short form (for tests)."""
     B, Tq, H, D = q.shape
     Tk, HK = k.shape[1], k.shape[2]
     if D not in (64, 128):
@@ -698,7 +699,7 @@ def attn_forward(q, k, v, window_t, window_s, scale, dual, seg=None):
     nv.call("ttcd_attn_fwd", nv.ptr(q), nv.ptr(k), nv.ptr(v), nv.ptr(o_t), nv.ptr(o_s), nv.ptr(lse_t), nv.ptr(lse_s),
             nv.i32(B), nv.i32(Tq), nv.i32(Tk), nv.i32(H), nv.i32(HK), nv.i32(D), nv.i64(ldq), nv.i64(ldk), nv.i64(ldv),
             nv.i64(sq), nv.i64(sk), nv.i64(sv), nv.i32(window_t or 0), nv.i32(window_s or 0), nv.f32(scale),
-            nv.ptr(None if seg is None else seg[0]), nv.stream_ptr())
+            nv.ptr(None if seg is None else seg[0]), nv.i32(form), nv.stream_ptr())
     return (q, k, v), o_t, o_s, lse_t, lse_s
 
 
