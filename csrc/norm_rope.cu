@@ -677,13 +677,71 @@ __device__ __forceinline__ void st8(bf16* p, const float (&f)[8]) {
   v.store(p);
 }
 
-// A warp owns a token: its rotary row and the norm weights are read once for all heads, nothing is divided, and the
-// heads come QK_U warp-wide loads at a time.  Bound by memory.  (One (token, head) item after the other, each behind a
-// 64-bit division and with its own rotary row, before: 65536 x 24 heads of 128, forward 239 -> 205 us, backward 584 -> 517.)
-constexpr int QK_U = 3;
+// Two splits of the work.  By items: a group of LPH lanes takes one (token, head) after the other, few registers, many warps.
+// By tokens: a warp owns a token, its rotary row and the norm weights are read once for all heads, nothing is divided, and
+// the heads come QK_FWD_U (QK_BWD_U) warp-wide loads at a time; that takes 117 registers (backward: 201), so it needs many
+// rows and turns of loads that are full.  Both are bound by memory at size; a head's result is the same in both, bit by bit
+// (the weight gradients sum in another order).  us, items | tokens, rows x heads:
+//   forward with norm, heads of 128: 600 x 24: 4.1 | 5.4, 5003 x 24: 16.2 | 15.7, 32768 x 24: 103 | 92, 32768 x 16 (turns 2/3
+//   full): 73 | 83; of 64: 32768 x 40: 85 | 85, 32768 x 20: 48 | 56;
+//   without norm: 128: 600 x 24: 3.8 | 4.5, 1500 x 24: 6.0 | 5.5, 32768 x 24: 97 | 80; 64: 10000 x 40: 25.6 | 25.5, 32768 x 40:
+//   81 | 72, 32768 x 20 (one turn): 46 | 48;
+//   backward with norm, 128: 5003 x 24: 38 | 53, 32768 x 24: 214 | 211, 65536 x 24: 584 | 517, 65536 x 16: 284 | 293; 64: 32768 x
+//   40: 188 | 219;  without: 128: 5003 x 24: 17 | 17, 32768 x 24: 150 | 131; 64: 32768 x 32: 103 | 93, 32768 x 20: 68 | 90.
+constexpr int QK_FWD_U = 3, QK_BWD_U = 2;
 
 template <int LPH>
-__global__ void __launch_bounds__(256) qk_norm_rope_fwd_vec_kernel(const QKRopeParams p) {
+__global__ void __launch_bounds__(256) qk_norm_rope_fwd_items_kernel(const QKRopeParams p) {
+  constexpr int GPW = 32 / LPH;                         // (token, head) items per warp
+  const int lane = threadIdx.x & 31, sub = lane % LPH, grp = lane / LPH;
+  const int warps = blockDim.x >> 5;
+  const int heads = p.H + p.HK;
+  const int64_t total = p.rows * heads;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * warps * GPW;
+  for (int64_t base = (static_cast<int64_t>(blockIdx.x) * warps + (threadIdx.x >> 5)) * GPW; base < total; base += step) {
+    const int64_t item = base + grp;
+    const bool live = item < total;
+    const int64_t row = live ? item / heads : 0;
+    const int h = live ? static_cast<int>(item % heads) : 0;
+    const bool is_q = h < p.H;
+    const int hh = is_q ? h : h - p.H;
+    const bf16* in = (is_q ? p.q_in + row * p.ldq : p.k_in + row * p.ldk) + hh * p.D + sub * 8;
+    bf16* out = (is_q ? p.q_out + row * p.ldqo : p.k_out + row * p.ldko) + hh * p.D + sub * 8;
+    const bf16* w = is_q ? p.qw : p.kw;
+    const int pos = p.positions != nullptr ? p.positions[row] : static_cast<int>(row % p.T) + p.pos_offset;
+    float x1[8], x2[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x1[i] = x2[i] = 0.f;
+    if (live) { ld8(in, x1); ld8(in + p.half, x2); }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss += x1[i] * x1[i] + x2[i] * x2[i];
+    float rstd = 1.f;
+    if (w != nullptr) rstd = rsqrtf(group_sum<LPH>(ss) / p.D + p.eps);
+    if (!live) continue;
+    float w1[8], w2[8], c[8], sn[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { w1[i] = w2[i] = c[i] = 1.f; sn[i] = 0.f; }
+    if (w != nullptr) { ld8(w + sub * 8, w1); ld8(w + p.half + sub * 8, w2); }
+    if (p.cos != nullptr) {
+      ld8(p.cos + static_cast<int64_t>(pos) * p.half + sub * 8, c);
+      ld8(p.sin + static_cast<int64_t>(pos) * p.half + sub * 8, sn);
+    }
+    float o1[8], o2[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float y1 = x1[i] * rstd * w1[i], y2 = x2[i] * rstd * w2[i];
+      o1[i] = y1 * c[i] - y2 * sn[i];
+      o2[i] = y1 * sn[i] + y2 * c[i];
+    }
+    st8(out, o1);
+    st8(out + p.half, o2);
+  }
+}
+
+template <int LPH>
+__global__ void __launch_bounds__(256) qk_norm_rope_fwd_tokens_kernel(const QKRopeParams p) {
+  constexpr int QK_U = QK_FWD_U;
   constexpr int GPW = 32 / LPH;                         // heads per warp-wide load
   const int lane = threadIdx.x & 31, sub = lane % LPH, grp = lane / LPH;
   const int warps = blockDim.x >> 5;
@@ -813,7 +871,100 @@ __global__ void __launch_bounds__(256) decode_qkv_kernel(const DecodeQKVParams p
 }
 
 template <int LPH>
-__global__ void __launch_bounds__(256) qk_norm_rope_bwd_vec_kernel(const QKRopeParams p) {
+__global__ void __launch_bounds__(256) qk_norm_rope_bwd_items_kernel(const QKRopeParams p) {
+  __shared__ float red[2][256];                           // [q|k][D <= 256], shared atomics at the end
+  constexpr int GPW = 32 / LPH;
+  const int lane = threadIdx.x & 31, sub = lane % LPH, grp = lane / LPH;
+  const int warps = blockDim.x >> 5;
+  const int heads = p.H + p.HK;
+  const int64_t total = p.rows * heads;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * warps * GPW;
+  float dwq1[8], dwq2[8], dwk1[8], dwk2[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) dwq1[i] = dwq2[i] = dwk1[i] = dwk2[i] = 0.f;
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) (&red[0][0])[i] = 0.f;
+  __syncthreads();
+
+  for (int64_t base = (static_cast<int64_t>(blockIdx.x) * warps + (threadIdx.x >> 5)) * GPW; base < total; base += step) {
+    const int64_t item = base + grp;
+    const bool live = item < total;
+    const int64_t row = live ? item / heads : 0;
+    const int h = live ? static_cast<int>(item % heads) : 0;
+    const bool is_q = h < p.H;
+    const int hh = is_q ? h : h - p.H;
+    const bf16* in = (is_q ? p.q_in + row * p.ldq : p.k_in + row * p.ldk) + hh * p.D + sub * 8;
+    const bf16* gin = (is_q ? p.dq + row * p.lddq : p.dk + row * p.lddk) + hh * p.D + sub * 8;
+    bf16* out = (is_q ? p.q_out + row * p.ldqo : p.k_out + row * p.ldko) + hh * p.D + sub * 8;
+    const bf16* w = is_q ? p.qw : p.kw;
+    const int pos = p.positions != nullptr ? p.positions[row] : static_cast<int>(row % p.T) + p.pos_offset;
+    float x1[8], x2[8], d1[8], d2[8], c[8], sn[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { x1[i] = x2[i] = d1[i] = d2[i] = 0.f; c[i] = 1.f; sn[i] = 0.f; }
+    if (live) {
+      ld8(gin, d1); ld8(gin + p.half, d2);
+      if (w != nullptr) { ld8(in, x1); ld8(in + p.half, x2); }
+      if (p.cos != nullptr) {
+        ld8(p.cos + static_cast<int64_t>(pos) * p.half + sub * 8, c);
+        ld8(p.sin + static_cast<int64_t>(pos) * p.half + sub * 8, sn);
+      }
+    }
+    float g1[8], g2[8];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      g1[i] = d1[i] * c[i] + d2[i] * sn[i];               // transpose of the rotation
+      g2[i] = -d1[i] * sn[i] + d2[i] * c[i];
+      ss += x1[i] * x1[i] + x2[i] * x2[i];
+    }
+    if (w == nullptr) {
+      if (live) { st8(out, g1); st8(out + p.half, g2); }
+      continue;
+    }
+    const float rstd = rsqrtf(group_sum<LPH>(ss) / p.D + p.eps);
+    float w1[8], w2[8];
+    ld8(w + sub * 8, w1);
+    ld8(w + p.half + sub * 8, w2);
+    float dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      x1[i] *= rstd;
+      x2[i] *= rstd;
+      if (live) {
+        if (is_q) { dwq1[i] += g1[i] * x1[i]; dwq2[i] += g2[i] * x2[i]; }
+        else      { dwk1[i] += g1[i] * x1[i]; dwk2[i] += g2[i] * x2[i]; }
+      }
+      g1[i] *= w1[i];
+      g2[i] *= w2[i];
+      dot += g1[i] * x1[i] + g2[i] * x2[i];
+    }
+    dot = group_sum<LPH>(dot) / p.D;
+    if (!live) continue;
+    float o1[8], o2[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      o1[i] = rstd * (g1[i] - x1[i] * dot);
+      o2[i] = rstd * (g2[i] - x2[i] * dot);
+    }
+    st8(out, o1);
+    st8(out + p.half, o2);
+  }
+  if (p.dqw_partial == nullptr) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    atomicAdd(&red[0][sub * 8 + i], dwq1[i]);
+    atomicAdd(&red[0][p.half + sub * 8 + i], dwq2[i]);
+    atomicAdd(&red[1][sub * 8 + i], dwk1[i]);
+    atomicAdd(&red[1][p.half + sub * 8 + i], dwk2[i]);
+  }
+  __syncthreads();
+  for (int col = threadIdx.x; col < p.D; col += blockDim.x) {
+    p.dqw_partial[static_cast<int64_t>(blockIdx.x) * p.D + col] = red[0][col];
+    p.dkw_partial[static_cast<int64_t>(blockIdx.x) * p.D + col] = red[1][col];
+  }
+}
+
+template <int LPH>
+__global__ void __launch_bounds__(256) qk_norm_rope_bwd_tokens_kernel(const QKRopeParams p) {
   __shared__ float red[2][256];                           // [q|k][D <= 256], shared atomics at the end
   constexpr int GPW = 32 / LPH;
   const int lane = threadIdx.x & 31, sub = lane % LPH, grp = lane / LPH;
@@ -841,7 +992,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_vec_kernel(const QKRopeP
       ld8(p.cos + static_cast<int64_t>(pos) * p.half + sub * 8, c);
       ld8(p.sin + static_cast<int64_t>(pos) * p.half + sub * 8, sn);
     }
-    constexpr int U = 2;
+    constexpr int U = QK_BWD_U;
     for (int h0 = grp; h0 - grp < heads; h0 += GPW * U) {
       Vec8 gr[U][2], in[U][2];
 #pragma unroll
@@ -1077,6 +1228,17 @@ static bool qk_vec_ok(const QKRopeParams& p) {
          al(p.cos) && al(p.sin);
 }
 
+// Whether the tokens form is the faster one (see the kernels for both sides of each line).
+static bool qk_by_tokens(const QKRopeParams& p, bool backward) {
+  const int lph = p.half / 8, heads = p.H + p.HK, per_turn = 32 / lph * (backward ? QK_BWD_U : QK_FWD_U);
+  const int turns = (heads + per_turn - 1) / per_turn;
+  const bool full = 8 * heads >= 7 * turns * per_turn, d128 = lph == 8;
+  if (lph != 4 && lph != 8) return false;
+  if (p.qw != nullptr) return d128 && (backward ? turns >= 3 && p.rows >= 32768 : full && p.rows >= 8192);
+  if (turns < 2 || (backward ? 5 * heads < 4 * turns * per_turn : 3 * heads < 2 * turns * per_turn)) return false;
+  return p.rows >= (!d128 ? 16384 : backward ? (turns >= 3 ? 8192 : 16384) : (full ? 1536 : 16384));
+}
+
 static int qk_check(int D, int half) { return (D > 256 || half * 2 > D || half <= 0) ? TTCD_ERR_ARG : TTCD_OK; }
 
 // Forward: q_out/k_out = rope(headnorm(q_in/k_in)).  Row strides in elements.
@@ -1096,10 +1258,14 @@ TTCD_EXPORT int ttcd_qk_norm_rope_fwd(const void* q_in, long long ldq, const voi
   const unsigned grid = static_cast<unsigned>(std::min<long long>((items + 7) / 8, 148LL * 16));
   if (qk_vec_ok(p)) {
     const int lph = half / 8;
-    const unsigned vgrid = static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 148LL * 16));
-    if (lph == 4) qk_norm_rope_fwd_vec_kernel<4><<<vgrid, 256, 0, st>>>(p);
-    else if (lph == 8) qk_norm_rope_fwd_vec_kernel<8><<<vgrid, 256, 0, st>>>(p);
-    else qk_norm_rope_fwd_vec_kernel<16><<<vgrid, 256, 0, st>>>(p);
+    const unsigned vgrid = static_cast<unsigned>(std::min<long long>((items * lph / 32 + 7) / 8 + 1, 148LL * 16));
+    const unsigned tgrid = static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 148LL * 16));
+    const bool tokens = qk_by_tokens(p, false);
+    if (tokens && lph == 4) qk_norm_rope_fwd_tokens_kernel<4><<<tgrid, 256, 0, st>>>(p);
+    else if (tokens) qk_norm_rope_fwd_tokens_kernel<8><<<tgrid, 256, 0, st>>>(p);
+    else if (lph == 4) qk_norm_rope_fwd_items_kernel<4><<<vgrid, 256, 0, st>>>(p);
+    else if (lph == 8) qk_norm_rope_fwd_items_kernel<8><<<vgrid, 256, 0, st>>>(p);
+    else qk_norm_rope_fwd_items_kernel<16><<<vgrid, 256, 0, st>>>(p);
     return static_cast<int>(cudaGetLastError());
   }
   if (half <= 32) qk_norm_rope_fwd_kernel<1><<<grid, 256, 0, st>>>(p);
@@ -1147,9 +1313,12 @@ TTCD_EXPORT int ttcd_qk_norm_rope_bwd(const void* dq, long long lddq, const void
   cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
   if (qk_vec_ok(p)) {
     const int lph = half / 8;
-    if (lph == 4) qk_norm_rope_bwd_vec_kernel<4><<<nblocks, 256, 0, st>>>(p);
-    else if (lph == 8) qk_norm_rope_bwd_vec_kernel<8><<<nblocks, 256, 0, st>>>(p);
-    else qk_norm_rope_bwd_vec_kernel<16><<<nblocks, 256, 0, st>>>(p);
+    const bool tokens = qk_by_tokens(p, true);
+    if (tokens && lph == 4) qk_norm_rope_bwd_tokens_kernel<4><<<nblocks, 256, 0, st>>>(p);
+    else if (tokens) qk_norm_rope_bwd_tokens_kernel<8><<<nblocks, 256, 0, st>>>(p);
+    else if (lph == 4) qk_norm_rope_bwd_items_kernel<4><<<nblocks, 256, 0, st>>>(p);
+    else if (lph == 8) qk_norm_rope_bwd_items_kernel<8><<<nblocks, 256, 0, st>>>(p);
+    else qk_norm_rope_bwd_items_kernel<16><<<nblocks, 256, 0, st>>>(p);
     return static_cast<int>(cudaGetLastError());
   }
   if (half <= 32) qk_norm_rope_bwd_kernel<1><<<nblocks, 256, 0, st>>>(p);

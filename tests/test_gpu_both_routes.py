@@ -1,0 +1,46 @@
+"""Ops that split their work in one way for large calls and in another for small ones: the two give the same values, bit by
+bit, so a large call is compared with the same rows in small calls (weight gradients, which sum over the rows, with float64).
+Sizes lie on both sides of each rule; the small route itself is compared with the oracle in the ops' own tests."""
+import pytest
+import torch
+
+from ttcd_b200 import ops
+from ttcd_b200.ops import cuda
+
+DEV, BF = "cuda:0", torch.bfloat16
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,H,HK", [(128, 4, 2), (128, 8, 4), (128, 7, 4), (128, 16, 16), (128, 3, 0), (64, 15, 5), (64, 16, 17)])
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("rows", [1600, 8200, 32771])
+def test_head_norm_and_rotary(D, H, HK, norm, rows):
+    torch.manual_seed(rows)
+    q, k = torch.randn(1, rows, H, D, device=DEV).to(BF), torch.randn(1, rows, HK, D, device=DEV).to(BF)
+    w = [(1 + 0.2 * torch.randn(D, device=DEV)).to(BF) if norm else None for _ in range(2)]
+    cos, sin = (torch.randn(rows, D // 2, device=DEV).to(BF) for _ in range(2))
+    dq, dk = torch.randn_like(q), torch.randn_like(k)
+
+    def run(a, b):
+        qs, ks = (t[:, a:b].contiguous().requires_grad_() for t in (q, k))
+        ws = [None if t is None else t.clone().requires_grad_() for t in w]
+        out = cuda.qk_norm_rope(qs, ks, *ws, 1e-6, cos, sin, a)
+        leaves = [qs] + ([ks] if HK else []) + [t for t in ws if t is not None]
+        grads = torch.autograd.grad(out if HK else out[:1], leaves, (dq[:, a:b], dk[:, a:b])[:2 if HK else 1])
+        return out, grads
+
+    out, grads = run(0, rows)
+    parts = [run(a, min(a + 1000, rows)) for a in range(0, rows, 1000)]
+    for i in range(2):
+        assert torch.equal(out[i], torch.cat([p[0][i] for p in parts], 1))
+    for i in range(2 if HK else 1):
+        assert torch.equal(grads[i], torch.cat([p[1][i] for p in parts], 1))
+    if norm:
+        n = 2 if HK else 1
+        for x, dy, g in zip((q, k)[:n], (dq, dk)[:n], grads[n:]):
+            xd, d = x[0].double(), dy[0].double()
+            lo, hi, c, s = d[..., :D // 2], d[..., D // 2:], cos.double()[:, None], sin.double()[:, None]
+            d = torch.cat([lo * c + hi * s, hi * c - lo * s], -1)
+            want = (d * xd * (xd.square().mean(-1, keepdim=True) + 1e-6).rsqrt()).sum((0, 1))
+            # fp32 sums of rows * heads terms of size ~1.5 in blocks (random signs), one rounding to bf16
+            assert ((g.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * (rows * x.shape[2]) ** 0.5).all()
