@@ -29,13 +29,34 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = raw;
 }
 
-// A thread keeps its 8 columns and takes SW_ROWS rows, whose loads are all in flight before the first is used; nothing is
-// divided.  65536 x 3072: 248 -> 211 us (188 us of bytes at the copy rate).  (The backward, with five streams, gained
-// nothing from it: 320 and 311, but 103 and 105 us at 7035 x 8192.)
-constexpr int SW_THREADS = 128, SW_ROWS = 4;
+// z = gate * sigmoid(gate) * up;  gate/up rows may be strided views of one packed buffer.  Two splits of the work: one vector
+// of 8 per thread and turn, or (by rows) a thread keeps its 8 columns and takes SW_ROWS rows, whose loads are all in flight
+// before the first is used, without a division.  Many wide rows gain from the second; a block of it covers 1024 columns, so
+// narrow rows leave its threads idle, and few rows leave it too few blocks.  us, by vectors | by rows, rows x columns:
+// 300 x 3072: 3.2 | 4.2, 2400 x 3072: 9.6 | 9.8, 5000 x 3072: 18.6 | 17.2, 40000 x 3072: 139 | 114, 5000 x 8192: 49 | 42;
+// 20000 x 512: 12.5 | 13.3, 40000 x 512: 25.9 | 24.8, 100000 x 256: 31.2 | 31.1, 100000 x 64: 8.8 | 29.8.
+// (The backward, with five streams, gained nothing from it: 320 and 311, but 103 and 105 us at 7035 x 8192.)
+constexpr int SW_THREADS = 128, SW_ROWS = 4, SW_COLS = SW_THREADS * 8;
 
-// z = gate * sigmoid(gate) * up;  gate/up rows may be strided views of one packed buffer.
-__global__ void __launch_bounds__(SW_THREADS) swiglu_fwd_kernel(const bf16* __restrict__ gate, const bf16* __restrict__ up,
+__global__ void __launch_bounds__(256) swiglu_fwd_vectors_kernel(const bf16* __restrict__ gate, const bf16* __restrict__ up,
+                                                                 bf16* __restrict__ z, int64_t rows, int d, int64_t ldg,
+                                                                 int64_t ldu, int64_t ldz) {
+  const int vec_per_row = d / 8;
+  const int64_t total = rows * vec_per_row;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = i / vec_per_row;
+    const int c = static_cast<int>(i % vec_per_row) * 8;
+    float g[8], u[8], o[8];
+    load8(gate + r * ldg + c, g);
+    load8(up + r * ldu + c, u);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = g[k] / (1.f + __expf(-g[k])) * u[k];
+    store8(z + r * ldz + c, o);
+  }
+}
+
+__global__ void __launch_bounds__(SW_THREADS) swiglu_fwd_rows_kernel(const bf16* __restrict__ gate, const bf16* __restrict__ up,
                                                                 bf16* __restrict__ z, int64_t rows, int d, int64_t ldg,
                                                                 int64_t ldu, int64_t ldz) {
   const int c = (blockIdx.y * SW_THREADS + threadIdx.x) * 8;
@@ -245,11 +266,19 @@ using namespace ttcd;
 TTCD_EXPORT int ttcd_swiglu_fwd(const void* gate, const void* up, void* z, long long rows, int d, long long ldg,
                                 long long ldu, long long ldz, void* stream_ptr) {
   if (d % 8 != 0 || ldg % 8 != 0 || ldu % 8 != 0 || ldz % 8 != 0 || rows <= 0) return TTCD_ERR_ARG;
+  const bf16* g = static_cast<const bf16*>(gate);
+  const bf16* u = static_cast<const bf16*>(up);
+  cudaStream_t st = static_cast<cudaStream_t>(stream_ptr);
   const long long row_blocks = (rows + SW_ROWS - 1) / SW_ROWS;
-  if (row_blocks > 0x7fffffffLL || d > 65535 * SW_THREADS * 8) return TTCD_ERR_SIZE;
-  const dim3 grid(static_cast<unsigned>(row_blocks), (d / 8 + SW_THREADS - 1) / SW_THREADS);
-  swiglu_fwd_kernel<<<grid, SW_THREADS, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
-      static_cast<const bf16*>(gate), static_cast<const bf16*>(up), static_cast<bf16*>(z), rows, d, ldg, ldu, ldz);
+  const int col_blocks = (d + SW_COLS - 1) / SW_COLS;
+  // by rows from 8 M elements, counting only the share of a block's threads that have columns
+  if (rows * d * d >= (8LL << 20) * SW_COLS * col_blocks && row_blocks <= 0x7fffffffLL && col_blocks <= 65535) {
+    swiglu_fwd_rows_kernel<<<dim3(static_cast<unsigned>(row_blocks), col_blocks), SW_THREADS, 0, st>>>(
+        g, u, static_cast<bf16*>(z), rows, d, ldg, ldu, ldz);
+  } else {
+    const unsigned grid = static_cast<unsigned>(std::min<long long>((rows * (d / 8) + 255) / 256, 148LL * 32));
+    swiglu_fwd_vectors_kernel<<<grid, 256, 0, st>>>(g, u, static_cast<bf16*>(z), rows, d, ldg, ldu, ldz);
+  }
   return static_cast<int>(cudaGetLastError());
 }
 

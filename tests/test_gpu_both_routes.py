@@ -44,3 +44,18 @@ def test_head_norm_and_rotary(D, H, HK, norm, rows):
             want = (d * xd * (xd.square().mean(-1, keepdim=True) + 1e-6).rsqrt()).sum((0, 1))
             # fp32 sums of rows * heads terms of size ~1.5 in blocks (random signs), one rounding to bf16
             assert ((g.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * (rows * x.shape[2]) ** 0.5).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [64, 520, 1024, 1032, 3072])
+@pytest.mark.parametrize("total", [8 << 20, 40 << 20])
+def test_swiglu(d, total):
+    rows = total // d + 3
+    torch.manual_seed(d)
+    gate_up = (2 * torch.randn(rows, 2 * d, device=DEV)).to(BF)
+    whole = cuda.swiglu_packed(gate_up)
+    assert torch.equal(whole, torch.cat([cuda.swiglu_packed(gate_up[a:a + 500]) for a in range(0, rows, 500)]))
+    g, u = gate_up[-700:, :d].double(), gate_up[-700:, d:].double()
+    want = torch.nn.functional.silu(g) * u
+    # one rounding to bf16; the fp32 exponential's error is far below it
+    assert ((whole[-700:].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
