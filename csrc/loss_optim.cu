@@ -32,19 +32,24 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
 // l2_factor > 0 adds the l2-warp term on EVERY row (ignored ones too, as the reference's fused linear-CE does,
 // fla/modules/fused_linear_cross_entropy.py:250-283): max logit * l2_factor * (*grad_scale) at the arg-max column
 // (the lowest column on ties); the loss value is unchanged by it.
-// A thread does the work of CE_U threads of a 1024-thread block, with an accumulator for each, so that its CE_U loads are in
-// flight together and several rows share an SM (one's reductions hide behind another's loads) while every sum keeps its
-// order.  us, with 1024 threads | now: 16384 x 32000: 704 | 615, with lse_part 513 | 426; 9472 x 151936: 1711 | 1570, 1084 | 981.
+// A block of 256 threads does the work of one of 1024: a thread has CE_U accumulators, so that its CE_U loads are in flight
+// together and several rows share an SM (one's reductions hide behind another's loads) while every sum keeps its order; the
+// outputs of the two are the same bit by bit.  With fewer rows than SMs there is nothing to share, and a long row takes what
+// one block's threads can have in flight: those get 1024.  us, 1024 | 256 threads: 16384 x 32000: 704 | 615, with lse_part
+// 513 | 426; 9472 x 151936: 1711 | 1570, 1084 | 981;  128 x 32000: 8.3 | 9.8, 150 x 32000: 13.4 | 13.0;  128 x 151936:
+// 26.5 | 37.0, 300 x 151936: 73 | 80, 450 x 151936: 102 | 103;  128 x 4096: 3.9 | 4.0, 150 x 4096: 5.1 | 4.5.
 // The gradient goes to `grad` (rows ld apart like the logits; it may be `logits` itself).
-constexpr int CE_THREADS = 256, CE_U = 4, CE_ROW = CE_THREADS * CE_U;
+constexpr int CE_ROW = 1024;
 
-// One value per thread of a CE_ROW-thread block, v[u] for thread u * CE_THREADS + threadIdx.x; block_reduce's order.
-__device__ __forceinline__ float ce_reduce(float (&v)[CE_U], float* scratch, bool is_max) {
+// One value per thread of a CE_ROW-thread block, v[u] for thread u * THREADS + threadIdx.x; block_reduce's order.
+template <int THREADS>
+__device__ __forceinline__ float ce_reduce(float (&v)[CE_ROW / THREADS], float* scratch, bool is_max) {
+  constexpr int CE_U = CE_ROW / THREADS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int u = 0; u < CE_U; ++u) {
     const float w = is_max ? warp_max(v[u]) : warp_sum(v[u]);
-    if (lane == 0) scratch[u * (CE_THREADS / 32) + warp] = w;
+    if (lane == 0) scratch[u * (THREADS / 32) + warp] = w;
   }
   __syncthreads();
   if (warp == 0) {
@@ -58,11 +63,13 @@ __device__ __forceinline__ float ce_reduce(float (&v)[CE_U], float* scratch, boo
   return out;
 }
 
-__global__ void __launch_bounds__(CE_THREADS) ce_rows_kernel(const bf16* logits, bf16* grad, const int64_t* __restrict__ labels,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) ce_rows_kernel(const bf16* logits, bf16* grad, const int64_t* __restrict__ labels,
                                                        float* __restrict__ loss_row, float* __restrict__ lse_row,
                                                        const float* __restrict__ grad_scale, int V, int64_t ld,
                                                        int ignore_index, int write_grad, float eps, float zeta,
                                                        float l2_factor, const float2* __restrict__ lse_part, int n_parts) {
+  constexpr int CE_U = CE_ROW / THREADS;
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
   const bf16* lr = logits + row * ld;
@@ -79,7 +86,7 @@ __global__ void __launch_bounds__(CE_THREADS) ce_rows_kernel(const bf16* logits,
     for (int base = threadIdx.x; base < n_parts; base += CE_ROW) {
 #pragma unroll
       for (int u = 0; u < CE_U; ++u) {
-        const int i = base + u * CE_THREADS;
+        const int i = base + u * THREADS;
         if (i >= n_parts) break;
         const float2 t = lse_part[row * n_parts + i];
         if (t.x > m[u]) {
@@ -94,12 +101,12 @@ __global__ void __launch_bounds__(CE_THREADS) ce_rows_kernel(const bf16* logits,
       uint4 raws[CE_U];
 #pragma unroll
       for (int u = 0; u < CE_U; ++u) {
-        const int i = base + u * CE_THREADS;
+        const int i = base + u * THREADS;
         if (i < nvec) raws[u] = *reinterpret_cast<const uint4*>(lr + i * 8);
       }
 #pragma unroll
       for (int u = 0; u < CE_U; ++u) {
-        const int i = base + u * CE_THREADS;
+        const int i = base + u * THREADS;
         if (i >= nvec) break;
         const uint32_t w[4] = {raws[u].x, raws[u].y, raws[u].z, raws[u].w};
         float f[8];
@@ -128,7 +135,7 @@ __global__ void __launch_bounds__(CE_THREADS) ce_rows_kernel(const bf16* logits,
     }
 #pragma unroll
     for (int u = 0; u < CE_U; ++u) {
-      const int i = nvec * 8 + threadIdx.x + u * CE_THREADS;       // fewer than 8 columns are left
+      const int i = nvec * 8 + threadIdx.x + u * THREADS;       // fewer than 8 columns are left
       if (i < V) {
         const float f = __bfloat162float(lr[i]);
         if (f > m[u]) {
@@ -141,18 +148,18 @@ __global__ void __launch_bounds__(CE_THREADS) ce_rows_kernel(const bf16* logits,
       }
     }
   }
-  const float gm = ce_reduce(m, scratch, true);
+  const float gm = ce_reduce<THREADS>(m, scratch, true);
 #pragma unroll
   for (int u = 0; u < CE_U; ++u) s[u] = (m[u] == -INFINITY) ? 0.f : s[u] * __expf(m[u] - gm);
-  const float gs = ce_reduce(s, scratch, false);
+  const float gs = ce_reduce<THREADS>(s, scratch, false);
   const float lse = gm + __logf(gs);
   float mean_x = 0.f;
-  if (eps != 0.f) mean_x = ce_reduce(sumx, scratch, false) / static_cast<float>(V);
+  if (eps != 0.f) mean_x = ce_reduce<THREADS>(sumx, scratch, false) / static_cast<float>(V);
   int arg_col = -1;
   if (l2_factor != 0.f && write_grad) {       // column indices are below 2^24: exact as floats
 #pragma unroll
     for (int u = 0; u < CE_U; ++u) m[u] = m[u] == gm ? -static_cast<float>(arg[u]) : -INFINITY;
-    arg_col = -static_cast<int>(ce_reduce(m, scratch, true));
+    arg_col = -static_cast<int>(ce_reduce<THREADS>(m, scratch, true));
   }
   const bool valid = label != ignore_index && label >= 0 && label < V;
   if (threadIdx.x == 0) {
@@ -169,12 +176,12 @@ __global__ void __launch_bounds__(CE_THREADS) ce_rows_kernel(const bf16* logits,
     uint4 raws[CE_U];
 #pragma unroll
     for (int u = 0; u < CE_U; ++u) {
-      const int i = base + u * CE_THREADS;
+      const int i = base + u * THREADS;
       if (i < nvec) raws[u] = *reinterpret_cast<const uint4*>(lr + i * 8);
     }
 #pragma unroll
     for (int u = 0; u < CE_U; ++u) {
-      const int i = base + u * CE_THREADS;
+      const int i = base + u * THREADS;
       if (i >= nvec) break;
       uint32_t w[4] = {raws[u].x, raws[u].y, raws[u].z, raws[u].w};
 #pragma unroll
@@ -418,7 +425,9 @@ TTCD_EXPORT int ttcd_ce_rows(const void* logits, void* grad, const long long* la
   if (rows <= 0 || V <= 0 || ld % 8 != 0 || (write_grad && (grad_scale == nullptr || grad == nullptr))) return TTCD_ERR_ARG;
   if (label_smoothing < 0.f || label_smoothing >= 1.f || V >= (1 << 24)) return TTCD_ERR_ARG;
   if (lse_part != nullptr && (n_parts <= 0 || label_smoothing != 0.f || l2_factor != 0.f)) return TTCD_ERR_ARG;
-  ce_rows_kernel<<<static_cast<unsigned>(rows), CE_THREADS, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
+  const bool wide = V > 8192 && rows <= 148LL * (V > 65536 ? 3 : 1);
+  auto kern = wide ? ce_rows_kernel<1024> : ce_rows_kernel<256>;
+  kern<<<static_cast<unsigned>(rows), wide ? 1024 : 256, 0, static_cast<cudaStream_t>(stream_ptr)>>>(
       static_cast<const bf16*>(logits), static_cast<bf16*>(grad), reinterpret_cast<const int64_t*>(labels), loss_row, lse_row, grad_scale, V, ld,
       ignore_index, write_grad, label_smoothing, lse_square_scale, l2_factor, reinterpret_cast<const float2*>(lse_part),
       n_parts);

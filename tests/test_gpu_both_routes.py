@@ -59,3 +59,23 @@ def test_swiglu(d, total):
     want = torch.nn.functional.silu(g) * u
     # one rounding to bf16; the fp32 exponential's error is far below it
     assert ((whole[-700:].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,rows", [(8192, 149), (8200, 149), (32000, 160), (32003, 160), (70000, 460)])
+@pytest.mark.parametrize("smoothing,z,l2", [(0.0, 0.0, 0.0), (0.1, 1e-3, 0.0), (0.0, 0.0, 1e-3)])
+def test_cross_entropy_rows(V, rows, smoothing, z, l2):
+    torch.manual_seed(V)
+    ld = -(-V // 8) * 8
+    logits = (3 * torch.randn(rows, ld, device=DEV)).to(BF)[:, :V]
+    labels = torch.randint(0, V, (rows,), device=DEV)
+    labels[1] = -100
+    scale = torch.full((1,), 0.25, device=DEV)
+
+    def run(a, b):
+        grad = torch.zeros(b - a, ld, dtype=BF, device=DEV)[:, :V]
+        return cuda._ce_rows(logits[a:b], labels[a:b], scale, -100, True, smoothing, z, l2, grad=grad), grad
+
+    loss, grad = run(0, rows)
+    parts = [run(a, min(a + 40, rows)) for a in range(0, rows, 40)]
+    assert torch.equal(loss, torch.cat([p[0] for p in parts])) and torch.equal(grad, torch.cat([p[1] for p in parts]))
