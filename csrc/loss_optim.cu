@@ -231,8 +231,9 @@ __global__ void __launch_bounds__(256) lse_merge_kernel(const bf16* __restrict__
 
 // Fused AdamW on a flat fp32 master shard.  grad is bf16 or fp32.  coef (device scalar, may be
 // null) multiplies the gradient (clip); skip (device int, may be null) != 0 leaves everything as is.
-// VEC: four elements per access (every array 16-byte aligned, bf16 ones 8); the last n % 4 elements one by one.
-// 65.5 M elements, bf16 gradient: 410 -> 308 us (284 us of bytes).
+// VEC: four elements per access (every array 16-byte aligned, bf16 ones 8); the last n % 4 elements one by one.  For 128 K
+// elements or more: below, a quarter of the threads is too few.  us, one | four per access, bf16 gradient: 1000: 2.1 | 2.6,
+// 100 K: 2.6 | 2.7, 200 K: 3.2 | 3.0, 600 K: 5.8 | 3.8, 65.5 M: 410 | 308 (284 us of bytes).
 template <typename GradT, bool VEC>
 __global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, const GradT* __restrict__ g,
                                                     float* __restrict__ m, float* __restrict__ v,
@@ -451,7 +452,7 @@ TTCD_EXPORT int ttcd_adamw(float* p, const void* g, int grad_is_bf16, float* m, 
   const uintptr_t wide = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v) |
                          (grad_is_bf16 ? 0 : reinterpret_cast<uintptr_t>(g));
   const uintptr_t narrow = reinterpret_cast<uintptr_t>(p_bf16) | (grad_is_bf16 ? reinterpret_cast<uintptr_t>(g) : 0);
-  const bool vec = (wide & 15u) == 0 && (narrow & 7u) == 0;
+  const bool vec = n >= (128 << 10) && (wide & 15u) == 0 && (narrow & 7u) == 0;
   const unsigned grid = flat_grid(vec ? (n + 3) / 4 : n);
   auto go = [&](auto kern, auto* grad) {
     kern<<<grid, 256, 0, st>>>(p, grad, m, v, static_cast<bf16*>(p_bf16), n, lr, beta1, beta2, eps, wd, bc1, bc2_sqrt, coef, skip);
