@@ -217,6 +217,30 @@ __global__ void __launch_bounds__(GV_WARPS * 32, (HI ? 1 : 2)) gemv_small_kernel
 template <bool HI, bool SWIGLU, bool NORM, bool WIDE, int STAGES>
 static int launch_gemv(const GemvParams& p, int smem, cudaStream_t stream) {
   auto kern = gemv_small_kernel<HI, SWIGLU, NORM, WIDE, STAGES>;
+// One row of x and nothing riding along: a warp per column of y, fp32 FMAs, x through L1; no ring to fill, no barrier between
+// groups.  Where a CTA of the kernel above has more than one group (N > 8 x 296) and K fills the warps' loads of 256.
+// us, this | the kernel above: 4096 x 1024: 4.6 | 5.0, 8192 x 1024: 5.8 | 8.0, 16384 x 2048: 13.1 | 15.2, 128256 x 2048: 76 |
+// 82;  2048 x 2048: 5.5 | 4.5, 1024 x 3072: 6.4 | 4.4, 49152 x 960: 25.4 | 20.2.
+__global__ void __launch_bounds__(256) gemv_row_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
+                                                       int N, int K, int64_t ldw, float alpha) {
+  const int lane = threadIdx.x & 31;
+  const int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (n >= N) return;
+  float acc = 0.f;
+  const bf16* wr = w + static_cast<int64_t>(n) * ldw;
+  for (int k = lane * 8; k < K; k += 256) {
+    const uint4 wv = *reinterpret_cast<const uint4*>(wr + k), xv = *reinterpret_cast<const uint4*>(x + k);
+    const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w}, xw[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 a = unpack_bf16(ww[i]), b = unpack_bf16(xw[i]);
+      acc = fmaf(a.x, b.x, fmaf(a.y, b.y, acc));
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  if (lane == 0) y[n] = __float2bfloat16(acc * alpha);
+}
+
   static bool configured = false;
   if (!configured) {
     TTCD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -277,5 +301,9 @@ TTCD_EXPORT int ttcd_gemv_small(const void* x, const void* w, void* y, const voi
     return norm ? dispatch_gemv<true, false, true>(p, stream) : dispatch_gemv<true, false, false>(p, stream);
   }
   if (swiglu) return norm ? dispatch_gemv<false, true, true>(p, stream) : dispatch_gemv<false, true, false>(p, stream);
+  if (M == 1 && !norm && !swiglu && res == nullptr && !early_w && N > 8 * gv_slots(false) && (K % 256 == 0 || K < 256)) {
+    gemv_row_kernel<<<static_cast<unsigned>((N + 7) / 8), 256, 0, stream>>>(p.x, p.w, p.y, N, K, ldw, alpha);
+    return static_cast<int>(cudaGetLastError());
+  }
   return norm ? dispatch_gemv<false, false, true>(p, stream) : dispatch_gemv<false, false, false>(p, stream);
 }

@@ -79,3 +79,13 @@ def test_cross_entropy_rows(V, rows, smoothing, z, l2):
     loss, grad = run(0, rows)
     parts = [run(a, min(a + 40, rows)) for a in range(0, rows, 40)]
     assert torch.equal(loss, torch.cat([p[0] for p in parts])) and torch.equal(grad, torch.cat([p[1] for p in parts]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K", [(3071, 1024), (3072, 1024), (3072, 1032), (4097, 2048), (9000, 256), (5000, 4096)])
+def test_one_row_times_weight(N, K):
+    torch.manual_seed(N)
+    x, w = torch.randn(1, K, device=DEV).to(BF), (torch.randn(N, K, device=DEV) * K ** -0.5).to(BF)
+    got, want = cuda.gemm(x, w.t(), alpha=0.5).double(), 0.5 * x.double() @ w.double().t()
+    # fp32 accumulation (K terms of size ~K^-1/2) and one rounding to bf16
+    assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -22 * K ** 0.5).all()
