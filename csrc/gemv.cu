@@ -14,11 +14,14 @@
 // The kernel may start while the one before it still runs (programmatic dependent launch): the first copies of w are
 // issued before it waits for that kernel when the caller says that no kernel still running can be writing w.
 //
-// Measured (us per launch in a graph, weights from HBM; 4096x1024 | 1024x2048 | 6144x1024 | 1024x3072 | 151936x1024):
-//   this kernel                      1 row 4.1 | 3.0 | 5.5 | 3.6 | 50     8 rows 4.3 | 3.3 | 5.8 | 4.0 | 51     16 rows 5.4 | 3.6 | 5.8 | 5.2 | 74
-//   one warp per column, fp32 FMAs   1 row 3.4 | 4.3 | 4.4 | 5.6 | 49     8 rows 8.1 | 9.9 | 11.6 | 13.8 | 180    16 rows 14 | 17 | 19 | 23 | 342
-// (before; at one row it gained a little where a CTA has more than one group, which the norm, SwiGLU and the early start
-// of the weights pay back in a decode step).
+// us per launch in a graph, weights from HBM (N x K), this kernel: 1 | 8 | 16 rows; in brackets one warp per column with fp32
+// FMAs, which one-row calls still take where it is the faster (gemv_row_kernel):
+//   4096 x 1024: 4.9 | 4.9 | 6.0 (4.6 | 8.8 | 15);  1024 x 3072: 4.4 | 4.6 | 5.9 (6.4 | 14.5 | 25);
+//   2048 x 8192: 11.0 | 13.0 | 20.1 (12.3 | 34 | 63);  16384 x 2048: 15.2 | 15.2 | 16.2 (13.1 | 39 | 71);
+//   151936 x 1024: 49 | 51 | 72 (47 | 175 | 338);  128256 x 2048: 82 | 84 | 92 (76 | 264 | 513).
+// Where two CTAs share an SM (up to 8 rows), groups of 16 rows of w (SwiGLU, or a wide output) leave a CTA's ring one stage
+// beyond K = 1568 (a stage of K = 2048 is 66 KB): nothing of it is in flight while it computes, only the other CTA reads.  The
+// wide output is at 6.4 TB/s all the same; SwiGLU of 8192 x 2048 takes 13.9 us (67 MB).
 #include "common.cuh"
 
 #include <algorithm>
@@ -214,9 +217,6 @@ __global__ void __launch_bounds__(GV_WARPS * 32, (HI ? 1 : 2)) gemv_small_kernel
   }
 }
 
-template <bool HI, bool SWIGLU, bool NORM, bool WIDE, int STAGES>
-static int launch_gemv(const GemvParams& p, int smem, cudaStream_t stream) {
-  auto kern = gemv_small_kernel<HI, SWIGLU, NORM, WIDE, STAGES>;
 // One row of x and nothing riding along: a warp per column of y, fp32 FMAs, x through L1; no ring to fill, no barrier between
 // groups.  Where a CTA of the kernel above has more than one group (N > 8 x 296) and K fills the warps' loads of 256.
 // us, this | the kernel above: 4096 x 1024: 4.6 | 5.0, 8192 x 1024: 5.8 | 8.0, 16384 x 2048: 13.1 | 15.2, 128256 x 2048: 76 |
@@ -241,6 +241,9 @@ __global__ void __launch_bounds__(256) gemv_row_kernel(const bf16* __restrict__ 
   if (lane == 0) y[n] = __float2bfloat16(acc * alpha);
 }
 
+template <bool HI, bool SWIGLU, bool NORM, bool WIDE, int STAGES>
+static int launch_gemv(const GemvParams& p, int smem, cudaStream_t stream) {
+  auto kern = gemv_small_kernel<HI, SWIGLU, NORM, WIDE, STAGES>;
   static bool configured = false;
   if (!configured) {
     TTCD_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -256,16 +259,18 @@ template <bool HI, bool SWIGLU, bool NORM, bool WIDE>
 static int stages_gemv(const GemvParams& p, cudaStream_t stream) {
   constexpr int KC = gv_xs(HI, NORM) * 32 * GV_WARPS;
   const int stage = (SWIGLU || WIDE ? 16 : 8) * gv_pitch(std::min(p.K, KC));
-  // as deep a ring as two CTAs per SM have room for (one stage is at most 99 KB)
-  if (4 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, WIDE, 4>(p, 4 * stage, stream);
-  if (3 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, WIDE, 3>(p, 3 * stage, stream);
-  if (2 * stage <= 100 * 1024) return launch_gemv<HI, SWIGLU, NORM, WIDE, 2>(p, 2 * stage, stream);
+  // as deep a ring as the CTAs of an SM have room for: two, or one with more than 8 rows (a stage is at most 99 KB)
+  constexpr int room = (HI ? 200 : 100) * 1024;
+  if (4 * stage <= room) return launch_gemv<HI, SWIGLU, NORM, WIDE, 4>(p, 4 * stage, stream);
+  if (3 * stage <= room) return launch_gemv<HI, SWIGLU, NORM, WIDE, 3>(p, 3 * stage, stream);
+  if (2 * stage <= room) return launch_gemv<HI, SWIGLU, NORM, WIDE, 2>(p, 2 * stage, stream);
   return launch_gemv<HI, SWIGLU, NORM, WIDE, 1>(p, stage, stream);
 }
 
 template <bool HI, bool SWIGLU, bool NORM>
 static int dispatch_gemv(const GemvParams& p, cudaStream_t stream) {
-  // many turns per CTA (an output vocabulary): twice the columns per turn halve the barriers (151936 x 1024: 78 -> 50 us, 6.2 TB/s)
+  // many turns per CTA (an output vocabulary): twice the columns per turn halve the barriers (151936 x 1024, one row: 78 -> 50 us,
+  // 6.2 TB/s; 128256 x 2048: 82 us, 6.4 TB/s, with a ring of one stage)
   if constexpr (!SWIGLU) {
     if (p.N >= 4 * 8 * gv_slots(HI) && p.K <= 2048) return stages_gemv<HI, SWIGLU, NORM, true>(p, stream);
   }
@@ -296,14 +301,14 @@ TTCD_EXPORT int ttcd_gemv_small(const void* x, const void* w, void* y, const voi
   p.alpha = alpha; p.eps = eps; p.early_w = early_w;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   const bool norm = norm_w != nullptr;
+  if (M == 1 && !norm && !swiglu && res == nullptr && !early_w && N > 8 * gv_slots(false) && (K % 256 == 0 || K < 256)) {
+    gemv_row_kernel<<<static_cast<unsigned>((N + 7) / 8), 256, 0, stream>>>(p.x, p.w, p.y, N, K, ldw, alpha);
+    return static_cast<int>(cudaGetLastError());
+  }
   if (M > 8) {
     if (swiglu) return norm ? dispatch_gemv<true, true, true>(p, stream) : dispatch_gemv<true, true, false>(p, stream);
     return norm ? dispatch_gemv<true, false, true>(p, stream) : dispatch_gemv<true, false, false>(p, stream);
   }
   if (swiglu) return norm ? dispatch_gemv<false, true, true>(p, stream) : dispatch_gemv<false, true, false>(p, stream);
-  if (M == 1 && !norm && !swiglu && res == nullptr && !early_w && N > 8 * gv_slots(false) && (K % 256 == 0 || K < 256)) {
-    gemv_row_kernel<<<static_cast<unsigned>((N + 7) / 8), 256, 0, stream>>>(p.x, p.w, p.y, N, K, ldw, alpha);
-    return static_cast<int>(cudaGetLastError());
-  }
   return norm ? dispatch_gemv<false, false, true>(p, stream) : dispatch_gemv<false, false, false>(p, stream);
 }
