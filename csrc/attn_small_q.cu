@@ -149,9 +149,12 @@ __global__ void __launch_bounds__(SQ_WARPS * 32) attn_small_q_partial_kernel(con
 // the lanes of a key leaves every lane with NV = U R / (D / 8) whole scores (so that each exponential is computed
 // once), and the probabilities travel back by shuffles for the fp32 P V.  Running max per pair, moved only when it
 // grows by 2^8.  No shared memory until the warps of a CTA are merged.
-// The fill count decides the split borders, so that every CTA of a captured launch has work however full the cache is.
-// Bound by the cache's bytes.  One launch for 1 x 8192 keys, 16/8 heads, D 128 (33.6 MB): the staging kernel above
-// took 40.8 us (135 KB of shared memory, so one CTA per SM that first loads and then computes, 1.7 waves).
+// The fill count decides the split borders: a captured launch cuts what is filled into as many ranges as it has CTAs per head
+// (whole turns each; the last ones are empty while little is filled).  With up to two pairs a CTA has at most 124 registers
+// per thread and two fit an SM; four and eight pairs take 182 to 232, one fits.
+// Bound by the cache's bytes: 8 x 8192 keys, 16/8 heads, D 128 (268 MB): 46 us, 0.9 of the copy rate.  1 x 8192 (33.6 MB):
+// 11 us; the staging kernel above took 40.8 us (135 KB of shared memory, so one CTA per SM that first loads and then
+// computes, 1.7 waves).
 constexpr int DEC_WARPS = 8;
 
 template <int D, int R>
@@ -371,17 +374,25 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, R <= 2 ? 2 : 1) attn_decode_pa
     float acc[DPL], lsum = 0.f;
 #pragma unroll
     for (int e = 0; e < DPL; ++e) acc[e] = 0.f;
-#pragma unroll 8
-    for (int s = sub; s < p.splits; s += WPP) {
-      const float2 t = __ldcg(&ml[s]);
-      float x[DPL];
+    constexpr int MB = 8;                           // splits in flight, also where fewer are left
+    for (int s0 = sub; s0 < p.splits; s0 += MB * WPP) {
+      float2 t[MB];
+      float x[MB][DPL];
 #pragma unroll
-      for (int e = 0; e < DPL; ++e) x[e] = __ldcg(p.part_o + (item * p.splits + s) * D + lane * DPL + e);
-      const bool some = t.x != -INFINITY;
-      const float w = some ? exp2f(t.x - M) : 0.f;
-      lsum = fmaf(some ? t.y : 0.f, w, lsum);
+      for (int u = 0; u < MB; ++u) {
+        const int s = s0 + u * WPP;
+        t[u] = s < p.splits ? __ldcg(&ml[s]) : make_float2(-INFINITY, 0.f);
 #pragma unroll
-      for (int e = 0; e < DPL; ++e) acc[e] = fmaf(some ? x[e] : 0.f, w, acc[e]);
+        for (int e = 0; e < DPL; ++e) x[u][e] = s < p.splits ? __ldcg(p.part_o + (item * p.splits + s) * D + lane * DPL + e) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < MB; ++u) {
+        const bool some = t[u].x != -INFINITY;      // (an empty split counts for nothing)
+        const float w = some ? exp2f(t[u].x - M) : 0.f;
+        lsum = fmaf(some ? t[u].y : 0.f, w, lsum);
+#pragma unroll
+        for (int e = 0; e < DPL; ++e) acc[e] = fmaf(some ? x[u][e] : 0.f, w, acc[e]);
+      }
     }
 #pragma unroll
     for (int e = 0; e < DPL; ++e) s_o[sub][r][lane * DPL + e] = acc[e];

@@ -89,3 +89,12 @@ def test_one_row_times_weight(N, K):
     got, want = cuda.gemm(x, w.t(), alpha=0.5).double(), 0.5 * x.double() @ w.double().t()
     # fp32 accumulation (K terms of size ~K^-1/2) and one rounding to bf16
     assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -22 * K ** 0.5).all()
+
+
+@pytest.mark.parametrize("D,pairs", [(64, 1), (64, 2), (64, 3), (64, 4), (64, 8), (128, 1), (128, 2), (128, 4), (128, 7)])
+@pytest.mark.parametrize("heads", [1, 5, 8, 64, 400])
+@pytest.mark.parametrize("Tk", [1, 127, 300, 2345, 70001])
+def test_key_ranges_of_a_decode_step(D, pairs, heads, Tk):
+    splits = cuda._decode_splits(heads, pairs, Tk, D)
+    turn = 8 * (32 // (D // 8)) * (8 if pairs <= 4 else 4)                  # warps x keys per load x loads
+    assert 1 <= splits <= -(-Tk // turn) and (splits == 1 or splits * heads <= 148 * (2 if pairs <= 2 else 1))

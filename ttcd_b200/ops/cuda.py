@@ -857,7 +857,7 @@ def attn_small_q(q, k, v, window=None, scale=None, kv_len=None, turns=None):
     v, ldv, sv = _attn_layout(v)
     # a decode step: the register kernel (16-byte reads of q), else 256 keys per CTA through shared memory
     few = Tq * (H // HK) <= 8 and q.data_ptr() % 16 == 0
-    splits = _decode_splits(B * HK, Tk) if few else -(-Tk // 256)     # the partial results are merged by a second pass
+    splits = _decode_splits(B * HK, Tq * (H // HK), Tk, D) if few else -(-Tk // 256)     # the partial results are merged by a second pass
     out = torch.empty(B, Tq, H, D, dtype=_BF16, device=q.device)
     part_o = torch.empty(B, H, Tq, splits, D, dtype=torch.float32, device=q.device)
     part_ml = torch.empty(B, H, Tq, splits, 2, dtype=torch.float32, device=q.device)
@@ -870,10 +870,15 @@ def attn_small_q(q, k, v, window=None, scale=None, kv_len=None, turns=None):
     return out
 
 
-def _decode_splits(heads: int, Tk: int, sms: int = 148) -> int:
-    """Key ranges per (sample, key/value head) of a decode step: two CTAs per SM in one wave, but no range shorter than
-    the 128 keys that a CTA takes per turn."""
-    return max(1, min(-(-Tk // 128), 2 * sms // heads))
+def _decode_splits(heads: int, pairs: int, Tk: int, D: int, sms: int = 148) -> int:
+    """Key ranges per (sample, key/value head) of a decode step: one wave of the CTAs that fit the chip (two per SM, one where
+    more than two (row, head) pairs take the registers), each with whole turns of a CTA (8 warps, 256 / D keys per load, 8
+    loads or, for more than four pairs, 4), none without keys.  us with ranges of 128 keys and two CTAs per SM throughout |
+    so: 32/8 heads, D 64, 1 x 8192 keys: 16.6 | 11.1, 8 x 1024: 14.8 | 10.7, 8 x 16384: 82 | 77; 32/4, D 128, 16 x 2345: 46 |
+    39; 16/8, D 128, 1 x 8192: 11.6 | 10.8."""
+    turn = 8 * (256 // D) * (8 if pairs <= 4 else 4)
+    most = max(1, min(-(-Tk // turn), sms * (2 if pairs <= 2 else 1) // heads))
+    return -(-Tk // (-(-Tk // (most * turn)) * turn))
 
 
 def lse_merge(o_a, lse_a, o_b, lse_b):
