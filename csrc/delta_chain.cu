@@ -289,6 +289,8 @@ static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t st
 // each other's waits.  us (BH x steps, D, Dv), before (scalar 16-bit shared-memory reads, every tile waited for) | now:
 // forward 32 x 64, 128, 128: 291 | 179; 12 x 47, 256, 512: 455 | 295; 96 x 64, 256, 512: 2769 | 2045 (one stage);
 // reverse, the same: 387 | 240; 720 | 429; 4466 | 3380 (one stage instead of two: 299; 557; 3749).
+// The one-stage forms are held to the registers of their CTAs per SM and spill a little: <256, 64> 76 bytes, <64, 32> 28,
+// <128, 32> 8 per thread.
 template <int D, int COLS>
 static int launch_delta_chain(const DeltaChainParams& p, int BH, cudaStream_t stream) {
   const bool alone = D == 256 && static_cast<int64_t>(p.Dv / COLS) * BH <= sm_count();
