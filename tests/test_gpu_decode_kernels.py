@@ -141,3 +141,46 @@ def test_fused_decode_step_matches_module_by_module(batch, heads, kv_heads, dim,
     for (k, v), (rk, rv) in zip(rings, dec.cache.layers.values()):
         for a, b in ((k, rk), (v, rv)):
             assert (a.float() - b.float()).norm() / b.float().norm() < 0.02
+
+
+@pytest.mark.parametrize("B,V", [(1, 1), (2, 7), (3, 4099), (16, 32000), (1, 151936)])
+def test_next_token_and_the_move_of_the_rings(B, V):
+    """Against torch.argmax (ties to the first, a NaN above all) and the arithmetic of the cache's own advance."""
+    torch.manual_seed(V)
+    logits = torch.randn(B, V, device=DEV).bfloat16()
+    logits[0, V // 2:] = logits[0].max()                      # ties
+    logits[0, V - 1] = -0.0
+    if B > 1:
+        logits[1, V // 3] = float("nan")
+    if B > 2:
+        logits[2] = float("-inf")
+    i64 = lambda *v: torch.tensor(v, dtype=torch.int64, device=DEV)          # noqa: E731
+    token, out, cursor, pos = i64(*[-1] * B).view(B, 1), torch.full((B, 3), -1, dtype=torch.int64, device=DEV), i64(1), i64(511)
+    positions, scratch = i64(*[511] * B).view(B, 1), torch.zeros(8 * B + 1, dtype=torch.int64, device=DEV)
+    rings = [(c, i64(0), torch.zeros(1, dtype=torch.int32, device=DEV)) for c in (512, 1000, 7)]
+    want = logits.float().argmax(-1)
+    for step in range(3):                                    # the last one finds its column past the end
+        cuda.decode_pick(logits, token, out, cursor, pos, positions, rings, scratch)
+        at = 512 + step
+        assert (token.view(-1) == want).all() and int(cursor) == 2 + step and int(pos) == at and (positions == at).all()
+        for c, slot, kv_len in rings:
+            assert int(slot) == at % c and int(kv_len) == min(at + 1, c)
+    assert (out[:, 0] == -1).all() and (out[:, 1] == want).all() and (out[:, 2] == want).all() and int(scratch[0]) == 0
+
+
+@pytest.mark.parametrize("B,HK,D,cap,n,start", [(1, 8, 128, 64, 64, 64), (2, 5, 64, 100, 37, 250), (3, 1, 64, 9, 9, 13), (1, 2, 128, 4096, 1, 1)])
+def test_ring_load_against_indexed_copies(B, HK, D, cap, n, start):
+    torch.manual_seed(n)
+    wide = torch.randn(B, n, 3 * HK * D, device=DEV).bfloat16()               # k and v as columns of one projection, and on their own
+    pairs = [(wide[..., :HK * D].view(B, n, HK, D), wide[..., HK * D:2 * HK * D].view(B, n, HK, D)),
+             tuple(torch.randn(B, n, HK, D, device=DEV).bfloat16() for _ in range(2)),
+             tuple(torch.randn(B * n * HK * D + 1, device=DEV).bfloat16()[1:].view(B, n, HK, D) for _ in range(2))]       # misaligned
+    rings = [tuple(torch.full((B, cap, HK, D), 7.0, device=DEV).bfloat16() for _ in range(2)) for _ in pairs]
+    assert cuda.ring_load([(*p, *r) for p, r in zip(pairs, rings)], start) == [2]
+    rows = torch.arange(start - n, start, device=DEV) % cap
+    for src, ring in zip(pairs[:2], rings):
+        for s, r in zip(src, ring):
+            want = torch.full_like(r, 7.0)
+            want.index_copy_(1, rows, s)
+            assert torch.equal(r, want)
+    assert (rings[2][0] == 7).all()

@@ -14,7 +14,7 @@ from __future__ import annotations
 
 import torch
 
-from .layers import Attention, GatedMLP, StaticWindowCache, WindowKVCache, _slab_view
+from .layers import Attention, GatedMLP, RMSNorm, StaticWindowCache, WindowKVCache, _slab_view
 
 
 def pack_projection_weights(model) -> int:
@@ -149,6 +149,7 @@ class GraphDecoder:
         self.fused = self._fused_weights(batch)
         heads = max(k.shape[2] for k, _ in self.cache.layers.values())
         self.turns = torch.zeros(batch * heads, dtype=torch.int32, device=dev)      # this decoder's merge counters
+        self.pick = torch.zeros(8 * batch + 1, dtype=torch.int64, device=dev)
         start = self.cache.start
         # warm-up on a side stream (allocator pools, rotary tables, lazily configured kernels), then rewind and capture
         side = torch.cuda.Stream(device=dev)
@@ -189,16 +190,25 @@ class GraphDecoder:
         x = core.embeddings(self.token.view(-1))
         for layer, weights in zip(core.layers, self.fused):
             x = _fused_block_step(layer, weights, x, self.cache, self.turns)
-        return cuda.gemv(core.norm(x), self.model.lm_head.weight, early_w=True)
+        norm = core.norm
+        if type(norm) is RMSNorm and norm.weight is not None and norm.weight.dtype == x.dtype and norm.weight.data_ptr() % 16 == 0:
+            return cuda.gemv(x, self.model.lm_head.weight, norm=(norm.weight, norm.eps), early_w=True)
+        return cuda.gemv(norm(x), self.model.lm_head.weight, early_w=True)
 
     @torch.no_grad()
     def _step(self) -> None:
         self.last_logits = self._logits()                # (kept for inspection; lives in the graph's pool)
+        cache = self.cache
+        if self.fused is not None and len(cache.slot) <= 4:
+            from ..ops import cuda
+            cuda.decode_pick(self.last_logits, self.token, self.out, self.cursor, cache.pos, cache.positions,
+                             [(c, cache.slot[c], cache.kv_len[c]) for c in cache.slot], self.pick)
+            return
         nxt = self.last_logits.float().argmax(-1, keepdim=True)
         self.token.copy_(nxt)
         self.out.index_copy_(1, self.cursor, nxt)
         self.cursor.add_(1)
-        self.cache.advance()
+        cache.advance()
 
     def fits(self, source: WindowKVCache, max_new_tokens: int) -> bool:
         """Whether a new prompt's cache can reuse this capture (same shapes, rings large enough, same weights)."""
@@ -225,20 +235,18 @@ class GraphDecoder:
     def load(self, source: WindowKVCache) -> None:
         """Copy a new prompt's keys and values into the rings (addresses unchanged) and rewind the device state."""
         start = next(iter(source.seen.values()))
-        for i, (k, v) in source.layers.items():
-            rk, rv = self.cache.layers[i]
-            n, cap = k.shape[1], self.cache.capacity[i]
-            rows = torch.arange(start - n, start, device=k.device) % cap
-            rk.index_copy_(1, rows, k)
-            rv.index_copy_(1, rows, v)
+        self.cache.fill(source, start)
         self.cache.start = start
         self.cache.reset(start)
         self.cursor.zero_()
+        self.taken = 0                          # tokens chosen since: the host's copy of the cursor
 
     @torch.no_grad()
     def run(self, first_token: torch.Tensor, steps: int, eos: set[int], check_every: int = 16) -> torch.Tensor:
         """``first_token`` [B,1] (chosen from the prefill logits) is fed to the first replay; returns the ``steps``
         tokens that follow it, cut after the step at which every sample had produced an end-of-sequence token."""
+        if self.taken + steps > self.out.shape[1]:
+            raise ValueError(f"{steps} more tokens after {self.taken} do not fit a decoder made for {self.out.shape[1]}")
         self.token.copy_(first_token)
         eos_t = torch.tensor(sorted(eos), device=self.token.device) if eos else None
         finished = torch.isin(first_token.squeeze(1), eos_t) if eos else None
@@ -248,6 +256,7 @@ class GraphDecoder:
             for _ in range(n):
                 self.graph.replay()
             self.cache.host_advance(n)
+            self.taken += n
             done += n
             if eos:
                 hit = torch.isin(self.out[:, :done], eos_t)

@@ -14,7 +14,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .. import ops
+from .. import _native, ops
 from ..ops import reference as ref_ops
 
 
@@ -156,9 +156,6 @@ class StaticWindowCache(WindowKVCache):
                 raise ValueError(f"layer {i}: {n} cached rows do not fit a ring of {cap}")
             rk = k.new_zeros(k.shape[0], cap, *k.shape[2:])
             rv = v.new_zeros(v.shape[0], cap, *v.shape[2:])
-            rows = torch.arange(self.start - n, self.start, device=dev) % cap
-            rk.index_copy_(1, rows, k)
-            rv.index_copy_(1, rows, v)
             self.layers[i] = (rk, rv)
             self.seen[i] = self.start
             self.capacity[i] = cap
@@ -167,7 +164,22 @@ class StaticWindowCache(WindowKVCache):
         self.positions._ttcd_bounded = True                      # never beyond max_position: no host check per step
         self.slot = {c: torch.zeros(1, dtype=torch.int64, device=dev) for c in set(self.capacity.values())}
         self.kv_len = {c: torch.zeros(1, dtype=torch.int32, device=dev) for c in set(self.capacity.values())}
+        self.fill(source, self.start)
         self.reset(self.start)
+
+    def fill(self, source: WindowKVCache, start: int) -> None:
+        """Copy the rows of ``source``, which end with token ``start`` - 1, to their places in the rings."""
+        at = list(source.layers)
+        todo = [(*source.layers[i], *self.layers[i]) for i in at]
+        left = range(len(at))
+        if _native.use_native(todo[0][0]):
+            from ..ops import cuda
+            left = cuda.ring_load(todo, start)
+        for j in left:
+            k, v, rk, rv = todo[j]
+            rows = torch.arange(start - k.shape[1], start, device=k.device) % rk.shape[1]
+            rk.index_copy_(1, rows, k)
+            rv.index_copy_(1, rows, v)
 
     def reset(self, position: int) -> None:
         """Point the device state at the token of absolute index ``position`` (the next one to be written)."""

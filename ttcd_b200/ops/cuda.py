@@ -159,6 +159,49 @@ def decode_qkv(qkv, ring_k, ring_v, slot, positions, qw, kw, eps, cos, sin, head
     return q
 
 
+def ring_load(layers: list[tuple], start: int) -> list[int]:
+    """Copies a prompt's last rows into ring buffers, all layers in one launch: ``layers`` holds (k, v, ring_k, ring_v) with k, v
+    [B, n, HK, D] and rings [B, capacity, HK, D]; row i of n goes to ring row (start - n + i) % capacity.  Returns the indices of
+    the entries it could not take (another dtype, rows that are not contiguous or not 16-byte aligned)."""
+    import ctypes
+    left, groups = [], {}
+    for at, (k, v, rk, rv) in enumerate(layers):
+        row = rk.shape[2] * rk.shape[3]
+        ok = (rk.is_contiguous() and rv.is_contiguous() and row % 8 == 0 and k.shape == v.shape and rk.shape == rv.shape
+              and k.shape[0] == rk.shape[0] and k.shape[2:] == rk.shape[2:] and k.shape[1] <= min(rk.shape[1], start)
+              and not (torch.is_grad_enabled() and (k.requires_grad or v.requires_grad)) and rk[0].numel() < 2 ** 31
+              and all(t.dtype == _BF16 and t.is_cuda and t.data_ptr() % 16 == 0 for t in (k, v, rk, rv))
+              and all(t.stride(3) == 1 and t.stride(2) == t.shape[3] and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0 for t in (k, v)))
+        if not ok:
+            left.append(at)
+        elif k.shape[1] > 0:
+            groups.setdefault((rk.shape[0], row), []).append(
+                [t.data_ptr() for t in (k, v, rk, rv)] + [k.stride(0), k.stride(1), v.stride(0), v.stride(1), rk.stride(0),
+                                                          k.shape[1], rk.shape[1]])
+    for (B, row), records in groups.items():
+        for i in range(0, len(records), 32):
+            part = records[i:i + 32]
+            flat = [x for r in part for x in r]
+            nv.call("ttcd_ring_load", (ctypes.c_longlong * len(flat))(*flat), nv.i32(len(part)), nv.i32(B), nv.i32(row), nv.i64(start),
+                    nv.stream_ptr())
+    return left
+
+
+def decode_pick(logits, token, out, cursor, pos, positions, rings: list[tuple], scratch):
+    """Greedy choice and the move to the next token in one launch: token [B, 1] and column ``cursor`` of out [B, columns] get the
+    arg-max of each row of logits; cursor, pos, positions [B, 1] and the rings' (capacity, slot, kv_len) advance.  ``scratch``:
+    int64 [8 B + 1], zero before the first call, this caller's own."""
+    import ctypes
+    B, V = logits.shape
+    n = len(rings)
+    caps = (ctypes.c_longlong * 4)(*[c for c, _, _ in rings])
+    slots = (ctypes.c_void_p * 4)(*[s.data_ptr() for _, s, _ in rings])
+    lens = (ctypes.c_void_p * 4)(*[k.data_ptr() for _, _, k in rings])
+    nv.call("ttcd_decode_pick", nv.ptr(logits), nv.i64(logits.stride(0)), nv.i32(B), nv.i32(V), nv.ptr(token), nv.ptr(out),
+            nv.i64(out.stride(0)), nv.i32(out.shape[1]), nv.ptr(cursor), nv.ptr(pos), nv.ptr(positions), slots, lens, caps, nv.i32(n),
+            nv.ptr(scratch[1:]), nv.ptr(scratch), nv.stream_ptr())
+
+
 class GradSlab:
     """Meeting point for the gradients of the column slices of one fused projection (q|k|v): the backward
     kernels of the consumers write straight into one [rows, n_total] buffer, so the projection's backward
