@@ -6,8 +6,8 @@
 // ([N, K] or [K, N]).  That covers y = x W^T, dx = dy W, dW = dy^T x and their batched forms
 // without any transposition pass.
 //
-// One CTA per SM; tile 128 x BN x 64.  Warp 0 streams operand tiles with TMA (128-byte swizzle,
-// no multicast) through a 4-stage mbarrier ring, one thread of warp 1 issues tcgen05.mma into a
+// One CTA per SM; tile 128 x BN x 64 (BN 256, 128 or 64: see gemm_tile_n).  Warp 0 streams operand tiles with TMA (128-byte swizzle,
+// no multicast) through a mbarrier ring of 4 to 8 stages, one thread of warp 1 issues tcgen05.mma into a
 // double-buffered TMEM accumulator (2 x BN fp32 columns), warps 2-5 drain the other accumulator
 // with tcgen05.ld and write C, so the epilogue of tile i overlaps the main loop of tile i+1.
 // Replaces the reference's cuBLAS calls behind nn.Linear / torch.matmul
@@ -66,7 +66,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  constexpr uint32_t TMEM_COLS = 2 * BN;  // 256 or 512: power of two
+  constexpr uint32_t TMEM_COLS = 2 * BN;  // 128, 256 or 512: power of two
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -380,6 +380,23 @@ static int dispatch_major(const CUtensorMap& ta, const CUtensorMap& tb, const CU
   return dispatch_out<BN, STAGES, true, true>(ta, tb, tc, c, cin, p, out_fp32, stream);
 }
 
+// Width of a tile.  256 columns are the cheapest per flop (operand traffic), but a grid of tiles runs in whole waves of the SMs,
+// and where the last wave is nearly empty, or the only one has few tiles, narrower tiles finish earlier.  Time of a launch in
+// units of one wave of 256-wide tiles, fitted to 230 shapes of the shipped models (M 300 .. 131072, N 1024 .. 128256, K 1024 ..
+// 128256): waves at 256; 0.56 waves + 0.07 at 128; 0.42 waves + 0.12 at 64.  us at 256 | 128 | 64:
+//   one wave, few tiles: 300 x 1024 x 3072: 25.6 | 19.5 | 17.4; 448 x 2048 x 8192: 57 | 38 | 31; 2048 x 1024 x 32000: 178 | 118 | 168
+//   a second wave that is nearly empty: 6002 x 1024 x 3072: 46 | 42 | 56; 6144 x 1024 x 22646: 259 | 228 | 345
+//   full waves: 3832 x 1024 x 3072: 28 | 32 | 41; 32768 x 1024 x 2816: 131 | 147 | 207
+static int gemm_tile_n(int64_t M, int64_t N, int64_t batch) {
+  const int64_t rows = (M + GEMM_BM - 1) / GEMM_BM * batch, sms = sm_count();
+  auto waves = [&](int bn) { return static_cast<double>((rows * ((N + bn - 1) / bn) + sms - 1) / sms); };
+  int best = 128;
+  double cost = 0.56 * waves(128) + 0.07;
+  const double narrow = 0.42 * waves(64) + 0.12;
+  if (narrow < cost) { best = 64; cost = narrow; }
+  return N >= 256 && waves(256) <= 1.06 * cost ? 256 : best;      // (5003 x 2048 x 2048, 3 | 2.87: 44 for 46 alone, no gain between others)
+}
+
 }  // namespace ttcd
 
 TTCD_DEFINE_STATUS_READER(gemm)
@@ -402,7 +419,8 @@ static int gemm_bf16_impl(const void* a, const void* b, void* c, const void* c_i
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   // every TMA box must fit inside its tensor: the caller pads tiny problems up to these minima
   if (M < GEMM_BM || N < 128 || K < GEMM_BK) return TTCD_ERR_ARG;
-  const int BN = N >= 256 ? 256 : 128;
+  // (the pairs of lse_part are per 256 or 128 columns, as the caller sized it)
+  const int BN = lse_part != nullptr ? (N >= 256 ? 256 : 128) : gemm_tile_n(M, N, batch);
   CUtensorMap ta, tb;
   int rc;
   const int a_bcast = (batch > 1 && stride_a == 0) ? 1 : 0;
@@ -433,6 +451,7 @@ static int gemm_bf16_impl(const void* a, const void* b, void* c, const void* c_i
                 : make_tmap_bf16_3d(&tc, c, N, M, batch, ldc, stride_c, 64, 32);
   if (rc != TTCD_OK) return rc;
   if (BN == 256) return dispatch_major<256, 4>(ta, tb, tc, c, c_in, p, a_mn, b_mn, out_fp32, stream);
+  if (BN == 64) return dispatch_major<64, 8>(ta, tb, tc, c, c_in, p, a_mn, b_mn, out_fp32, stream);
   return dispatch_major<128, 6>(ta, tb, tc, c, c_in, p, a_mn, b_mn, out_fp32, stream);
 }
 

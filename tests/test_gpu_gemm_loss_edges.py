@@ -91,3 +91,24 @@ def test_loss_gradient_is_linear_in_what_arrives(linear):
     assert abs(float(by_weight.double() - want)) <= 2.0 ** -8 * float(want.abs()) + 2.0 ** -20 * float(one.double().abs().sum())
     (several,) = torch.autograd.grad(loss(), x, torch.tensor([1.0, 4.0], device=DEV), is_grads_batched=True)
     assert torch.equal(several[0], one) and torch.equal(several[1], 4 * one)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,M,N,K", [
+    (1, 128, 128, 64), (1, 300, 1024, 3072), (1, 448, 2056, 520), (1, 1024, 1032, 2328), (1, 130, 19000, 72),          # 64 or 128 wide
+    (1, 2048, 1024, 200), (1, 6002, 1024, 136), (3, 1030, 1160, 264), (1, 129, 136, 1000),                             # 128 wide
+    (1, 3832, 1024, 200), (2, 1100, 2050 // 8 * 8, 128)])                                                              # 256 wide
+@pytest.mark.parametrize("a_t,b_t,out", [(False, True, "bf16"), (False, False, "bf16"), (True, False, "fp32"), (True, True, "bf16+c")])
+def test_gemm_of_every_tile_width_against_float64(batch, M, N, K, a_t, b_t, out):
+    """Shapes on both sides of the rule for the tile's width, with remainders of rows, columns and K, every operand order."""
+    torch.manual_seed(M + N)
+    M, N = M // 8 * 8 if a_t else M, N // 8 * 8
+    mk = lambda r, c, t: (torch.randn(batch, c, r, device=DEV).bfloat16().transpose(1, 2) if t                         # noqa: E731
+                          else torch.randn(batch, r, c, device=DEV).bfloat16())
+    a, b = mk(M, K, a_t), mk(K, N, b_t)
+    c = torch.randn(batch, M, N, device=DEV).bfloat16() if out == "bf16+c" else None
+    got = cuda.gemm(a, b, out_dtype=torch.float32 if out == "fp32" else torch.bfloat16, c_in=c, beta=0.0 if c is None else 1.0).double()
+    want = a.double() @ b.double() + (0.0 if c is None else c.double())
+    # K / 16 accumulation steps, each cut within an ulp or two (2^-23, 2^-22) of a partial sum of up to 4 sqrt(K); then one rounding to bf16
+    bound = max(K, 16) / 16 * 2.0 ** -22 * 4 * K ** 0.5 + (0.0 if out == "fp32" else want.abs() * 2.0 ** -8)
+    assert got.shape == want.shape and ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())
