@@ -12,13 +12,16 @@
 // with tcgen05.ld and write C, so the epilogue of tile i overlaps the main loop of tile i+1.
 // Replaces the reference's cuBLAS calls behind nn.Linear / torch.matmul
 // (custom_models/ipttcd/modeling_ipttcdv9_lowcopy_scanfuse.py:113-200).
-#include "common.cuh"
+#include "gemm.cuh"
 
 namespace ttcd {
 
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
-constexpr int GEMM_THREADS = 192;
+// warps that drain an accumulator: four, or with SwiGLU one per 32 lanes and 32 columns of C (four of them take 22 k cycles for what the
+// MMAs of a 1024-long product make in 8 k: exponential, division and a dependent chain per value)
+__host__ __device__ constexpr int gemm_epi_warps(int bn, bool swiglu) { return swiglu ? bn / 16 : 4; }
+__host__ __device__ constexpr int gemm_threads(int bn, bool swiglu) { return 64 + 32 * gemm_epi_warps(bn, swiglu); }
 
 struct GemmParams {
   int64_t M, N, K, batch;
@@ -31,7 +34,10 @@ struct GemmParams {
   int m_fastest;             // raster order inside a batch entry: consecutive tiles walk M (the B panel is the big one)
   float2* lse_part;          // optional [batch*M][tiles_n]: per row and column tile (max, sum of exp(x - max)) of the
                              // bf16-rounded outputs, for a log-sum-exp over the row without another pass (bf16 out only)
+  int64_t seg1, seg2;        // first column of the second and third matrix that B's rows come from (past the last: there is none)
+  int round_first;           // the product is rounded to bf16 before Cin is added
 };
+struct GemmBMaps { CUtensorMap m[3]; };
 
 template <int BN, int STAGES>
 struct GemmSmem {
@@ -46,12 +52,16 @@ struct GemmSmem {
   static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 4) * 8 + 16;
 };
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool HAS_CIN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+// SWIGLU: B's rows are half gate, half up; a tile of BN rows of B makes BN / 2 columns of C.  The product never reaches memory:
+// gate | up of 65536 x 3072 (K 1024) and the pass that combined them took 600 + 250 us, with 1.6 GB between them; 585 us so.
+template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool HAS_CIN, bool SWIGLU = false>
+__global__ void __launch_bounds__(gemm_threads(BN, SWIGLU), 1)
+gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ GemmBMaps tma_bs,
             const __grid_constant__ CUtensorMap tma_c, OutT* __restrict__ C, const OutT* __restrict__ Cin,
             const GemmParams p) {
   using S = GemmSmem<BN, STAGES>;
+  constexpr int CN = SWIGLU ? BN / 2 : BN;         // columns of C per tile
+  static_assert(!SWIGLU || (!A_MN && !B_MN && !HAS_CIN && sizeof(OutT) == 2), "inference product");
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: required by the 128-byte swizzle pattern shared by TMA and UMMA.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -75,12 +85,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 4);  // one arrival per epilogue warp
+      mbar_init(tempty_bar(b), gemm_epi_warps(BN, SWIGLU));  // one arrival per epilogue warp
     }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tma_a);
-    tma_prefetch_desc(&tma_b);
+    tma_prefetch_desc(&tma_bs.m[0]);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
@@ -105,7 +115,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         const int b = static_cast<int>(tile / tiles_per_batch);
         const int64_t r = tile % tiles_per_batch;
         const int m0 = static_cast<int>(p.m_fastest ? r % p.tiles_m : r / p.tiles_n) * GEMM_BM;
-        const int n0 = static_cast<int>(p.m_fastest ? r / p.tiles_m : r % p.tiles_n) * BN;
+        int n0 = static_cast<int>(p.m_fastest ? r / p.tiles_m : r % p.tiles_n) * CN;
+        const int seg = SWIGLU ? 0 : (n0 >= p.seg1) + (n0 >= p.seg2);      // (a tile lies in one of them)
+        const CUtensorMap* tma_b = &tma_bs.m[seg];
+        if (seg > 0) n0 -= static_cast<int>(seg == 1 ? p.seg1 : p.seg2);
         const int za = p.a_bcast ? 0 : b, zb = p.b_bcast ? 0 : b;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, 101)) { ok = false; break; }
@@ -120,12 +133,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             for (int h = 0; h < GEMM_BM / 64; ++h)
               tma_load_3d(sa + h * (GEMM_BK * 128), &tma_a, full_bar(stage), m0 + h * 64, k0, za);
           }
-          if (!B_MN) {
-            tma_load_3d(sb, &tma_b, full_bar(stage), k0, n0, zb);
+          if constexpr (SWIGLU) {
+            tma_load_3d(sb, &tma_bs.m[0], full_bar(stage), k0, n0, zb);
+            tma_load_3d(sb + CN * 128, &tma_bs.m[1], full_bar(stage), k0, n0, zb);
+          } else if (!B_MN) {
+            tma_load_3d(sb, tma_b, full_bar(stage), k0, n0, zb);
           } else {
 #pragma unroll
             for (int h = 0; h < BN / 64; ++h)
-              tma_load_3d(sb + h * (GEMM_BK * 128), &tma_b, full_bar(stage), n0 + h * 64, k0, zb);
+              tma_load_3d(sb + h * (GEMM_BK * 128), tma_b, full_bar(stage), n0 + h * 64, k0, zb);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -172,7 +188,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..)
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t acc_phase[2] = {0, 0};
     int acc = 0;
@@ -181,7 +197,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       const int b = static_cast<int>(tile / tiles_per_batch);
       const int64_t r = tile % tiles_per_batch;
       const int64_t m0 = (p.m_fastest ? r % p.tiles_m : r / p.tiles_n) * GEMM_BM;
-      const int64_t n0 = (p.m_fastest ? r / p.tiles_m : r % p.tiles_n) * BN;
+      const int64_t n0 = (p.m_fastest ? r / p.tiles_m : r % p.tiles_n) * CN;
       if (!mbar_wait(tfull_bar(acc), acc_phase[acc], abort_flag, 104)) { ok = false; break; }
       tc_fence_after_sync();
       const int64_t row = m0 + quarter * 32 + lane;
@@ -191,7 +207,48 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       OutT* crow = C + b * p.stride_c + row * p.ldc;
       const OutT* cin_row = HAS_CIN ? (Cin + b * p.stride_c + row * p.ldc) : nullptr;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
-      if constexpr (sizeof(OutT) == 2) {
+      if constexpr (SWIGLU) {
+        // this warp's 32 columns; it and its neighbour fill one box of 64
+        const int part = (warp - 2) >> 2, pair = part >> 1, c = part * 32;
+        uint8_t* buf = smem + S::EPI_OFFSET + quarter * 8192 + pair * 4096;
+        auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter * 2 + pair) : "memory"); };
+        uint32_t vg[32], vu[32];
+        tmem_ld32(t_row + c, vg);
+        tmem_ld32(t_row + CN + c, vu);
+        if ((part & 1) == 0 && lane == 0) tma_store_wait_read0();     // the last tile's store has released the buffer
+        tmem_ld_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tempty_bar(acc));      // the accumulator is in registers
+        meet();
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) {
+          float o[8];
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            const float2 gate = unpack_bf16(pack_bf16(__uint_as_float(vg[j + e]) * rs, __uint_as_float(vg[j + e + 1]) * rs));
+            const float2 up = unpack_bf16(pack_bf16(__uint_as_float(vu[j + e]) * rs, __uint_as_float(vu[j + e + 1]) * rs));
+            o[e] = gate.x / (1.f + __expf(-gate.x)) * up.x;
+            o[e + 1] = gate.y / (1.f + __expf(-gate.y)) * up.y;
+          }
+          uint4 w;
+          w.x = pack_bf16(o[0], o[1]);
+          w.y = pack_bf16(o[2], o[3]);
+          w.z = pack_bf16(o[4], o[5]);
+          w.w = pack_bf16(o[6], o[7]);
+          *reinterpret_cast<uint4*>(buf + sw128_offset(lane, (c & 32) / 8 + (j >> 3))) = w;
+        }
+        fence_proxy_async_smem();
+        meet();
+        const int64_t col = n0 + pair * 64;
+        if ((part & 1) == 0 && lane == 0 && col < p.N) {
+          tma_store_3d(&tma_c, smem_u32(buf), static_cast<int>(col), static_cast<int>(m0 + quarter * 32), b);
+          tma_store_commit();
+        }
+        acc_phase[acc] ^= 1u;
+        acc ^= 1;
+        continue;
+      } else if constexpr (sizeof(OutT) == 2) {
         // bf16 output: TMEM -> registers -> swizzled shared memory -> TMA store of a 32-row x 64-column box
         // (full 128-byte lines, clipped at the matrix edges by the tensor map); two staging buffers per warp.
         uint8_t* stage = smem + S::EPI_OFFSET + quarter * 8192;
@@ -214,6 +271,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 #pragma unroll
             for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(j < 32 ? v0[(j & 31) + e] : v1[(j & 31) + e]) * rs;
             if constexpr (HAS_CIN) {
+              if (p.round_first) {
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {
+                  const float2 t = unpack_bf16(pack_bf16(f[e], f[e + 1]));
+                  f[e] = t.x; f[e + 1] = t.y;
+                }
+              }
               if (row_ok && col + j + 8 <= p.N) {
                 const uint4 cv = *reinterpret_cast<const uint4*>(cin_row + col + j);
                 const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
@@ -342,11 +406,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
   }
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool HAS_CIN>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* c, const void* cin,
+template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool HAS_CIN, bool SWIGLU = false>
+static int launch_gemm(const CUtensorMap& ta, const GemmBMaps& tb, const CUtensorMap& tc, void* c, const void* cin,
                        const GemmParams& p, cudaStream_t stream) {
   using S = GemmSmem<BN, STAGES>;
-  auto kern = gemm_kernel<BN, STAGES, A_MN, B_MN, OutT, HAS_CIN>;
+  auto kern = gemm_kernel<BN, STAGES, A_MN, B_MN, OutT, HAS_CIN, SWIGLU>;
   constexpr int smem_bytes = S::TOTAL + 1024;
   static bool configured = false;  // per instantiation; attribute is per function, device-independent here
   if (!configured) {
@@ -355,12 +419,12 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   }
   const int64_t total = p.tiles_m * p.tiles_n * p.batch;
   const int grid = static_cast<int>(total < sm_count() ? total : sm_count());
-  kern<<<grid, GEMM_THREADS, smem_bytes, stream>>>(ta, tb, tc, static_cast<OutT*>(c), static_cast<const OutT*>(cin), p);
+  kern<<<grid, gemm_threads(BN, SWIGLU), smem_bytes, stream>>>(ta, tb, tc, static_cast<OutT*>(c), static_cast<const OutT*>(cin), p);
   return static_cast<int>(cudaGetLastError());
 }
 
 template <int BN, int STAGES, bool A_MN, bool B_MN>
-static int dispatch_out(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* c, const void* cin,
+static int dispatch_out(const CUtensorMap& ta, const GemmBMaps& tb, const CUtensorMap& tc, void* c, const void* cin,
                         const GemmParams& p, int out_fp32, cudaStream_t stream) {
   const bool has_cin = cin != nullptr && p.beta != 0.f && !p.accumulate;
   if (out_fp32) {
@@ -372,7 +436,7 @@ static int dispatch_out(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
 }
 
 template <int BN, int STAGES>
-static int dispatch_major(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, void* c, const void* cin,
+static int dispatch_major(const CUtensorMap& ta, const GemmBMaps& tb, const CUtensorMap& tc, void* c, const void* cin,
                           const GemmParams& p, int a_mn, int b_mn, int out_fp32, cudaStream_t stream) {
   if (!a_mn && !b_mn) return dispatch_out<BN, STAGES, false, false>(ta, tb, tc, c, cin, p, out_fp32, stream);
   if (!a_mn && b_mn) return dispatch_out<BN, STAGES, false, true>(ta, tb, tc, c, cin, p, out_fp32, stream);
@@ -404,55 +468,78 @@ TTCD_DEFINE_STATUS_READER(gemm)
 // a: [batch][M][K] (a_mn = 0, row stride lda) or [batch][K][M] (a_mn = 1).  b likewise with N.
 // c / c_in: [batch][M][N], row stride ldc, bf16 or fp32 (out_fp32).  Strides in elements.
 // c_in may alias c.  row_scale: optional bf16 [batch*M].
-static int gemm_bf16_impl(const void* a, const void* b, void* c, const void* c_in, const void* row_scale,
-                         long long M, long long N, long long K, long long batch, long long lda,
-                         long long ldb, long long ldc, long long stride_a, long long stride_b,
-                         long long stride_c, int a_mn, int b_mn, int out_fp32, float alpha, float beta,
-                         float* lse_part, void* stream_ptr) {
-  using namespace ttcd;
+int ttcd::gemm_run(const GemmCall& g, cudaStream_t stream) {
+  const int64_t M = g.M, N = g.N, K = g.K, batch = g.batch;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return TTCD_ERR_ARG;
-  if (lse_part != nullptr && (out_fp32 || (reinterpret_cast<uintptr_t>(lse_part) & 7u))) return TTCD_ERR_ARG;
-  const int elem_c = out_fp32 ? 4 : 2;
-  if ((reinterpret_cast<uintptr_t>(c) & 15u) || (ldc * elem_c) % 16 != 0 || (stride_c * elem_c) % 16 != 0)
+  if (g.lse_part != nullptr && (g.out_fp32 || (reinterpret_cast<uintptr_t>(g.lse_part) & 7u))) return TTCD_ERR_ARG;
+  const int elem_c = g.out_fp32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(g.c) & 15u) || (g.ldc * elem_c) % 16 != 0 || (g.stride_c * elem_c) % 16 != 0)
     return TTCD_ERR_ARG;
-  if (c_in != nullptr && (reinterpret_cast<uintptr_t>(c_in) & 15u)) return TTCD_ERR_ARG;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
+  if (g.c_in != nullptr && (reinterpret_cast<uintptr_t>(g.c_in) & 15u)) return TTCD_ERR_ARG;
   // every TMA box must fit inside its tensor: the caller pads tiny problems up to these minima
   if (M < GEMM_BM || N < 128 || K < GEMM_BK) return TTCD_ERR_ARG;
-  // (the pairs of lse_part are per 256 or 128 columns, as the caller sized it)
-  const int BN = lse_part != nullptr ? (N >= 256 ? 256 : 128) : gemm_tile_n(M, N, batch);
-  CUtensorMap ta, tb;
+  const bool pieces = g.swiglu || g.n1 != 0;
+  if (pieces && (g.b_mn || batch != 1 || g.lse_part != nullptr || g.b2 == nullptr)) return TTCD_ERR_ARG;
+  if (g.swiglu && (g.a_mn || g.out_fp32 || g.c_in != nullptr || g.n1 != 0)) return TTCD_ERR_ARG;
+  if (g.round_first && (g.out_fp32 || g.c_in == nullptr || g.beta != 1.f)) return TTCD_ERR_ARG;
+  const int64_t n3 = N - g.n1 - g.n2;
+  if (g.n1 != 0 && (g.n1 < 0 || g.n2 <= 0 || n3 < 0 || (n3 > 0 && g.b3 == nullptr))) return TTCD_ERR_ARG;
+  // the rows of B per tile (with SwiGLU gate and up; the pairs of lse_part are per 256 or 128 columns, as the caller sized it)
+  int BN = g.lse_part != nullptr ? (N >= 256 ? 256 : 128) : gemm_tile_n(M, g.swiglu ? 2 * N : N, batch);
+  if (g.swiglu && BN < 128) BN = 128;              // (a box of C is 64 columns wide)
+  if (g.n1 != 0) {                                 // a tile's rows of B come from one matrix, and its box fits in it
+    int64_t least = g.n1 < g.n2 ? g.n1 : g.n2;
+    if (n3 > 0 && n3 < least) least = n3;
+    while (BN > 64 && (g.n1 % BN != 0 || (n3 > 0 && g.n2 % BN != 0) || least < BN)) BN /= 2;
+    if (g.n1 % BN != 0 || (n3 > 0 && g.n2 % BN != 0) || least < BN) return TTCD_ERR_ARG;
+  }
+  CUtensorMap ta;
+  GemmBMaps tb;
   int rc;
-  const int a_bcast = (batch > 1 && stride_a == 0) ? 1 : 0;
-  const int b_bcast = (batch > 1 && stride_b == 0) ? 1 : 0;
-  const long long batch_a = a_bcast ? 1 : batch, batch_b = b_bcast ? 1 : batch;
-  if (!a_mn) rc = make_tmap_bf16_3d(&ta, a, K, M, batch_a, lda, stride_a, 64, GEMM_BM);
-  else       rc = make_tmap_bf16_3d(&ta, a, M, K, batch_a, lda, stride_a, 64, GEMM_BK);
+  const int a_bcast = (batch > 1 && g.stride_a == 0) ? 1 : 0;
+  const int b_bcast = (batch > 1 && g.stride_b == 0) ? 1 : 0;
+  const int64_t batch_a = a_bcast ? 1 : batch, batch_b = b_bcast ? 1 : batch;
+  if (!g.a_mn) rc = make_tmap_bf16_3d(&ta, g.a, K, M, batch_a, g.lda, g.stride_a, 64, GEMM_BM);
+  else         rc = make_tmap_bf16_3d(&ta, g.a, M, K, batch_a, g.lda, g.stride_a, 64, GEMM_BK);
   if (rc != TTCD_OK) return rc;
-  if (!b_mn) rc = make_tmap_bf16_3d(&tb, b, K, N, batch_b, ldb, stride_b, 64, BN);
-  else       rc = make_tmap_bf16_3d(&tb, b, N, K, batch_b, ldb, stride_b, 64, GEMM_BK);
+  if (g.b_mn) rc = make_tmap_bf16_3d(&tb.m[0], g.b, N, K, batch_b, g.ldb, g.stride_b, 64, GEMM_BK);
+  else        rc = make_tmap_bf16_3d(&tb.m[0], g.b, K, g.n1 != 0 ? g.n1 : N, batch_b, g.ldb, g.stride_b, 64, g.swiglu ? BN / 2 : BN);
   if (rc != TTCD_OK) return rc;
+  tb.m[1] = tb.m[2] = tb.m[0];
+  if (pieces) {
+    rc = make_tmap_bf16_3d(&tb.m[1], g.b2, K, g.swiglu ? N : g.n2, 1, g.ldb, 0, 64, g.swiglu ? BN / 2 : BN);
+    if (rc == TTCD_OK && g.n1 != 0 && n3 > 0) rc = make_tmap_bf16_3d(&tb.m[2], g.b3, K, n3, 1, g.ldb, 0, 64, BN);
+    if (rc != TTCD_OK) return rc;
+  }
+  const int CN = g.swiglu ? BN / 2 : BN;
   GemmParams p;
   p.M = M; p.N = N; p.K = K; p.batch = batch;
-  p.ldc = ldc; p.stride_c = stride_c;
+  p.ldc = g.ldc; p.stride_c = g.stride_c;
   p.tiles_m = (M + GEMM_BM - 1) / GEMM_BM;
-  p.tiles_n = (N + BN - 1) / BN;
-  p.alpha = alpha; p.beta = beta;
-  p.row_scale = static_cast<const bf16*>(row_scale);
+  p.tiles_n = (N + CN - 1) / CN;
+  p.alpha = g.alpha; p.beta = g.beta;
+  p.row_scale = static_cast<const bf16*>(g.row_scale);
   p.a_bcast = a_bcast; p.b_bcast = b_bcast;
+  p.seg1 = g.n1 != 0 ? g.n1 : INT64_MAX;
+  p.seg2 = g.n1 != 0 && n3 > 0 ? g.n1 + g.n2 : INT64_MAX;
+  p.round_first = g.round_first;
   // the operand panel that is re-streamed once per step of the outer tile loop should be the smaller one (it then
   // lives in the 126 MB L2): walk M fastest when the B panel (N x K) is the larger
-  p.m_fastest = N > M ? 1 : 0;
-  p.lse_part = reinterpret_cast<float2*>(lse_part);
+  p.m_fastest = (g.swiglu ? 2 * N : N) > M ? 1 : 0;
+  p.lse_part = reinterpret_cast<float2*>(g.lse_part);
   // adding to C where it stands needs no read of C; not when batch entries share C (their order would not be fixed)
-  p.accumulate = out_fp32 && c_in == c && beta == 1.f && (batch == 1 || stride_c != 0) ? 1 : 0;
+  p.accumulate = g.out_fp32 && g.c_in == g.c && g.beta == 1.f && (batch == 1 || g.stride_c != 0) ? 1 : 0;
   CUtensorMap tc;
-  rc = out_fp32 ? make_tmap_f32_3d(&tc, c, N, M, batch, ldc, stride_c, 32, 32)
-                : make_tmap_bf16_3d(&tc, c, N, M, batch, ldc, stride_c, 64, 32);
+  rc = g.out_fp32 ? make_tmap_f32_3d(&tc, g.c, N, M, batch, g.ldc, g.stride_c, 32, 32)
+                  : make_tmap_bf16_3d(&tc, g.c, N, M, batch, g.ldc, g.stride_c, 64, 32);
   if (rc != TTCD_OK) return rc;
-  if (BN == 256) return dispatch_major<256, 4>(ta, tb, tc, c, c_in, p, a_mn, b_mn, out_fp32, stream);
-  if (BN == 64) return dispatch_major<64, 8>(ta, tb, tc, c, c_in, p, a_mn, b_mn, out_fp32, stream);
-  return dispatch_major<128, 6>(ta, tb, tc, c, c_in, p, a_mn, b_mn, out_fp32, stream);
+  if (g.swiglu) {
+    if (BN == 256) return launch_gemm<256, 4, false, false, bf16, false, true>(ta, tb, tc, g.c, nullptr, p, stream);
+    return launch_gemm<128, 6, false, false, bf16, false, true>(ta, tb, tc, g.c, nullptr, p, stream);
+  }
+  if (BN == 256) return dispatch_major<256, 4>(ta, tb, tc, g.c, g.c_in, p, g.a_mn, g.b_mn, g.out_fp32, stream);
+  if (BN == 64) return dispatch_major<64, 8>(ta, tb, tc, g.c, g.c_in, p, g.a_mn, g.b_mn, g.out_fp32, stream);
+  return dispatch_major<128, 6>(ta, tb, tc, g.c, g.c_in, p, g.a_mn, g.b_mn, g.out_fp32, stream);
 }
 
 TTCD_EXPORT int ttcd_gemm_bf16(const void* a, const void* b, void* c, const void* c_in, const void* row_scale,
@@ -460,8 +547,12 @@ TTCD_EXPORT int ttcd_gemm_bf16(const void* a, const void* b, void* c, const void
                                long long ldb, long long ldc, long long stride_a, long long stride_b,
                                long long stride_c, int a_mn, int b_mn, int out_fp32, float alpha, float beta,
                                void* stream_ptr) {
-  return gemm_bf16_impl(a, b, c, c_in, row_scale, M, N, K, batch, lda, ldb, ldc, stride_a, stride_b, stride_c, a_mn, b_mn,
-                        out_fp32, alpha, beta, nullptr, stream_ptr);
+  ttcd::GemmCall g;
+  g.a = a; g.b = b; g.c = c; g.c_in = c_in; g.row_scale = row_scale;
+  g.M = M; g.N = N; g.K = K; g.batch = batch; g.lda = lda; g.ldb = ldb; g.ldc = ldc;
+  g.stride_a = stride_a; g.stride_b = stride_b; g.stride_c = stride_c;
+  g.a_mn = a_mn; g.b_mn = b_mn; g.out_fp32 = out_fp32; g.alpha = alpha; g.beta = beta;
+  return ttcd::gemm_run(g, static_cast<cudaStream_t>(stream_ptr));
 }
 
 // Same GEMM (bf16 output) that also leaves, per output row and column tile, the pair (max, sum of exp(x - max)) of the
@@ -472,6 +563,19 @@ TTCD_EXPORT int ttcd_gemm_bf16_lse(const void* a, const void* b, void* c, long l
                                    long long lda, long long ldb, long long ldc, int a_mn, int b_mn, float alpha,
                                    float* lse_part, void* stream_ptr) {
   if (lse_part == nullptr) return TTCD_ERR_ARG;
-  return gemm_bf16_impl(a, b, c, nullptr, nullptr, M, N, K, 1, lda, ldb, ldc, 0, 0, M * ldc, a_mn, b_mn, 0, alpha, 0.f,
-                        lse_part, stream_ptr);
+  ttcd::GemmCall g;
+  g.a = a; g.b = b; g.c = c; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.stride_c = M * ldc;
+  g.a_mn = a_mn; g.b_mn = b_mn; g.alpha = alpha; g.lse_part = lse_part;
+  return ttcd::gemm_run(g, static_cast<cudaStream_t>(stream_ptr));
+}
+
+// Products of inference (K-major operands, bf16 [M, K] times rows of B): up to three matrices side by side (b [n1, K], b2 [n2, K],
+// b3 the rest; n1 = 0: b alone), res (may be null, [M, N] like c) added to the rounded product, swiglu of b (gate) and b2 (up).
+TTCD_EXPORT int ttcd_gemm_pieces(const void* a, const void* b, const void* b2, const void* b3, void* c, const void* res, long long M,
+                                 long long N, long long K, long long lda, long long ldb, long long ldc, long long n1, long long n2,
+                                 int swiglu, void* stream_ptr) {
+  ttcd::GemmCall g;
+  g.a = a; g.b = b; g.b2 = b2; g.b3 = b3; g.c = c; g.c_in = res; g.beta = res != nullptr ? 1.f : 0.f; g.round_first = res != nullptr;
+  g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb; g.ldc = ldc; g.stride_c = M * ldc; g.n1 = n1; g.n2 = n2; g.swiglu = swiglu;
+  return ttcd::gemm_run(g, static_cast<cudaStream_t>(stream_ptr));
 }
