@@ -109,3 +109,28 @@ def test_a_tensor_parallel_state_runs_the_modules(monkeypatch):
     model = _model()
     monkeypatch.setattr(layers, "_tp_state", lambda: SimpleNamespace(world=2))
     assert _fused(model) is None
+
+
+def _plain(model):
+    """Which blocks a prompt would run natively (the rule itself needs no GPU)."""
+    from ttcd_b200.models.prefill import PlainBlocks
+    runner = PlainBlocks(torch.zeros(1, 300, 128, dtype=torch.bfloat16), None)
+    return [runner._tensors(block) is not None for block in model.model.layers]
+
+
+def test_the_stock_blocks_run_natively_but_for_the_fast_weight_one():
+    assert _plain(_model()) == [True, False]
+
+
+@pytest.mark.parametrize("change", ["mlp_forward_replaced", "mlp_features_replaced", "hook_on_a_block", "computed_weight"])
+def test_a_changed_block_runs_its_modules_over_a_prompt(change):
+    model = _model()
+    CHANGES[change](model)
+    assert _plain(model) == [False, False]
+
+
+def test_a_method_replaced_on_a_class_is_run_over_a_prompt(monkeypatch):
+    model = _model()
+    assert _plain(model) == [True, False]
+    monkeypatch.setattr(GatedMLP, "features", lambda self, x: x)
+    assert _plain(model) == [False, False]

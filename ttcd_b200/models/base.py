@@ -173,9 +173,16 @@ class DecoderModel(DecoderPreTrainedModel):
         hidden_states = inputs_embeds
         all_hidden = () if output_hidden_states else None
         nvtx = _NVTX and hidden_states.is_cuda
+        plain = None
+        if hidden_states.is_cuda and not self.training and not output_hidden_states and not nvtx:
+            from .prefill import plain_blocks
+            plain = plain_blocks(hidden_states, attention_mask, past_key_values, kwargs)
         for i, layer in enumerate(self.layers):
             if output_hidden_states:
                 all_hidden += (hidden_states,)
+            if plain is not None and (done := plain(layer, hidden_states)) is not None:
+                hidden_states = done
+                continue
             if nvtx:
                 torch.cuda.nvtx.range_push(f"layer{i}")
             if self.gradient_checkpointing and self.training and self._checkpoint_layer(layer):

@@ -1,0 +1,140 @@
+"""A prompt through the plain decoder blocks of a model (inference) with one native call per block.
+
+A block run module by module takes ~370 us of Python for eleven launches; a chat-sized prompt is bound by that.  Where a block
+is the stock one, with nothing hooked or replaced, gradients off and no padding, its launches are issued from C++
+(``ttcd_block_prefill``), weights that do not lie side by side need not be put there, SwiGLU and the residual sums ride on the
+products that feed them.  Fast-weight blocks that run their dual path, and everything else, go through the modules.
+
+Mirrors the block order of the reference (custom_models/ipttcd/modeling_ipttcdv9.py:794-850,
+fla/models/transformer/modeling_transformer.py:43-122); the roundings are the module path's.
+"""
+from __future__ import annotations
+
+import ctypes
+
+import torch
+
+from .. import _native as nv
+from . import layers
+from .decoding import _STEP_METHODS, _as_defined
+from .layers import Attention, GatedMLP, RMSNorm, WindowKVCache
+
+_BF16 = torch.bfloat16
+
+
+_METHODS = ("forward", "project_qkv", "finish", "features", "__call__")      # what the native call computes on behalf of
+_stock: dict | None = None
+
+
+def _methods(cls) -> tuple:
+    return tuple(getattr(cls, n, None) for n in _METHODS)
+
+
+def _stock_classes() -> dict:
+    """The classes that the native call stands for, with their methods as this package defines them."""
+    global _stock
+    if _stock is None:
+        from .modeling_ipttcdv9 import IPTTCDBlock, IPTTCDMLP
+        from .modeling_transformer import TransformerBlock
+        _stock = {cls: _methods(cls) for cls in (IPTTCDBlock, TransformerBlock, IPTTCDMLP, GatedMLP, Attention, RMSNorm, torch.nn.Linear)}
+    return _stock
+
+
+class PlainBlocks:
+    """Runs the blocks it can of one forward pass; made by ``plain_blocks``."""
+
+    def __init__(self, x: torch.Tensor, past):
+        self.past, self.device = past, x.device
+        self.B, self.T, self.hidden = x.shape
+        self.scratch: dict = {}
+        # classes that still are what this package made them, methods that a program may have replaced on an instance
+        self.classes = {cls for cls, methods in _stock_classes().items() if _methods(cls) == methods} if _as_defined() else set()
+        self.blocks = {cls for cls in self.classes if cls.__name__.endswith("Block")}
+        self.replaceable = frozenset(_METHODS + _STEP_METHODS)
+
+    def _buffers(self, q_cols: int, inter: int, heads: int):
+        key = (q_cols, inter, heads)
+        got = self.scratch.get(key)
+        if got is None:
+            rows, dev = self.B * self.T, self.device
+            new = lambda cols: torch.empty(rows, cols, dtype=_BF16, device=dev)      # noqa: E731
+            f32 = lambda n: torch.empty(n, dtype=torch.float32, device=dev)          # noqa: E731
+            self.scratch[key] = got = (new(self.hidden), f32(rows), new(q_cols), new(q_cols), f32(heads * rows), new(self.hidden), new(inter))
+        return got
+
+    def _tensors(self, block):
+        """The block's weights in the native call's order, or None where it has to run through its modules.  (Runs per block and
+        pass: plain dictionaries, as a module's attribute lookup costs more than what is asked here.)"""
+        if type(block) not in self.blocks or block.training:
+            return None
+        if getattr(block, "is_ttt_layer", False) and self.T >= block.ttt_chunk:
+            return None
+        parts = block._modules
+        attn, mlp = parts["attn"], parts["mlp"]
+        if type(attn) is not Attention or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128):
+            return None
+        linears = [attn._modules[n] for n in ("q_proj", "k_proj", "v_proj", "o_proj")] + [mlp._modules.get(n) for n in ("gate_proj", "up_proj", "down_proj")]
+        norms = [parts["attn_norm"], parts["mlp_norm"]] + ([attn._modules["q_norm"], attn._modules["k_norm"]] if attn.qk_norm else [])
+        for m in (block, attn, mlp, *linears, *norms):
+            if type(m) not in self.classes or m._forward_hooks or m._forward_pre_hooks or not self.replaceable.isdisjoint(m.__dict__):
+                return None
+        hidden, inter = attn.hidden_size, mlp.intermediate_size
+        if hidden != self.hidden or min(hidden, inter) < 128 or hidden % 8 or inter % 8 or attn.num_heads % attn.num_kv_heads:
+            return None
+        if any(m._parameters["bias"] is not None for m in linears):
+            return None
+        # a weight that is made from others (a parametrization) is not in _parameters
+        ws = [m._parameters.get("weight") for m in (*norms[:2], *linears, *norms[2:])]
+        device = self.device
+        for w in ws:
+            if type(w) is not torch.nn.Parameter or w.dtype is not _BF16 or w.device != device or not w.is_contiguous() or w.data_ptr() % 16:
+                return None
+        if getattr(ws[2], "_ttcd_gather", None) is not None:
+            return None
+        return ws if attn.qk_norm else ws + [None, None]
+
+    def __call__(self, block, x: torch.Tensor):
+        """The block's output, or None where it has to run through its modules (nothing has been done then)."""
+        ws = self._tensors(block)
+        if ws is None or not x.is_contiguous() or x.data_ptr() % 16:
+            return None
+        attn = block.attn
+        past, B, T = self.past, self.B, self.T
+        H, HK, D = attn.num_heads, attn.num_kv_heads, attn.head_dim
+        if past is not None and past.get_seq_length(attn.layer_idx) > 0:
+            return None
+        cos = sin = None
+        if not attn.use_nope:
+            cos, sin = attn.rotary.tables(max(T, attn.max_position_embeddings or 0), x.device, x.dtype)
+            if not (cos.is_contiguous() and sin.is_contiguous()) or cos.dtype != _BF16 or (cos.data_ptr() | sin.data_ptr()) % 16:
+                return None
+        q_cols, kv_cols = H * D, HK * D
+        normed, rstd, q, o, lse, total, z = self._buffers(q_cols, block.mlp.intermediate_size, H)
+        qkv = torch.empty(B, T, q_cols + 2 * kv_cols, dtype=_BF16, device=x.device)
+        k = torch.empty(B, T, HK, D, dtype=_BF16, device=x.device)
+        out = torch.empty_like(x)
+        at = [t.data_ptr() for t in (x, out, normed, rstd, qkv, q, k, o, lse, total, z)]
+        at += [0 if w is None else w.data_ptr() for w in ws]
+        at += [0, 0] if cos is None else [cos.data_ptr(), sin.data_ptr()]
+        at += [B, T, self.hidden, block.mlp.intermediate_size, H, HK, D, attn.window_size or 0, D // 2 if cos is None else cos.shape[-1]]
+        eps = (ctypes.c_float * 4)(block.attn_norm.eps, block.mlp_norm.eps, attn.q_norm.eps if attn.qk_norm else 0.0, D ** -0.5)
+        nv.call("ttcd_block_prefill", (ctypes.c_longlong * len(at))(*at), eps, nv.stream_ptr())
+        if past is not None:
+            if not attn.qk_norm and cos is None:
+                k = qkv[..., q_cols:q_cols + kv_cols].view(B, T, HK, D)
+            past.update(k, qkv[..., q_cols + kv_cols:].view(B, T, HK, D), attn.layer_idx, attn.window_size)
+        return out
+
+
+def plain_blocks(x: torch.Tensor, attention_mask, past, kwargs) -> PlainBlocks | None:
+    """A runner for this forward pass, or None where all of it goes through the modules."""
+    from ..ops import cuda, selective
+    if attention_mask is not None or torch.is_grad_enabled() or cuda._watched() or any(v is not None for v in kwargs.values()):
+        return None
+    if type(x) is not torch.Tensor or x.dim() != 3 or x.shape[1] < 128 or not nv.use_native(x) or not nv.has("ttcd_block_prefill"):
+        return None
+    if past is not None and type(past) is not WindowKVCache:
+        return None
+    if layers._tp_state() is not None or layers._cp_state() is not None or selective.current() is not None:
+        return None
+    return PlainBlocks(x, past)
