@@ -97,7 +97,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
     tmem_relinquish();
   }
   tc_fence_before_sync();
+  pdl_wait();                                      // (what is above touches nothing that the kernel before may write)
   __syncthreads();
+  pdl_launch_dependents();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -419,7 +421,7 @@ static int launch_gemm(const CUtensorMap& ta, const GemmBMaps& tb, const CUtenso
   }
   const int64_t total = p.tiles_m * p.tiles_n * p.batch;
   const int grid = static_cast<int>(total < sm_count() ? total : sm_count());
-  kern<<<grid, gemm_threads(BN, SWIGLU), smem_bytes, stream>>>(ta, tb, tc, static_cast<OutT*>(c), static_cast<const OutT*>(cin), p);
+  launch_after(total <= sm_count(), kern, grid, gemm_threads(BN, SWIGLU), smem_bytes, stream, ta, tb, tc, static_cast<OutT*>(c), static_cast<const OutT*>(cin), p);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -38,6 +38,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const bf16* __restrict
                                                           const bf16* __restrict__ w, bf16* __restrict__ y,
                                                           bf16* __restrict__ sum_out, float* __restrict__ rstd_out,
                                                           int64_t rows, int D, float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -692,6 +694,8 @@ constexpr int QK_FWD_U = 3, QK_BWD_U = 2;
 
 template <int LPH>
 __global__ void __launch_bounds__(256) qk_norm_rope_fwd_items_kernel(const QKRopeParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int GPW = 32 / LPH;                         // (token, head) items per warp
   const int lane = threadIdx.x & 31, sub = lane % LPH, grp = lane / LPH;
   const int warps = blockDim.x >> 5;
@@ -741,6 +745,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_fwd_items_kernel(const QKRop
 
 template <int LPH>
 __global__ void __launch_bounds__(256) qk_norm_rope_fwd_tokens_kernel(const QKRopeParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int QK_U = QK_FWD_U;
   constexpr int GPW = 32 / LPH;                         // heads per warp-wide load
   const int lane = threadIdx.x & 31, sub = lane % LPH, grp = lane / LPH;
@@ -1100,7 +1106,7 @@ TTCD_EXPORT int ttcd_rmsnorm_fwd(const void* x, const void* res, const void* w, 
   }
   const int chunks = (D + 255) / 256;
 #define LAUNCH(C)                                                                                          \
-  rmsnorm_fwd_kernel<C><<<grid, warps * 32, 0, st>>>(static_cast<const bf16*>(x), static_cast<const bf16*>(res), \
+  launch_after(small_launch(grid), rmsnorm_fwd_kernel<C>, grid, warps * 32, 0, st, static_cast<const bf16*>(x), static_cast<const bf16*>(res), \
                                                      static_cast<const bf16*>(w), static_cast<bf16*>(y),       \
                                                      static_cast<bf16*>(sum_out), rstd, rows, D, eps)
   switch (chunks) {
@@ -1261,11 +1267,11 @@ TTCD_EXPORT int ttcd_qk_norm_rope_fwd(const void* q_in, long long ldq, const voi
     const unsigned vgrid = static_cast<unsigned>(std::min<long long>((items * lph / 32 + 7) / 8 + 1, 148LL * 16));
     const unsigned tgrid = static_cast<unsigned>(std::min<long long>((rows + 7) / 8, 148LL * 16));
     const bool tokens = qk_by_tokens(p, false);
-    if (tokens && lph == 4) qk_norm_rope_fwd_tokens_kernel<4><<<tgrid, 256, 0, st>>>(p);
-    else if (tokens) qk_norm_rope_fwd_tokens_kernel<8><<<tgrid, 256, 0, st>>>(p);
-    else if (lph == 4) qk_norm_rope_fwd_items_kernel<4><<<vgrid, 256, 0, st>>>(p);
-    else if (lph == 8) qk_norm_rope_fwd_items_kernel<8><<<vgrid, 256, 0, st>>>(p);
-    else qk_norm_rope_fwd_items_kernel<16><<<vgrid, 256, 0, st>>>(p);
+    if (tokens && lph == 4) launch_after(small_launch(tgrid), qk_norm_rope_fwd_tokens_kernel<4>, tgrid, 256, 0, st, p);
+    else if (tokens) launch_after(small_launch(tgrid), qk_norm_rope_fwd_tokens_kernel<8>, tgrid, 256, 0, st, p);
+    else if (lph == 4) launch_after(small_launch(vgrid), qk_norm_rope_fwd_items_kernel<4>, vgrid, 256, 0, st, p);
+    else if (lph == 8) launch_after(small_launch(vgrid), qk_norm_rope_fwd_items_kernel<8>, vgrid, 256, 0, st, p);
+    else launch_after(small_launch(vgrid), qk_norm_rope_fwd_items_kernel<16>, vgrid, 256, 0, st, p);
     return static_cast<int>(cudaGetLastError());
   }
   if (half <= 32) qk_norm_rope_fwd_kernel<1><<<grid, 256, 0, st>>>(p);
