@@ -212,6 +212,16 @@ struct DkdvCfg {
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16;
 };
 
+// This CTA's head (of all samples) and tile: heads fastest, up to 16 together, so that the tiles of a head that run at the same time or
+// soon after one another still share its rows in the L2 (128 heads of 4096 tokens in one group: a train step 1 % slower).
+__device__ __forceinline__ void bwd_tile(int heads, int tiles, int& hb, int& tile) {
+  constexpr int GROUP = 16;
+  const int first = static_cast<int>(blockIdx.x) / (GROUP * tiles) * GROUP, id = static_cast<int>(blockIdx.x) - first * tiles;
+  const int here = min(GROUP, heads - first);
+  hb = first + id % here;
+  tile = id / here;
+}
+
 template <int D>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_constant__ CUtensorMap tma_k,
@@ -235,9 +245,10 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_con
   float* vecs = reinterpret_cast<float*>(smem + C::VEC_OFF);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heads fastest, keys ascending: the key blocks that few queries see (the last ones) fill the last wave
-  const int hb = static_cast<int>(blockIdx.x) % p.heads_kv;
-  const int n0 = static_cast<int>(blockIdx.x) / p.heads_kv * 128;
+  // keys ascending: the key blocks that few queries see (the last ones) fill the last wave
+  int hb, tile;
+  bwd_tile(p.heads_kv, (p.Tk + 127) / 128, hb, tile);
+  const int n0 = tile * 128;
   const int kvh = hb % p.HK;
   const int b = hb / p.HK;
   const int G = p.H / p.HK;
@@ -569,9 +580,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tma_q, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // heads fastest, queries descending: the rows that see few keys (the first ones) fill the last wave
-  const int hb = static_cast<int>(blockIdx.x) % p.heads_q;
-  const int m0 = ((p.Tq + 127) / 128 - 1 - static_cast<int>(blockIdx.x) / p.heads_q) * 128;
+  // queries descending: the rows that see few keys (the first ones) fill the last wave
+  int hb, tile;
+  bwd_tile(p.heads_q, (p.Tq + 127) / 128, hb, tile);
+  const int m0 = ((p.Tq + 127) / 128 - 1 - tile) * 128;
   const int h = hb % p.H;
   const int b = hb / p.H;
   const int kvh = h / (p.H / p.HK);
