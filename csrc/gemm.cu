@@ -194,6 +194,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t acc_phase[2] = {0, 0};
     int acc = 0;
+    // stores of this warp so far: the two staging buffers take turns over the tiles too.  (Counted anew in each tile, a tile with an odd
+    // number of stores, 64 columns wide or cut at the edge, left its last store on the buffer that the next tile writes first.)
+    int stores = 0;
     bool ok = true;
     for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       const int b = static_cast<int>(tile / tiles_per_batch);
@@ -254,19 +257,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
         // bf16 output: TMEM -> registers -> swizzled shared memory -> TMA store of a 32-row x 64-column box
         // (full 128-byte lines, clipped at the matrix edges by the tensor map); two staging buffers per warp.
         uint8_t* stage = smem + S::EPI_OFFSET + quarter * 8192;
-        int chunk = 0;
         const bool want_lse = p.lse_part != nullptr;
         float run_m = -INFINITY, run_s = 0.f;
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 64, ++chunk) {
+        for (int c = 0; c < BN; c += 64, ++stores) {
+          const int64_t col = n0 + c;
+          if (col >= p.N) break;                      // nothing of this box is in C: no store, no turn
           uint32_t v0[32], v1[32];
           tmem_ld32(t_row + c, v0);
           tmem_ld32(t_row + c + 32, v1);
           if (lane == 0) tma_store_wait_read1();      // the store issued two chunks ago has released this buffer
           __syncwarp();
           tmem_ld_wait();
-          uint8_t* buf = stage + (chunk & 1) * 4096;
-          const int64_t col = n0 + c;
+          uint8_t* buf = stage + (stores & 1) * 4096;
 #pragma unroll
           for (int j = 0; j < 64; j += 8) {
             float f[8];
@@ -324,7 +327,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0 && col < p.N) {
+          if (lane == 0) {
             tma_store_3d(&tma_c, smem_u32(buf), static_cast<int>(col), static_cast<int>(m0 + quarter * 32), b);
             tma_store_commit();
           }
@@ -335,15 +338,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
         // touch 32 lines per instruction with 16 bytes each.  `accumulate` adds the box to C in the L2 instead of
         // reading C into the epilogue: lm_head weight gradient of 640 rows (128256 x 2048, K 640): 1.36 ms before.
         uint8_t* stage = smem + S::EPI_OFFSET + quarter * 8192;
-        int chunk = 0;
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32, ++chunk) {
+        for (int c = 0; c < BN; c += 32, ++stores) {
+          const int64_t col = n0 + c;
+          if (col >= p.N) break;
           uint32_t v[32];
           tmem_ld32(t_row + c, v);
           if (lane == 0) tma_store_wait_read1();      // the store issued two chunks ago has released this buffer
           __syncwarp();
           tmem_ld_wait();
-          uint8_t* buf = stage + (chunk & 1) * 4096;
+          uint8_t* buf = stage + (stores & 1) * 4096;
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             float4 o;
@@ -355,8 +359,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
           }
           fence_proxy_async_smem();
           __syncwarp();
-          const int64_t col = n0 + c;
-          if (lane == 0 && col < p.N) {
+          if (lane == 0) {
             const int x = static_cast<int>(col), yy = static_cast<int>(m0 + quarter * 32);
             if (p.accumulate) tma_reduce_add_3d(&tma_c, smem_u32(buf), x, yy, b);
             else tma_store_3d(&tma_c, smem_u32(buf), x, yy, b);

@@ -112,3 +112,22 @@ def test_gemm_of_every_tile_width_against_float64(batch, M, N, K, a_t, b_t, out)
     # K / 16 accumulation steps, each cut within an ulp or two (2^-23, 2^-22) of a partial sum of up to 4 sqrt(K); then one rounding to bf16
     bound = max(K, 16) / 16 * 2.0 ** -22 * 4 * K ** 0.5 + (0.0 if out == "fp32" else want.abs() * 2.0 ** -8)
     assert got.shape == want.shape and ((got - want).abs() <= bound).all(), float(((got - want).abs() - bound).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(12000, 192, 64), (12000, 192, 2048), (9600, 136, 72), (20000, 1088, 64), (20000, 1088, 520), (16500, 320, 64),
+                                   (20000, 168, 136), (20000, 1056, 64)])
+@pytest.mark.parametrize("out", ["bf16", "fp32", "bf16+c"])
+def test_gemm_with_several_tiles_per_cta_and_an_odd_number_of_stores_in_one(M, N, K, out):
+    """A tile of one store (64 columns wide, or cut there by the edge) is followed by another tile of the same CTA, whose first store
+    must not go through the staging buffer that the former one is read from.  Short products, so that the stores follow one another."""
+    torch.manual_seed(M + N + K)
+    a, b = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    c = torch.randn(1, M, N, device=DEV).bfloat16() if out == "bf16+c" else None
+    want = a.double() @ b.double().T + (0.0 if c is None else c[0].double())
+    # K / 16 accumulation steps, each cut within an ulp or two (2^-23, 2^-22) of a partial sum of up to 4 sqrt(K); then one rounding to bf16
+    bound = max(K, 16) / 16 * 2.0 ** -22 * 4 * K ** 0.5 + (0.0 if out == "fp32" else want.abs() * 2.0 ** -8)
+    for _ in range(5):
+        got = cuda.gemm(a, b.T, out_dtype=torch.float32 if out == "fp32" else torch.bfloat16, c_in=c, beta=0.0 if c is None else 1.0)
+        err = (got.view(M, N).double() - want).abs() - bound
+        assert (err <= 0).all(), float(err.max())

@@ -39,3 +39,19 @@ def test_swiglu_on_the_product(M, K, N):
             nv.i64(K), nv.i64(K), nv.i64(N), nv.i64(0), nv.i64(0), nv.i32(1), nv.stream_ptr())
     want = cuda.swiglu(cuda.gemm(x, g.transpose(0, 1)).view(M, N), cuda.gemm(x, u.transpose(0, 1)).view(M, N))
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("M,K", [(300, 960), (700, 960), (3000, 64), (9001, 960)])
+def test_weights_in_pieces_that_leave_no_wide_tile(M, K):
+    """960 + 320 + 320 columns: tiles are 64 wide, and from 6 rows of tiles on a CTA has more than one of them."""
+    torch.manual_seed(M)
+    sizes = (960, 320, 320)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    ws = [torch.randn(n, K, device=DEV).bfloat16() for n in sizes]
+    res = torch.randn(M, 1600, device=DEV).bfloat16()
+    want = cuda.gemm(x, torch.cat(ws).transpose(0, 1)).view(M, -1)
+    for r in (None, res) * 3:
+        out = torch.empty(M, 1600, device=DEV).bfloat16()
+        nv.call("ttcd_gemm_pieces", nv.ptr(x), nv.ptr(ws[0]), nv.ptr(ws[1]), nv.ptr(ws[2]), nv.ptr(out), nv.ptr(r), nv.i64(M), nv.i64(1600),
+                nv.i64(K), nv.i64(K), nv.i64(K), nv.i64(1600), nv.i64(960), nv.i64(320), nv.i32(0), nv.stream_ptr())
+        assert torch.equal(out, want if r is None else want + r)
