@@ -52,6 +52,21 @@ struct GemmSmem {
   static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 4) * 8 + 16;
 };
 
+// Whether `ok` holds for every thread of the two warps that meet at named barrier `bar`.
+__device__ __forceinline__ bool pair_all(bool ok, int bar) {
+  uint32_t all;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred P, Q;\n\t"
+      "setp.ne.b32 P, %1, 0;\n\t"
+      "bar.red.and.pred Q, %2, 64, P;\n\t"
+      "selp.u32 %0, 1, 0, Q;\n\t}"
+      : "=r"(all)
+      : "r"(static_cast<uint32_t>(ok)), "r"(bar)
+      : "memory");
+  return all != 0;
+}
+
 // SWIGLU: B's rows are half gate, half up; a tile of BN rows of B makes BN / 2 columns of C.  The product never reaches memory:
 // gate | up of 65536 x 3072 (K 1024) and the pass that combined them took 600 + 250 us, with 1.6 GB between them; 585 us so.
 template <int BN, int STAGES, bool A_MN, bool B_MN, typename OutT, bool HAS_CIN, bool SWIGLU = false>
@@ -203,7 +218,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
       const int64_t r = tile % tiles_per_batch;
       const int64_t m0 = (p.m_fastest ? r % p.tiles_m : r / p.tiles_n) * GEMM_BM;
       const int64_t n0 = (p.m_fastest ? r / p.tiles_m : r % p.tiles_n) * CN;
-      if (!mbar_wait(tfull_bar(acc), acc_phase[acc], abort_flag, 104)) { ok = false; break; }
+      // With SwiGLU a warp and its neighbour fill one box: 32 columns each, of 64.
+      const int part = (warp - 2) >> 2, pair = part >> 1, pair_bar = 1 + quarter * 2 + pair;
+      ok = mbar_wait(tfull_bar(acc), acc_phase[acc], abort_flag, 104);
+      if constexpr (SWIGLU) {
+        if ((part & 1) == 0 && lane == 0) tma_store_wait_read0();     // the last tile's store has released the buffer
+        // The two go on or leave together: one that left alone would keep the other at their next barrier for good.
+        ok = pair_all(ok, pair_bar);
+      }
+      if (!ok) break;
       tc_fence_after_sync();
       const int64_t row = m0 + quarter * 32 + lane;
       const bool row_ok = row < p.M;
@@ -213,19 +236,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
       const OutT* cin_row = HAS_CIN ? (Cin + b * p.stride_c + row * p.ldc) : nullptr;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
       if constexpr (SWIGLU) {
-        // this warp's 32 columns; it and its neighbour fill one box of 64
-        const int part = (warp - 2) >> 2, pair = part >> 1, c = part * 32;
+        const int c = part * 32;
         uint8_t* buf = smem + S::EPI_OFFSET + quarter * 8192 + pair * 4096;
-        auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter * 2 + pair) : "memory"); };
         uint32_t vg[32], vu[32];
         tmem_ld32(t_row + c, vg);
         tmem_ld32(t_row + CN + c, vu);
-        if ((part & 1) == 0 && lane == 0) tma_store_wait_read0();     // the last tile's store has released the buffer
         tmem_ld_wait();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(tempty_bar(acc));      // the accumulator is in registers
-        meet();
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
           float o[8];
@@ -244,7 +263,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ G
           *reinterpret_cast<uint4*>(buf + sw128_offset(lane, (c & 32) / 8 + (j >> 3))) = w;
         }
         fence_proxy_async_smem();
-        meet();
+        asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
         const int64_t col = n0 + pair * 64;
         if ((part & 1) == 0 && lane == 0 && col < p.N) {
           tma_store_3d(&tma_c, smem_u32(buf), static_cast<int>(col), static_cast<int>(m0 + quarter * 32), b);
