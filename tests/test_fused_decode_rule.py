@@ -1,4 +1,7 @@
 """Which models a decode step may bypass the modules of: the stock ones, and none of whose parts a program has replaced."""
+import subprocess
+import sys
+from pathlib import Path
 from types import MethodType, SimpleNamespace
 
 import pytest
@@ -7,6 +10,7 @@ import torch.nn as nn
 
 from ttcd_b200 import ops
 from ttcd_b200.models import IPTTCDv9Config, IPTTCDv9ForCausalLM, layers
+from ttcd_b200.models.base import DecoderForCausalLM
 from ttcd_b200.models.decoding import GraphDecoder, pack_projection_weights
 from ttcd_b200.models.layers import GatedMLP
 
@@ -134,3 +138,31 @@ def test_a_method_replaced_on_a_class_is_run_over_a_prompt(monkeypatch):
     assert _plain(model) == [True, False]
     monkeypatch.setattr(GatedMLP, "features", lambda self, x: x)
     assert _plain(model) == [False, False]
+
+
+BEFORE_THE_FIRST_PROMPT = """
+import torch
+from ttcd_b200.models import layers, modeling_ipttcdv9
+cls = {"GatedMLP": layers.GatedMLP, "IPTTCDBlock": modeling_ipttcdv9.IPTTCDBlock}["%s"]
+inner = cls.%s
+cls.%s = lambda self, *a, **k: inner(self, *a, **k)
+from tests.test_fused_decode_rule import _fused, _model, _plain
+model = _model()
+assert not any(_plain(model)), "a prompt"
+assert _fused(model) is None, "a decode step"
+"""
+
+
+@pytest.mark.parametrize("cls,method", [("GatedMLP", "features"), ("IPTTCDBlock", "forward")])
+def test_a_method_replaced_on_a_class_before_the_first_prompt_is_run(cls, method):
+    """In a process of its own: import, replace, run."""
+    root = Path(__file__).resolve().parents[1]
+    done = subprocess.run([sys.executable, "-c", BEFORE_THE_FIRST_PROMPT % (cls, method, method)], cwd=root, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr[-2000:]
+
+
+def test_a_model_class_with_another_forward_runs_it_in_every_decode_step(monkeypatch):
+    model = _model()
+    inner = DecoderForCausalLM.forward
+    monkeypatch.setattr(DecoderForCausalLM, "forward", lambda self, *a, **k: inner(self, *a, **k))
+    assert _fused(model) is None

@@ -17,6 +17,7 @@ from .modeling_ipttcdv9 import IPTTCDBlock, IPTTCDForCausalLM, IPTTCDMLP, IPTTCD
 from .modeling_ipttt import FastWeightCache, IPTTTBlock, IPTTTForCausalLM, IPTTTMLP, IPTTTModel
 from .modeling_ipttt_llama import IPTTTLlamaForCausalLM, TTTDynamicCache, ipttt_config_from_llama
 from .modeling_transformer import TransformerBlock, TransformerForCausalLM, TransformerModel
+from . import stock  # noqa: F401  (records the classes as they are defined here)
 
 IPTTCDv9Model = IPTTCDModel
 IPTTCDv9ForCausalLM = IPTTCDForCausalLM

@@ -78,17 +78,19 @@ def _fused_block_weights(block, batch: int):
     """The weights of a block whose decode step runs as six launches (``_fused_block_step``), or None where the step has
     to go through the modules: another kind of block or of a part of it, an option the step has no kernel for, a hook, a
     replaced method, a weight that is computed."""
-    from .layers import RMSNorm, _tp_state
+    from .layers import _tp_state
     from .modeling_ipttcdv9 import IPTTCDBlock, IPTTCDMLP
     from .modeling_transformer import TransformerBlock
-    if type(block) not in (IPTTCDBlock, TransformerBlock) or block.training or batch > 16 or _tp_state() is not None:
+    from .stock import unchanged
+    stock = unchanged()                 # (a method may have been replaced on a class)
+    if type(block) not in stock & {IPTTCDBlock, TransformerBlock} or block.training or batch > 16 or _tp_state() is not None:
         return None
     if type(block) is IPTTCDBlock and block.is_ttt_layer and block.ttt_chunk <= 1:       # one token would be a whole chunk
         return None
-    if not _as_defined(*block.modules()) or type(block.mlp) not in (GatedMLP, IPTTCDMLP):
+    if not _as_defined(*block.modules()) or type(block.mlp) not in stock & {GatedMLP, IPTTCDMLP}:
         return None
     attn, mlp = block.attn, block.mlp
-    if type(attn) is not Attention or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128):
+    if type(attn) is not Attention or not {Attention, RMSNorm} <= stock or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128):
         return None
     norms = [block.attn_norm, block.mlp_norm] + ([attn.q_norm, attn.k_norm] if attn.qk_norm else [])
     if any(type(n) is not RMSNorm or n.weight is None for n in norms):
@@ -170,6 +172,9 @@ class GraphDecoder:
     def _fused_weights(self, batch: int):
         """Per block the weights of its fused step; None if any part of the model has to run module by module."""
         from .base import DecoderForCausalLM, DecoderModel
+        from .stock import unchanged
+        if not {DecoderForCausalLM, DecoderModel, RMSNorm} <= unchanged():
+            return None
         model, core, head = self.model, self.model.model, self.model.lm_head
         if type(model).forward is not DecoderForCausalLM.forward or type(core).forward is not DecoderModel.forward:
             return None

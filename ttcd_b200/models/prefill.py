@@ -15,29 +15,11 @@ import ctypes
 import torch
 
 from .. import _native as nv
-from . import layers
-from .decoding import _STEP_METHODS, _as_defined
-from .layers import Attention, GatedMLP, RMSNorm, WindowKVCache
+from . import layers, stock
+from .decoding import _as_defined
+from .layers import Attention, WindowKVCache
 
 _BF16 = torch.bfloat16
-
-
-_METHODS = ("forward", "project_qkv", "finish", "features", "__call__")      # what the native call computes on behalf of
-_stock: dict | None = None
-
-
-def _methods(cls) -> tuple:
-    return tuple(getattr(cls, n, None) for n in _METHODS)
-
-
-def _stock_classes() -> dict:
-    """The classes that the native call stands for, with their methods as this package defines them."""
-    global _stock
-    if _stock is None:
-        from .modeling_ipttcdv9 import IPTTCDBlock, IPTTCDMLP
-        from .modeling_transformer import TransformerBlock
-        _stock = {cls: _methods(cls) for cls in (IPTTCDBlock, TransformerBlock, IPTTCDMLP, GatedMLP, Attention, RMSNorm, torch.nn.Linear)}
-    return _stock
 
 
 class PlainBlocks:
@@ -48,9 +30,9 @@ class PlainBlocks:
         self.B, self.T, self.hidden = x.shape
         self.scratch: dict = {}
         # classes that still are what this package made them, methods that a program may have replaced on an instance
-        self.classes = {cls for cls, methods in _stock_classes().items() if _methods(cls) == methods} if _as_defined() else set()
+        self.classes = stock.unchanged() if _as_defined() else set()
         self.blocks = {cls for cls in self.classes if cls.__name__.endswith("Block")}
-        self.replaceable = frozenset(_METHODS + _STEP_METHODS)
+        self.replaceable = frozenset(stock.METHODS)
 
     def _buffers(self, q_cols: int, inter: int, heads: int):
         key = (q_cols, inter, heads)
