@@ -166,3 +166,45 @@ def test_a_model_class_with_another_forward_runs_it_in_every_decode_step(monkeyp
     inner = DecoderForCausalLM.forward
     monkeypatch.setattr(DecoderForCausalLM, "forward", lambda self, *a, **k: inner(self, *a, **k))
     assert _fused(model) is None
+
+
+def _with_linears(path, **widths):
+    """Modules of other extents in the place of the stock ones, the attributes left as they were."""
+    def change(model):
+        parent = model.get_submodule(path)
+        for name, (n_in, n_out) in widths.items():
+            setattr(parent, name, nn.Linear(n_in, n_out, bias=False).to(torch.bfloat16))
+    return change
+
+
+@pytest.mark.parametrize("change", [
+    _with_linears("model.layers.0.mlp", gate_proj=(128, 128), up_proj=(128, 128), down_proj=(128, 128)),        # a pruned MLP
+    _with_linears("model.layers.0.mlp", up_proj=(128, 264)),
+    _with_linears("model.layers.0.attn", k_proj=(128, 128), v_proj=(128, 128)),
+    _with_linears("model.layers.0.attn", o_proj=(64, 128)),
+    lambda model: setattr(model.model.layers[0].attn, "q_norm", layers.RMSNorm(32).to(torch.bfloat16)),
+    lambda model: setattr(model.model.layers[0], "mlp_norm", layers.RMSNorm(64).to(torch.bfloat16)),
+    lambda model: setattr(model.model.layers[0].mlp, "intermediate_size", 512)])
+def test_a_block_with_weights_of_other_extents_runs_its_modules_over_a_prompt(change):
+    model = _model()
+    change(model)
+    assert _plain(model) == [False, False]
+
+
+def test_a_pruned_mlp_still_works():
+    model = _model()
+    ids = torch.arange(40).view(1, 40) % 64
+    _with_linears("model.layers.0.mlp", gate_proj=(128, 64), up_proj=(128, 64), down_proj=(64, 128))(model)
+    with torch.no_grad():
+        assert model(input_ids=ids).logits.isfinite().all()
+
+
+@pytest.mark.parametrize("table", [(200, 32), (300, 33), (300, 64)])
+def test_a_rotary_table_that_does_not_cover_the_prompt_is_left_to_the_modules(table, monkeypatch):
+    from ttcd_b200.models import prefill
+    model = _model()
+    block = model.model.layers[0]
+    monkeypatch.setattr(prefill.nv, "call", lambda *a: pytest.fail("launched"))
+    monkeypatch.setattr(block.attn.rotary, "tables", lambda *a: (torch.zeros(table, dtype=torch.bfloat16),) * 2)
+    x = torch.zeros(1, 300, 128, dtype=torch.bfloat16)
+    assert prefill.PlainBlocks(x, None)(block, x) is None

@@ -67,9 +67,14 @@ class PlainBlocks:
             return None
         # a weight that is made from others (a parametrization) is not in _parameters
         ws = [m._parameters.get("weight") for m in (*norms[:2], *linears, *norms[2:])]
+        # the native call goes by these extents; modules put in the place of the stock ones (a pruned MLP, say) may have others
+        dim, q_cols, kv_cols = attn.head_dim, attn.num_heads * attn.head_dim, attn.num_kv_heads * attn.head_dim
+        shapes = ((hidden,), (hidden,), (q_cols, hidden), (kv_cols, hidden), (kv_cols, hidden), (hidden, q_cols), (inter, hidden), (inter, hidden),
+                  (hidden, inter), (dim,), (dim,))
         device = self.device
-        for w in ws:
-            if type(w) is not torch.nn.Parameter or w.dtype is not _BF16 or w.device != device or not w.is_contiguous() or w.data_ptr() % 16:
+        for w, shape in zip(ws, shapes):
+            if (type(w) is not torch.nn.Parameter or w.dtype is not _BF16 or w.device != device or w.shape != shape or not w.is_contiguous()
+                    or w.data_ptr() % 16):
                 return None
         if getattr(ws[2], "_ttcd_gather", None) is not None:
             return None
@@ -88,7 +93,9 @@ class PlainBlocks:
         cos = sin = None
         if not attn.use_nope:
             cos, sin = attn.rotary.tables(max(T, attn.max_position_embeddings or 0), x.device, x.dtype)
-            if not (cos.is_contiguous() and sin.is_contiguous()) or cos.dtype != _BF16 or (cos.data_ptr() | sin.data_ptr()) % 16:
+            if cos.dim() != 2 or cos.shape != sin.shape or cos.shape[0] < T or 2 * cos.shape[1] > D:
+                return None
+            if any(t.dtype is not _BF16 or not t.is_contiguous() or t.data_ptr() % 16 for t in (cos, sin)):
                 return None
         q_cols, kv_cols = H * D, HK * D
         normed, rstd, q, o, lse, total, z = self._buffers(q_cols, block.mlp.intermediate_size, H)
