@@ -208,3 +208,14 @@ def test_a_rotary_table_that_does_not_cover_the_prompt_is_left_to_the_modules(ta
     monkeypatch.setattr(block.attn.rotary, "tables", lambda *a: (torch.zeros(table, dtype=torch.bfloat16),) * 2)
     x = torch.zeros(1, 300, 128, dtype=torch.bfloat16)
     assert prefill.PlainBlocks(x, None)(block, x) is None
+
+
+@pytest.mark.parametrize("change", [lambda x: x[:, ::2].contiguous(), lambda x: x.float(), lambda x: x[..., :64].contiguous(), lambda x: (x, None)])
+def test_what_another_block_hands_on_is_looked_at_before_every_block(change, monkeypatch):
+    """A hook on a block may drop tokens, or change the type; the blocks that follow must not go by the prompt's extents."""
+    from ttcd_b200.models import prefill
+    monkeypatch.setattr(prefill.nv, "call", lambda *a: pytest.fail("launched"))
+    model = _model()
+    x = torch.zeros(1, 300, 128, dtype=torch.bfloat16)
+    runner = prefill.PlainBlocks(x, None)
+    assert runner(model.model.layers[0], change(x)) is None

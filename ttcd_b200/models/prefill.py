@@ -26,7 +26,7 @@ class PlainBlocks:
     """Runs the blocks it can of one forward pass; made by ``plain_blocks``."""
 
     def __init__(self, x: torch.Tensor, past):
-        self.past, self.device = past, x.device
+        self.past, self.device, self.shape = past, x.device, x.shape
         self.B, self.T, self.hidden = x.shape
         self.scratch: dict = {}
         # classes that still are what this package made them, methods that a program may have replaced on an instance
@@ -82,6 +82,9 @@ class PlainBlocks:
 
     def __call__(self, block, x: torch.Tensor):
         """The block's output, or None where it has to run through its modules (nothing has been done then)."""
+        # (a block that ran through its modules, or a hook on it, may have handed on anything)
+        if type(x) is not torch.Tensor or x.shape != self.shape or x.dtype is not _BF16 or x.device != self.device:
+            return None
         ws = self._tensors(block)
         if ws is None or not x.is_contiguous() or x.data_ptr() % 16:
             return None
