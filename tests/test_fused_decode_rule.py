@@ -219,3 +219,27 @@ def test_what_another_block_hands_on_is_looked_at_before_every_block(change, mon
     x = torch.zeros(1, 300, 128, dtype=torch.bfloat16)
     runner = prefill.PlainBlocks(x, None)
     assert runner(model.model.layers[0], change(x)) is None
+
+
+def _one_projection(model):
+    """q, k and v from one linear of the program's own, the three taken out."""
+    attn = model.model.layers[0].attn
+    attn.qkv_proj = nn.Linear(128, 256, bias=False).to(torch.bfloat16)
+    for name in ("q_proj", "k_proj", "v_proj"):
+        delattr(attn, name)
+    attn.project_qkv = MethodType(lambda self, x, *a, **k: tuple(t.unflatten(-1, (-1, 64)) for t in self.qkv_proj(x).split((128, 64, 64), -1)), attn)
+
+
+def _no_norm(model):
+    block = model.model.layers[0]
+    del block.mlp_norm
+    block.forward = MethodType(lambda self, x, *a, **k: x + self.mlp(self.attn_norm(x)), block)
+
+
+@pytest.mark.parametrize("change", [_one_projection, _no_norm])
+def test_a_block_without_a_stock_part_runs_its_modules_over_a_prompt(change):
+    model = _model()
+    change(model)
+    assert _plain(model) == [False, False]
+    with torch.no_grad():
+        assert model(input_ids=torch.arange(40).view(1, 40) % 64, use_cache=False).logits.isfinite().all()

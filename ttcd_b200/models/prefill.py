@@ -52,18 +52,18 @@ class PlainBlocks:
         if getattr(block, "is_ttt_layer", False) and self.T >= block.ttt_chunk:
             return None
         parts = block._modules
-        attn, mlp = parts["attn"], parts["mlp"]
-        if type(attn) is not Attention or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128):
+        attn, mlp = parts.get("attn"), parts.get("mlp")
+        if type(attn) is not Attention or attn.use_output_gate or attn.use_l2_softmax or attn.head_dim not in (64, 128) or mlp is None:
             return None
-        linears = [attn._modules[n] for n in ("q_proj", "k_proj", "v_proj", "o_proj")] + [mlp._modules.get(n) for n in ("gate_proj", "up_proj", "down_proj")]
-        norms = [parts["attn_norm"], parts["mlp_norm"]] + ([attn._modules["q_norm"], attn._modules["k_norm"]] if attn.qk_norm else [])
+        linears = [attn._modules.get(n) for n in ("q_proj", "k_proj", "v_proj", "o_proj")] + [mlp._modules.get(n) for n in ("gate_proj", "up_proj", "down_proj")]
+        norms = [parts.get("attn_norm"), parts.get("mlp_norm")] + ([attn._modules.get("q_norm"), attn._modules.get("k_norm")] if attn.qk_norm else [])
         for m in (block, attn, mlp, *linears, *norms):
             if type(m) not in self.classes or m._forward_hooks or m._forward_pre_hooks or not self.replaceable.isdisjoint(m.__dict__):
                 return None
         hidden, inter = attn.hidden_size, mlp.intermediate_size
         if hidden != self.hidden or min(hidden, inter) < 128 or hidden % 8 or inter % 8 or attn.num_heads % attn.num_kv_heads:
             return None
-        if any(m._parameters["bias"] is not None for m in linears):
+        if any(m._parameters.get("bias") is not None for m in linears):
             return None
         # a weight that is made from others (a parametrization) is not in _parameters
         ws = [m._parameters.get("weight") for m in (*norms[:2], *linears, *norms[2:])]
