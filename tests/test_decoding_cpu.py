@@ -84,3 +84,22 @@ def test_l2_softmax_attention_statement_and_model_path():
     out.loss.backward()
     assert all(p.grad is not None for p in l2.parameters())
     assert not torch.allclose(out.logits, plain(input_ids=ids).logits, atol=1e-3)
+
+
+def test_prompts_on_another_device_are_left_to_indexed_copies(monkeypatch):
+    """The launch that loads the rings goes to the current device; layers elsewhere (or with more samples than a grid has) do not ride
+    along.  Tensors without memory: nothing is launched here."""
+    import warnings
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from ttcd_b200.ops import cuda
+    layers = []
+    monkeypatch.setattr(cuda.nv, "call", lambda symbol, record, count, *a: layers.append(count.value))
+    monkeypatch.setattr(cuda.nv, "stream_ptr", lambda: None)
+    with warnings.catch_warnings(), FakeTensorMode(), torch.no_grad():
+        warnings.simplefilter("ignore")
+        new = lambda batch, n: torch.empty(batch, n, 2, 64, dtype=torch.bfloat16, device="cuda:0")      # noqa: E731
+        todo = [(new(batch, 10), new(batch, 10), new(batch, 16), new(batch, 16)) for batch in (1, 65536, 1)]
+        for here, left in ((0, [1]), (1, [0, 1, 2])):
+            monkeypatch.setattr(torch.cuda, "current_device", lambda: here)
+            assert cuda.ring_load(todo, 10) == left
+    assert layers == [2]

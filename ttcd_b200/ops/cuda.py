@@ -162,15 +162,16 @@ def decode_qkv(qkv, ring_k, ring_v, slot, positions, qw, kw, eps, cos, sin, head
 def ring_load(layers: list[tuple], start: int) -> list[int]:
     """Copies a prompt's last rows into ring buffers, all layers in one launch: ``layers`` holds (k, v, ring_k, ring_v) with k, v
     [B, n, HK, D] and rings [B, capacity, HK, D]; row i of n goes to ring row (start - n + i) % capacity.  Returns the indices of
-    the entries it could not take (another dtype, rows that are not contiguous or not 16-byte aligned)."""
+    the entries it could not take (another dtype, a device that is not the current one, more samples than a grid has, rows that
+    are not contiguous or not 16-byte aligned)."""
     import ctypes
-    left, groups = [], {}
+    left, groups, here = [], {}, torch.cuda.current_device()
     for at, (k, v, rk, rv) in enumerate(layers):
         row = rk.shape[2] * rk.shape[3]
         ok = (rk.is_contiguous() and rv.is_contiguous() and row % 8 == 0 and k.shape == v.shape and rk.shape == rv.shape
               and k.shape[0] == rk.shape[0] and k.shape[2:] == rk.shape[2:] and k.shape[1] <= min(rk.shape[1], start)
               and not (torch.is_grad_enabled() and (k.requires_grad or v.requires_grad)) and rk[0].numel() < 2 ** 31
-              and all(t.dtype == _BF16 and t.is_cuda and t.data_ptr() % 16 == 0 for t in (k, v, rk, rv))
+              and rk.shape[0] <= 65535 and all(t.dtype == _BF16 and t.is_cuda and t.get_device() == here and t.data_ptr() % 16 == 0 for t in (k, v, rk, rv))
               and all(t.stride(3) == 1 and t.stride(2) == t.shape[3] and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0 for t in (k, v)))
         if not ok:
             left.append(at)
