@@ -17,10 +17,10 @@ int ttcd_attn_fwd(const void* q, const void* k, const void* v, void* o_t, void* 
 }
 
 // p: x, x_out, normed, rstd, qkv, q, k, o, lse, sum, z (device addresses; see below), the weights attn_norm, mlp_norm, Wq, Wk, Wv, Wo, Wg,
-// Wu, Wd, q_norm, k_norm (or 0), cos, sin (or 0), then B, T, hidden, inter, H, HK, D, window (0: none), heads' rotary half.
+// Wu, Wd, q_norm, k_norm (or 0), cos, sin (or 0), then B, T, hidden, inter, H, HK, D, window (0: none), heads' rotary half, wide.
 //   x, x_out, normed, sum [B T, hidden]; rstd [B T] fp32; qkv [B T, (H + 2 HK) D]; q [B T, H D]; k [B T, HK D]; o [B T, H D]; lse [B, H, T]
 //   fp32; z [B T, inter].  k (after norm and rotary; untouched where there is neither) and the last HK D columns of qkv are what a
-//   cache keeps.  All bf16 contiguous and 16-byte aligned; B T >= 128, T >= 128, hidden and inter >= 128 and multiples of 8, D 64 or 128.
+//   cache keeps.  wide [(H + 2 HK) D, hidden] (or 0): room for Wq, Wk and Wv side by side where that is the faster way.  All bf16 contiguous and 16-byte aligned; B T >= 128, T >= 128, hidden and inter >= 128 and multiples of 8, D 64 or 128.
 // f: eps of attn_norm, of mlp_norm, of q_norm / k_norm, the scores' scale.
 TTCD_EXPORT int ttcd_block_prefill(const long long* p, const float* f, void* stream_ptr) {
   using namespace ttcd;
@@ -32,6 +32,7 @@ TTCD_EXPORT int ttcd_block_prefill(const long long* p, const float* f, void* str
     return TTCD_ERR_ARG;
   for (int i = 0; i < 24; ++i)
     if ((p[i] == 0 && i < 20) || p[i] % 16 != 0) return TTCD_ERR_ARG;
+  if (p[33] % 16 != 0) return TTCD_ERR_ARG;
   const int64_t rows = B * T, q_cols = H * D, kv_cols = HK * D, cols = q_cols + 2 * kv_cols;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   bf16* const qkv = static_cast<bf16*>(at(4));
@@ -41,7 +42,17 @@ TTCD_EXPORT int ttcd_block_prefill(const long long* p, const float* f, void* str
   GemmCall g;
   g.a = at(2); g.b = at(13); g.c = qkv; g.M = rows; g.N = cols; g.K = hidden; g.lda = g.ldb = hidden; g.ldc = cols; g.stride_c = rows * cols;
   if (p[14] != p[13] + q_cols * hidden * 2 || p[15] != p[14] + kv_cols * hidden * 2) {     // three matrices, not one
-    g.b2 = at(14); g.b3 = at(15); g.n1 = q_cols; g.n2 = kv_cols;
+    if (p[33] != 0 && gemm_pieces_slow(rows, hidden, q_cols, kv_cols, kv_cols)) {
+      int64_t row = 0;
+      for (int i = 0; i < 3; ++i) {
+        const int64_t n = i == 0 ? q_cols : kv_cols;
+        TTCD_CUDA_CHECK(cudaMemcpyAsync(static_cast<bf16*>(at(33)) + row * hidden, at(13 + i), n * hidden * 2, cudaMemcpyDeviceToDevice, stream));
+        row += n;
+      }
+      g.b = at(33);
+    } else {
+      g.b2 = at(14); g.b3 = at(15); g.n1 = q_cols; g.n2 = kv_cols;
+    }
   }
   rc = gemm_run(g, stream);
   if (rc != TTCD_OK) return rc;

@@ -475,14 +475,26 @@ static int dispatch_major(const CUtensorMap& ta, const GemmBMaps& tb, const CUte
 //   one wave, few tiles: 300 x 1024 x 3072: 25.6 | 19.5 | 17.4; 448 x 2048 x 8192: 57 | 38 | 31; 2048 x 1024 x 32000: 178 | 118 | 168
 //   a second wave that is nearly empty: 6002 x 1024 x 3072: 46 | 42 | 56; 6144 x 1024 x 22646: 259 | 228 | 345
 //   full waves: 3832 x 1024 x 3072: 28 | 32 | 41; 32768 x 1024 x 2816: 131 | 147 | 207
-static int gemm_tile_n(int64_t M, int64_t N, int64_t batch) {
+static double gemm_tile_cost(int bn, int64_t M, int64_t N, int64_t batch) {
   const int64_t rows = (M + GEMM_BM - 1) / GEMM_BM * batch, sms = sm_count();
-  auto waves = [&](int bn) { return static_cast<double>((rows * ((N + bn - 1) / bn) + sms - 1) / sms); };
+  const double waves = static_cast<double>((rows * ((N + bn - 1) / bn) + sms - 1) / sms);
+  return bn == 256 ? waves : bn == 128 ? 0.56 * waves + 0.07 : 0.42 * waves + 0.12;
+}
+static int gemm_tile_n(int64_t M, int64_t N, int64_t batch) {
   int best = 128;
-  double cost = 0.56 * waves(128) + 0.07;
-  const double narrow = 0.42 * waves(64) + 0.12;
+  double cost = gemm_tile_cost(128, M, N, batch);
+  const double narrow = gemm_tile_cost(64, M, N, batch);
   if (narrow < cost) { best = 64; cost = narrow; }
-  return N >= 256 && waves(256) <= 1.06 * cost ? 256 : best;      // (5003 x 2048 x 2048, 3 | 2.87: 44 for 46 alone, no gain between others)
+  return N >= 256 && gemm_tile_cost(256, M, N, batch) <= 1.06 * cost ? 256 : best;      // (5003 x 2048 x 2048, 3 | 2.87: 44 for 46 alone, no gain between others)
+}
+
+// The widest tile, bn columns at most, whose rows of B come from one matrix each (n3 may be 0) and whose box fits in it; 0: none.
+static int gemm_piece_width(int bn, int64_t n1, int64_t n2, int64_t n3) {
+  int64_t least = n1 < n2 ? n1 : n2;
+  if (n3 > 0 && n3 < least) least = n3;
+  for (; bn >= 64; bn /= 2)
+    if (n1 % bn == 0 && (n3 == 0 || n2 % bn == 0) && least >= bn) return bn;
+  return 0;
 }
 
 }  // namespace ttcd
@@ -512,10 +524,8 @@ int ttcd::gemm_run(const GemmCall& g, cudaStream_t stream) {
   int BN = g.lse_part != nullptr ? (N >= 256 ? 256 : 128) : gemm_tile_n(M, g.swiglu ? 2 * N : N, batch);
   if (g.swiglu && BN < 128) BN = 128;              // (a box of C is 64 columns wide)
   if (g.n1 != 0) {                                 // a tile's rows of B come from one matrix, and its box fits in it
-    int64_t least = g.n1 < g.n2 ? g.n1 : g.n2;
-    if (n3 > 0 && n3 < least) least = n3;
-    while (BN > 64 && (g.n1 % BN != 0 || (n3 > 0 && g.n2 % BN != 0) || least < BN)) BN /= 2;
-    if (g.n1 % BN != 0 || (n3 > 0 && g.n2 % BN != 0) || least < BN) return TTCD_ERR_ARG;
+    BN = gemm_piece_width(BN, g.n1, g.n2, n3);
+    if (BN == 0) return TTCD_ERR_ARG;
   }
   CUtensorMap ta;
   GemmBMaps tb;
@@ -564,6 +574,18 @@ int ttcd::gemm_run(const GemmCall& g, cudaStream_t stream) {
   if (BN == 256) return dispatch_major<256, 4>(ta, tb, tc, g.c, g.c_in, p, g.a_mn, g.b_mn, g.out_fp32, stream);
   if (BN == 64) return dispatch_major<64, 8>(ta, tb, tc, g.c, g.c_in, p, g.a_mn, g.b_mn, g.out_fp32, stream);
   return dispatch_major<128, 6>(ta, tb, tc, g.c, g.c_in, p, g.a_mn, g.b_mn, g.out_fp32, stream);
+}
+
+// Weights of 960 + 320 + 320 columns leave no wider tile than 64, which costs 0.42 of a 256-wide one for a quarter of the columns; three
+// copies of a few MB take ~12 us, a unit of the cost ~6.7 ns of K.  us apart | copied, then one product:
+//   960 + 320 + 320, K 960: 4000 rows: 26.7 | 31.8, 8000: 39.7 | 39.9, 16000: 67.6 | 58.4, 65536: 240 | 171
+//   1024 + 192 + 192, K 1024: 8000 rows: 37.9 | 42.0, 16000: 63.6 | 60.4;  576 + 192 + 192, K 576: 16000: 32.8 | 40.0, 65536: 102 | 83
+// 128-wide tiles are not worth the copies (2048 + 128 + 128, K 2048, 65536 rows: 453 | 462).
+bool ttcd::gemm_pieces_slow(int64_t M, int64_t K, int64_t n1, int64_t n2, int64_t n3) {
+  const int64_t N = n1 + n2 + n3;
+  const int want = gemm_tile_n(M, N, 1);
+  if (want == 64 || gemm_piece_width(want, n1, n2, n3) != 64) return false;
+  return (gemm_tile_cost(64, M, N, 1) - gemm_tile_cost(want, M, N, 1)) * static_cast<double>(K) > 1800.0;
 }
 
 TTCD_EXPORT int ttcd_gemm_bf16(const void* a, const void* b, void* c, const void* c_in, const void* row_scale,

@@ -22,5 +22,7 @@ struct GemmCall {
   int swiglu = 0;
 };
 int gemm_run(const GemmCall& call, cudaStream_t stream);
+// Whether B's rows from matrices of n1, n2 and n3 rows make the product of M rows slower than putting them side by side first does.
+bool gemm_pieces_slow(int64_t M, int64_t K, int64_t n1, int64_t n2, int64_t n3);
 
 }  // namespace ttcd

@@ -68,3 +68,13 @@ def test_fast_weight_blocks_and_other_families_take_their_own_way(monkeypatch):
         with monkeypatch.context() as m:
             m.setattr(nv, "call", lambda symbol, *a, _c=nv.call: (_ for _ in ()).throw(AssertionError(symbol)) if symbol == "ttcd_block_prefill" else _c(symbol, *a))
             model(input_ids=ids, past_key_values=past, use_cache=True)
+
+
+@pytest.mark.parametrize("seq", [300, 700, 9000, 13000])
+def test_weights_that_leave_narrow_tiles_only(seq, monkeypatch):
+    """q|k|v of 960 + 320 + 320 columns: from three matrices, over one and several tiles per CTA, or copied side by side (13000 rows)."""
+    model = _model(15, 5, 64, 960, 256, 4096, False)
+    ids = torch.randint(0, 512, (1, seq), device=DEV)
+    got, kv, ran = _run(model, ids, True, monkeypatch)
+    want, kv_want, _ = _run(model, ids, False, monkeypatch)
+    assert ran == [True] * 3 and torch.equal(got, want) and all(torch.equal(a, b) for a, b in zip(kv, kv_want))

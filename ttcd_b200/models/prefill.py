@@ -34,14 +34,16 @@ class PlainBlocks:
         self.blocks = {cls for cls in self.classes if cls.__name__.endswith("Block")}
         self.replaceable = frozenset(stock.METHODS)
 
-    def _buffers(self, q_cols: int, inter: int, heads: int):
-        key = (q_cols, inter, heads)
+    def _buffers(self, q_cols: int, kv_cols: int, inter: int, heads: int):
+        key = (q_cols, kv_cols, inter, heads)
         got = self.scratch.get(key)
         if got is None:
             rows, dev = self.B * self.T, self.device
             new = lambda cols: torch.empty(rows, cols, dtype=_BF16, device=dev)      # noqa: E731
             f32 = lambda n: torch.empty(n, dtype=torch.float32, device=dev)          # noqa: E731
-            self.scratch[key] = got = (new(self.hidden), f32(rows), new(q_cols), new(q_cols), f32(heads * rows), new(self.hidden), new(inter))
+            # weights whose widths leave narrow tiles only may be put side by side (the native call decides)
+            wide = torch.empty(q_cols + 2 * kv_cols, self.hidden, dtype=_BF16, device=dev) if (q_cols | kv_cols) % 128 else None
+            self.scratch[key] = got = (new(self.hidden), f32(rows), new(q_cols), new(q_cols), f32(heads * rows), new(self.hidden), new(inter), wide)
         return got
 
     def _tensors(self, block):
@@ -101,14 +103,15 @@ class PlainBlocks:
             if any(t.dtype is not _BF16 or not t.is_contiguous() or t.data_ptr() % 16 for t in (cos, sin)):
                 return None
         q_cols, kv_cols = H * D, HK * D
-        normed, rstd, q, o, lse, total, z = self._buffers(q_cols, block.mlp.intermediate_size, H)
+        normed, rstd, q, o, lse, total, z, wide = self._buffers(q_cols, kv_cols, block.mlp.intermediate_size, H)
         qkv = torch.empty(B, T, q_cols + 2 * kv_cols, dtype=_BF16, device=x.device)
         k = torch.empty(B, T, HK, D, dtype=_BF16, device=x.device)
         out = torch.empty_like(x)
         at = [t.data_ptr() for t in (x, out, normed, rstd, qkv, q, k, o, lse, total, z)]
         at += [0 if w is None else w.data_ptr() for w in ws]
         at += [0, 0] if cos is None else [cos.data_ptr(), sin.data_ptr()]
-        at += [B, T, self.hidden, block.mlp.intermediate_size, H, HK, D, attn.window_size or 0, D // 2 if cos is None else cos.shape[-1]]
+        at += [B, T, self.hidden, block.mlp.intermediate_size, H, HK, D, attn.window_size or 0, D // 2 if cos is None else cos.shape[-1],
+               0 if wide is None else wide.data_ptr()]
         eps = (ctypes.c_float * 4)(block.attn_norm.eps, block.mlp_norm.eps, attn.q_norm.eps if attn.qk_norm else 0.0, D ** -0.5)
         nv.call("ttcd_block_prefill", (ctypes.c_longlong * len(at))(*at), eps, nv.stream_ptr())
         if past is not None:
