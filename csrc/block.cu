@@ -19,8 +19,9 @@ int ttcd_attn_fwd(const void* q, const void* k, const void* v, void* o_t, void* 
 // p: x, x_out, normed, rstd, qkv, q, k, o, lse, sum, z (device addresses; see below), the weights attn_norm, mlp_norm, Wq, Wk, Wv, Wo, Wg,
 // Wu, Wd, q_norm, k_norm (or 0), cos, sin (or 0), then B, T, hidden, inter, H, HK, D, window (0: none), heads' rotary half, wide.
 //   x, x_out, normed, sum [B T, hidden]; rstd [B T] fp32; qkv [B T, (H + 2 HK) D]; q [B T, H D]; k [B T, HK D]; o [B T, H D]; lse [B, H, T]
-//   fp32; z [B T, inter].  k (after norm and rotary; untouched where there is neither) and the last HK D columns of qkv are what a
-//   cache keeps.  wide [(H + 2 HK) D, hidden] (or 0): room for Wq, Wk and Wv side by side where that is the faster way.  All bf16 contiguous and 16-byte aligned; B T >= 128, T >= 128, hidden and inter >= 128 and multiples of 8, D 64 or 128.
+//   fp32; z [B T, inter]; normed may be x_out, sum may lie over q, and z over q and o.  k (after norm and rotary; untouched where there is neither) and
+//   the last HK D columns of qkv are what a cache keeps.  wide [(H + 2 HK) D, hidden] (or 0): room for Wq, Wk and Wv side by side where
+//   that is the faster way.  All bf16 contiguous and 16-byte aligned; B T >= 128, T >= 128, hidden and inter >= 128 and multiples of 8, D 64 or 128.
 // f: eps of attn_norm, of mlp_norm, of q_norm / k_norm, the scores' scale.
 TTCD_EXPORT int ttcd_block_prefill(const long long* p, const float* f, void* stream_ptr) {
   using namespace ttcd;

@@ -243,3 +243,18 @@ def test_a_block_without_a_stock_part_runs_its_modules_over_a_prompt(change):
     assert _plain(model) == [False, False]
     with torch.no_grad():
         assert model(input_ids=torch.arange(40).view(1, 40) % 64, use_cache=False).logits.isfinite().all()
+
+
+def test_scratch_of_native_blocks_is_given_back_to_a_block_that_runs_its_modules(monkeypatch):
+    from ttcd_b200.models import prefill
+    launches = []
+    monkeypatch.setattr(prefill.nv, "call", lambda symbol, record, *a: launches.append(list(record)))
+    monkeypatch.setattr(prefill.nv, "stream_ptr", lambda: None)
+    plain, fast_weight = _model().model.layers
+    x = torch.zeros(1, 300, 128, dtype=torch.bfloat16)
+    runner = prefill.PlainBlocks(x, None)
+    assert runner(plain, x) is not None and runner.scratch
+    assert runner(fast_weight, x) is None and not runner.scratch
+    # one piece of memory: the sum lies over q, which is done with by then, o behind both, the MLP's features behind the sum
+    q, o, total, z = (launches[0][i] for i in (5, 7, 9, 10))
+    assert total == q and o == q + 300 * 128 * 2 and z == total + 300 * 128 * 2

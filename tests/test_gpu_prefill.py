@@ -78,3 +78,22 @@ def test_weights_that_leave_narrow_tiles_only(seq, monkeypatch):
     got, kv, ran = _run(model, ids, True, monkeypatch)
     want, kv_want, _ = _run(model, ids, False, monkeypatch)
     assert ran == [True] * 3 and torch.equal(got, want) and all(torch.equal(a, b) for a, b in zip(kv, kv_want))
+
+
+@pytest.mark.parametrize("seq,inter,ttt_layers", [(20000, 1536, (1,)), (20000, 512, ()), (9000, 1536, (2,))])
+def test_a_prompt_takes_no_more_memory_than_its_modules(seq, inter, ttt_layers, monkeypatch):
+    model = _model(8, 4, 64, 512, inter, 4096, True, ttt_layers=ttt_layers)
+    ids = torch.randint(0, 512, (1, seq), device=DEV)
+    peak = []
+    for native in (True, False):
+        with monkeypatch.context() as m, torch.no_grad():
+            if not native:
+                m.setattr(prefill, "plain_blocks", lambda *a: None)
+            model(input_ids=ids[:, :256], logits_to_keep=1)         # (what stays: rotary tables)
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            torch.cuda.reset_peak_memory_stats()
+            at = torch.cuda.memory_allocated()
+            model(input_ids=ids, logits_to_keep=1)
+            peak.append(torch.cuda.max_memory_allocated() - at)
+    assert peak[0] <= 1.02 * peak[1], peak

@@ -38,12 +38,16 @@ class PlainBlocks:
         key = (q_cols, kv_cols, inter, heads)
         got = self.scratch.get(key)
         if got is None:
+            self.scratch.clear()
             rows, dev = self.B * self.T, self.device
-            new = lambda cols: torch.empty(rows, cols, dtype=_BF16, device=dev)      # noqa: E731
+            new = lambda n: torch.empty(n, dtype=_BF16, device=dev)                  # noqa: E731
             f32 = lambda n: torch.empty(n, dtype=torch.float32, device=dev)          # noqa: E731
+            # one piece of memory: q, then the sum in its place; o, read for the last time before z is written beside the sum
+            at_o = rows * max(q_cols, self.hidden)
+            piece = new(max(at_o + rows * q_cols, rows * (self.hidden + inter)))
             # weights whose widths leave narrow tiles only may be put side by side (the native call decides)
-            wide = torch.empty(q_cols + 2 * kv_cols, self.hidden, dtype=_BF16, device=dev) if (q_cols | kv_cols) % 128 else None
-            self.scratch[key] = got = (new(self.hidden), f32(rows), new(q_cols), new(q_cols), f32(heads * rows), new(self.hidden), new(inter), wide)
+            wide = new((q_cols + 2 * kv_cols) * self.hidden) if (q_cols | kv_cols) % 128 else None
+            self.scratch[key] = got = (f32(rows), piece, piece[at_o:], f32(heads * rows), piece, piece[rows * self.hidden:], wide)
         return got
 
     def _tensors(self, block):
@@ -84,6 +88,12 @@ class PlainBlocks:
 
     def __call__(self, block, x: torch.Tensor):
         """The block's output, or None where it has to run through its modules (nothing has been done then)."""
+        out = self._run(block, x)
+        if out is None:
+            self.scratch.clear()        # the modules have need of the memory
+        return out
+
+    def _run(self, block, x):
         # (a block that ran through its modules, or a hook on it, may have handed on anything)
         if type(x) is not torch.Tensor or x.shape != self.shape or x.dtype is not _BF16 or x.device != self.device:
             return None
@@ -103,11 +113,11 @@ class PlainBlocks:
             if any(t.dtype is not _BF16 or not t.is_contiguous() or t.data_ptr() % 16 for t in (cos, sin)):
                 return None
         q_cols, kv_cols = H * D, HK * D
-        normed, rstd, q, o, lse, total, z, wide = self._buffers(q_cols, kv_cols, block.mlp.intermediate_size, H)
+        rstd, q, o, lse, total, z, wide = self._buffers(q_cols, kv_cols, block.mlp.intermediate_size, H)
         qkv = torch.empty(B, T, q_cols + 2 * kv_cols, dtype=_BF16, device=x.device)
         k = torch.empty(B, T, HK, D, dtype=_BF16, device=x.device)
-        out = torch.empty_like(x)
-        at = [t.data_ptr() for t in (x, out, normed, rstd, qkv, q, k, o, lse, total, z)]
+        out = torch.empty_like(x)           # holds the normed rows until it is written
+        at = [t.data_ptr() for t in (x, out, out, rstd, qkv, q, k, o, lse, total, z)]
         at += [0 if w is None else w.data_ptr() for w in ws]
         at += [0, 0] if cos is None else [cos.data_ptr(), sin.data_ptr()]
         at += [B, T, self.hidden, block.mlp.intermediate_size, H, HK, D, attn.window_size or 0, D // 2 if cos is None else cos.shape[-1],
