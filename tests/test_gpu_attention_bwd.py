@@ -195,3 +195,26 @@ def test_combine_kernel_matches_torch(D):
     torch.testing.assert_close(delta_p, want_t + r * want_s, rtol=1e-4, atol=2e-3)
     want_do = do_t.float() + r.transpose(1, 2).unsqueeze(-1) * do_s.float()
     torch.testing.assert_close(do_p.float(), want_do, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("B,T,H,HK,D", [(2, 513, 15, 5, 64), (1, 300, 20, 20, 64), (3, 257, 8, 8, 128), (5, 300, 8, 4, 128)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_more_heads_than_run_together(B, T, H, HK, D, dual):
+    """Tiles run in groups of 16 heads (of all samples): more than one group of queries' or keys' heads, the last one not full; memory
+    that no tile writes would show as NaN."""
+    q, k, v = _inputs(B, T, H, HK, D)
+    qf, kf, vf = (t.detach().float().requires_grad_() for t in (q, k, v))
+    if dual:
+        outs, want = ops.dual_window_attention(q, k, v, 200, 100), ref.dual_window_attention(qf, kf, vf, 200, 100)
+    else:
+        outs, want = (ops.attention(q, k, v, window=200),), (ref.attention(qf, kf, vf, 200),)
+    grads = [torch.randn_like(o) for o in outs]
+    torch.use_deterministic_algorithms(True, warn_only=True)              # fills new memory with NaN
+    try:
+        torch.autograd.backward(outs, grads)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    torch.autograd.backward(want, [g.float() for g in grads])
+    _check(q.grad, qf.grad, "dq")
+    _check(k.grad, kf.grad, "dk")
+    _check(v.grad, vf.grad, "dv")

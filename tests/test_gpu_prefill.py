@@ -97,3 +97,14 @@ def test_a_prompt_takes_no_more_memory_than_its_modules(seq, inter, ttt_layers, 
             model(input_ids=ids, logits_to_keep=1)
             peak.append(torch.cuda.max_memory_allocated() - at)
     assert peak[0] <= 1.02 * peak[1], peak
+
+
+@pytest.mark.parametrize("seq", [128, 300, 511, 512])
+def test_a_fast_weight_block_below_its_chunk_is_a_plain_one(seq, monkeypatch):
+    """What every chat-sized prompt of the shipped models is (chunks of 4096)."""
+    model = _model(4, 2, 64, 256, 384, 256, True, ttt_layers=(1,))
+    model.model.layers[1].ttt_chunk = model.model.layers[1].mlp.ttt_chunk = 512
+    ids = torch.randint(0, 512, (2, seq), device=DEV)
+    got, kv, ran = _run(model, ids, True, monkeypatch)
+    want, kv_want, _ = _run(model, ids, False, monkeypatch)
+    assert ran == [True, seq < 512, True] and torch.equal(got, want) and all(torch.equal(a, b) for a, b in zip(kv, kv_want))
