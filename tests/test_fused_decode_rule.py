@@ -1,4 +1,5 @@
 """Which models a decode step may bypass the modules of: the stock ones, and none of whose parts a program has replaced."""
+import struct
 import subprocess
 import sys
 from pathlib import Path
@@ -248,7 +249,7 @@ def test_a_block_without_a_stock_part_runs_its_modules_over_a_prompt(change):
 def test_scratch_of_native_blocks_is_given_back_to_a_block_that_runs_its_modules(monkeypatch):
     from ttcd_b200.models import prefill
     launches = []
-    monkeypatch.setattr(prefill.nv, "call", lambda symbol, record, *a: launches.append(list(record)))
+    monkeypatch.setattr(prefill.nv, "call", lambda symbol, record, *a: launches.append(struct.unpack("34q", record)))
     monkeypatch.setattr(prefill.nv, "stream_ptr", lambda: None)
     plain, fast_weight = _model().model.layers
     x = torch.zeros(1, 300, 128, dtype=torch.bfloat16)
