@@ -213,7 +213,8 @@ struct DkdvCfg {
 };
 
 // This CTA's head (of all samples) and tile: heads fastest, up to 16 together, so that the tiles of a head that run at the same time or
-// soon after one another still share its rows in the L2 (128 heads of 4096 tokens in one group: a train step 1 % slower).
+// soon after one another still share its rows in the L2.  Backward, all heads together | by 16, ms: 5000 tokens, 16/8, D 128, windows
+// 4096 / 2048: 0.431 | 0.410; 8 x 4096, 16/8, D 128, 2048 / 1024: 1.746 | 1.665.
 __device__ __forceinline__ void bwd_tile(int heads, int tiles, int& hb, int& tile) {
   constexpr int GROUP = 16;
   const int first = static_cast<int>(blockIdx.x) / (GROUP * tiles) * GROUP, id = static_cast<int>(blockIdx.x) - first * tiles;
@@ -958,9 +959,11 @@ static int launch_bwd(const BwdMaps& m, AttnBwdParams p, int B, cudaStream_t str
   k1<<<p.heads_kv * ((p.Tk + 127) / 128), BWD_THREADS, smem1, stream>>>(m.q64, m.k128, m.v128, m.dot64, m.doc64, m.kh128, m.vh128, p);
   TTCD_CUDA_CHECK(cudaGetLastError());
   // dQ reads nothing that dK / dV writes: its CTAs start on SMs that the other kernel's last wave leaves idle, and wait for it only
-  // before they end.  (That kernel starts when everything before it is done, so all inputs are there.)  Forward + backward, with
-  // the last waves ordered as they are, against one kernel after the other in ascending order, ms: 5000 tokens, 16/8 heads, D 128,
-  // windows 4096 / 2048: 0.555 -> 0.478; 2 x 10007, 15/5, D 64, 8192 / 4096: 2.30 -> 2.24; 20000, 16/16, D 64, 2048 / 1024: no change.
+  // before they end.  (That kernel starts when everything before it is done, so all inputs are there.)  Forward + backward, ms: one kernel
+  // after the other in ascending order | ordered so that short tiles fill the last waves | dQ beside the end of dK / dV too:
+  //   5000 tokens, 16/8 heads, D 128, windows 4096 / 2048: 0.566 | 0.482 | 0.472;  5003, 32/8, D 64, no window: 0.750 | 0.632 | 0.617;
+  //   2 x 10007, 15/5, D 64, 8192 / 4096: 2.34 | 2.21 | 2.19;  65536, 16/8, D 128, 8192 / 4096: 17.6 | 17.6 | 17.7;
+  //   no gain with many short waves: 20000, 16/16, D 64, 2048 / 1024: 1.295 | 1.31 | 1.30;  8 x 4096, the same: 1.72 | 1.745 | 1.74.
   return launch_after(true, k2, p.heads_q * ((p.Tq + 127) / 128), BWD_THREADS, smem2, stream, m.q128, m.k64, m.v64, m.dot128, m.doc128, m.kh64,
                       m.vh64, p);
 }
